@@ -350,6 +350,159 @@ __device__ __forceinline__ void sort_candidates_two_warps(float *cand_k, uint32_
     __syncwarp();
 }
 
+// ---------------------------------------------------------------------------
+// Few candidates: most of what an expansion scores lies beyond the last beam slot and cannot enter
+// (the merge takes a candidate only where it is strictly smaller). `worst` is the beam's last key;
+// candidates above it are dropped before the sort, and when at most kFewSurvivors are left they are
+// inserted one by one instead of being sorted (15 exchange steps) and merged (5 + log2 NB steps).
+// A key equal to the last slot's stays: whether it enters is the networks' business.
+// Which elements are beyond the last slot changes neither the multiset nor, among equal keys, the
+// slots of the elements that stay: a comparator treats any two keys above the threshold alike.
+// The insertion gives the network's beam only when every key involved is distinct (a network may swap
+// equal keys, those that were in the beam before included). Otherwise the survivors, if they are
+// distinct among themselves, are still ranked by counting, and only the merge runs as a network; equal
+// survivors, or a NaN, send the expansion through both networks.
+// Bound by instruction issue and by the networks' chain of 20 dependent shuffles. Measured, networks
+// only against this: build of 1M x 128 rows (beams 64 and 128) 238 to 215 ms, 10,000 queries at beam 32
+// 655 to 627 us, 2,000 at beam 128 1136 to 1078 us.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kFewSurvivors = 8;
+
+__device__ __forceinline__ bool differs(float a, float b) { return a < b || a > b; }   // false for NaN
+
+template<int NB>
+__device__ __forceinline__ float last_key(const float (&bk)[NB], uint32_t beam) {   // beam is a multiple of 32, NB divides it
+    return __shfl_sync(kFullMask, bk[NB - 1], (beam - 1u) / NB);
+}
+
+// Candidates: slot 32*i + lane is (ck[i], cv[i]) in lane `lane`, survivors are the lanes of mask[i].
+// Which keys are equal (this lane's part of it): kTieSurvivors two survivors, or a survivor that is no
+// finite number; kTieBeam a survivor and a beam key, or two beam keys.
+constexpr uint32_t kTieSurvivors = 1, kTieBeam = 2;
+
+template<int NB, int NC>
+__device__ __forceinline__ uint32_t survivor_ties(const float (&bk)[NB], const float (&ck)[NC], const uint32_t (&mask)[NC]) {
+    const uint32_t lane = lane_id();
+    const float up = __shfl_up_sync(kFullMask, bk[NB - 1], 1);
+    bool own = false, with_beam = false;
+#pragma unroll
+    for (int i = 0; i < NB; i++) {
+        const float prev = i > 0 ? bk[i > 0 ? i - 1 : 0] : up;
+        with_beam = with_beam || (!(bk[i] >= FLT_MAX) && !(prev < bk[i]) && !(i == 0 && lane == 0));
+    }
+#pragma unroll
+    for (int n = 0; n < NC; n++) {
+        for (uint32_t m = mask[n]; m != 0; m &= m - 1u) {
+            const uint32_t src = (uint32_t) __ffs(m) - 1u;
+            const float c = __shfl_sync(kFullMask, ck[n], src);
+            own = own || !(c < FLT_MAX);
+#pragma unroll
+            for (int o = 0; o < NC; o++)
+                own = own || (((mask[o] >> lane) & 1u) && !(o == n && lane == src) && !differs(ck[o], c));
+#pragma unroll
+            for (int i = 0; i < NB; i++) with_beam = with_beam || !differs(bk[i], c);
+        }
+    }
+    return (own ? kTieSurvivors : 0u) | (with_beam ? kTieBeam : 0u);
+}
+
+// Survivors (distinct keys) in ascending order: afterwards lane j < count holds the j-th in (k, v), the
+// other lanes an empty slot. count <= kFewSurvivors.
+template<int NC>
+__device__ __forceinline__ void rank_survivors(const float (&ck)[NC], const uint32_t (&cv)[NC], const uint32_t (&mask)[NC], float &k, uint32_t &v) {
+    const uint32_t lane = lane_id();
+    uint32_t rank[NC];
+#pragma unroll
+    for (int n = 0; n < NC; n++) rank[n] = 0;
+#pragma unroll
+    for (int n = 0; n < NC; n++)
+        for (uint32_t m = mask[n]; m != 0; m &= m - 1u) {
+            const float c = __shfl_sync(kFullMask, ck[n], __ffs(m) - 1);
+#pragma unroll
+            for (int o = 0; o < NC; o++) rank[o] += c < ck[o] ? 1u : 0u;
+        }
+    float k_out = FLT_MAX;
+    uint32_t v_out = kInvalid;
+#pragma unroll
+    for (int n = 0; n < NC; n++)
+        for (uint32_t m = mask[n]; m != 0; m &= m - 1u) {
+            const int src = __ffs(m) - 1;
+            const float c = __shfl_sync(kFullMask, ck[n], src);
+            const uint32_t id = __shfl_sync(kFullMask, cv[n], src), r = __shfl_sync(kFullMask, rank[n], src);
+            if (lane == r) { k_out = c; v_out = id; }
+        }
+    k = k_out;
+    v = v_out;
+}
+
+template<int NB, int NC>
+__device__ __forceinline__ void insert_survivors(float (&bk)[NB], uint32_t (&bv)[NB], const float (&ck)[NC], const uint32_t (&cv)[NC],
+                                                 const uint32_t (&mask)[NC]) {
+    const uint32_t lane = lane_id();
+#pragma unroll
+    for (int n = 0; n < NC; n++) {
+        for (uint32_t m = mask[n]; m != 0; m &= m - 1u) {
+            const uint32_t src = (uint32_t) __ffs(m) - 1u;
+            const float c = __shfl_sync(kFullMask, ck[n], src);
+            const uint32_t id = __shfl_sync(kFullMask, cv[n], src);
+            const float up_k = __shfl_up_sync(kFullMask, bk[NB - 1], 1);
+            const uint32_t up_v = __shfl_up_sync(kFullMask, bv[NB - 1], 1);
+#pragma unroll
+            for (int i = NB - 1; i >= 0; i--) {
+                const float pk = i > 0 ? bk[i > 0 ? i - 1 : 0] : up_k;   // the slot before this one
+                const uint32_t pv = i > 0 ? bv[i > 0 ? i - 1 : 0] : up_v;
+                const bool here = (i == 0 && lane == 0) || pk < c;
+                if (bk[i] > c) {
+                    bk[i] = here ? c : pk;
+                    bv[i] = here ? id : pv;
+                }
+            }
+        }
+    }
+}
+
+template<int NB>
+__device__ __forceinline__ void trim_beam(float (&bk)[NB], uint32_t (&bv)[NB], uint32_t beam) {
+#pragma unroll
+    for (int i = 0; i < NB; i++) {
+        if (NB * lane_id() + i >= beam) {   // the reference keeps only `beam` slots between iterations
+            bk[i] = FLT_MAX;
+            bv[i] = kInvalid;
+        }
+    }
+}
+
+// Drops the candidates beyond the beam's last slot ((FLT_MAX, kInvalid), as an empty slot) and does as
+// much of the merge as few survivors allow. kMergeDone: the beam is merged. kMergeSorted: (ck[0], cv[0]) of lane j
+// is the j-th survivor, the merge is left to do. kMergeSort: both are.
+// open_seed: the seed row held a valid id with distance FLT_MAX; while such an entry may sit among the
+// beam's empty slots, which of them a merge replaces is the network's business too.
+enum MergeState : int { kMergeDone = 0, kMergeSorted = 1, kMergeSort = 2 };
+
+template<int NB, int NC>
+__device__ __forceinline__ MergeState merge_few(float (&bk)[NB], uint32_t (&bv)[NB], uint32_t beam, float (&ck)[NC], uint32_t (&cv)[NC], bool open_seed) {
+    const float worst = last_key<NB>(bk, beam);
+    uint32_t left[NC], count = 0;
+#pragma unroll
+    for (int n = 0; n < NC; n++) {
+        const bool in = cv[n] != kInvalid && !(ck[n] > worst);
+        left[n] = __ballot_sync(kFullMask, in);
+        count += __popc(left[n]);
+        if (!in) { ck[n] = FLT_MAX; cv[n] = kInvalid; }
+    }
+    if (count == 0) return kMergeDone;
+    if (count > kFewSurvivors) return kMergeSort;
+    const uint32_t ties = __reduce_or_sync(kFullMask, survivor_ties<NB, NC>(bk, ck, left));
+    if (ties & kTieSurvivors) return kMergeSort;
+    if (ties || (open_seed && worst == FLT_MAX)) {
+        rank_survivors<NC>(ck, cv, left, ck[0], cv[0]);
+        return kMergeSorted;
+    }
+    insert_survivors<NB, NC>(bk, bv, ck, cv, left);
+    trim_beam<NB>(bk, bv, beam);
+    return kMergeDone;
+}
+
 // The search loop proper. On return bk/bv hold the beam (ascending, position
 // j = NB*lane + i, ids still carrying the explored flag). Returns the number of
 // expansions; *rows_read accumulates data rows fetched.
@@ -365,28 +518,8 @@ __device__ __forceinline__ uint32_t beam_loop(float (&bk)[NB], uint32_t (&bv)[NB
     bool terminate = false;
     uint32_t rows = 0;
     while (true) {
-        // -- sort the candidates (search_kernel.cuh:9-37) --
-        // The reference sorts MAX_CANDIDATE = 64 slots even for degree <= 32, the upper half being
-        // padding (FLT_MAX, 0xffffffff). As long as every FLT_MAX slot carries the padding id, the
-        // first `degree` outputs of that network equal those of the 32-slot network on the real
-        // slots alone, ties included (checked exhaustively-at-random in
-        // tests/test_oracle_primitives.py); the only input that breaks this is the seed row's
-        // excluded id (valid id, FLT_MAX), flagged by wide_first_sort. Used by the build kernels
-        // (instruction bound); the query search kernel is bound by row gathers and measured
-        // slower with it.
-        if (NARROW_SORT && NC == 2 && degree <= 32 && !(wide_first_sort && iter == 0)) {
-            float ck[1] = {lane < degree ? s.cand_dist[lane] : FLT_MAX};
-            uint32_t cv[1] = {lane < degree ? s.cand_id[lane] : kInvalid};
-            warp_sort<1>(ck, cv);
-            __syncwarp();
-            if (lane < degree && lane < p.beam) {
-                s.cand_dist[lane] = ck[0];
-                s.cand_id[lane] = cv[0];
-            }
-            __syncwarp();
-        } else if constexpr (NC == 8) {
-            sort_candidates_two_warps(s.cand_dist, s.cand_id, degree, p.beam);
-        } else {
+        MergeState state = kMergeSort;
+        if (iter != 0) {
             float ck[NC];
             uint32_t cv[NC];
 #pragma unroll
@@ -395,49 +528,94 @@ __device__ __forceinline__ uint32_t beam_loop(float (&bk)[NB], uint32_t (&bv)[NB
                 ck[i] = (j < degree) ? s.cand_dist[j] : FLT_MAX;
                 cv[i] = (j < degree) ? s.cand_id[j] : kInvalid;
             }
-            warp_sort<NC>(ck, cv);
-            __syncwarp();
+            state = merge_few<NB, NC>(bk, bv, p.beam, ck, cv, wide_first_sort);
+            if (state != kMergeDone) {   // back to the strip: the survivors at their slots, or sorted from slot 0 on
 #pragma unroll
-            for (int i = 0; i < NC; i++) {
-                const uint32_t j = NC * lane + i;
-                if (j < degree && j < p.beam) {
-                    s.cand_dist[j] = ck[i];
-                    s.cand_id[j] = cv[i];
+                for (int i = 0; i < NC; i++) {
+                    const uint32_t j = lane + 32u * i;
+                    const bool gone = state == kMergeSorted && i > 0;
+                    if (j < degree) { s.cand_dist[j] = gone ? FLT_MAX : ck[i]; s.cand_id[j] = gone ? kInvalid : cv[i]; }
                 }
+                __syncwarp();
             }
-            __syncwarp();
         }
-        // -- merge into the beam (search_kernel.cuh:97-147) --
-        if (iter == 0) {
+        if (state == kMergeSort) {
+            // -- sort the candidates (search_kernel.cuh:9-37) --
+            // The reference sorts MAX_CANDIDATE = 64 slots even for degree <= 32, the upper half being
+            // padding (FLT_MAX, 0xffffffff). As long as every FLT_MAX slot carries the padding id, the
+            // first `degree` outputs of that network equal those of the 32-slot network on the real
+            // slots alone, ties included (checked exhaustively-at-random in
+            // tests/test_oracle_primitives.py); the only input that breaks this is the seed row's
+            // excluded id (valid id, FLT_MAX), flagged by wide_first_sort. Used by the build kernels
+            // (instruction bound); the query search kernel is bound by row gathers and measured
+            // slower with it.
+            if (NARROW_SORT && NC == 2 && degree <= 32 && !(wide_first_sort && iter == 0)) {
+                float ck[1] = {lane < degree ? s.cand_dist[lane] : FLT_MAX};
+                uint32_t cv[1] = {lane < degree ? s.cand_id[lane] : kInvalid};
+                warp_sort<1>(ck, cv);
+                __syncwarp();
+                if (lane < degree && lane < p.beam) {
+                    s.cand_dist[lane] = ck[0];
+                    s.cand_id[lane] = cv[0];
+                }
+                __syncwarp();
+            } else if constexpr (NC == 8) {
+                sort_candidates_two_warps(s.cand_dist, s.cand_id, degree, p.beam);
+            } else {
+                float ck[NC];
+                uint32_t cv[NC];
 #pragma unroll
-            for (int i = 0; i < NB; i++) {
-                const uint32_t j = NB * lane + i;
-                const bool take = (j < p.beam) && (j < degree);
-                bk[i] = take ? s.cand_dist[j] : FLT_MAX;
-                bv[i] = take ? s.cand_id[j] : kInvalid;
-            }
-        } else if constexpr (NB == 16) {
-            merge_beam_two_warps(bk, bv, p.beam, degree, s.cand_dist, s.cand_id, reinterpret_cast<float *>(s.tail), s.tail + 512);
-        } else {
+                for (int i = 0; i < NC; i++) {
+                    const uint32_t j = lane + 32u * i;
+                    ck[i] = (j < degree) ? s.cand_dist[j] : FLT_MAX;
+                    cv[i] = (j < degree) ? s.cand_id[j] : kInvalid;
+                }
+                warp_sort<NC>(ck, cv);
+                __syncwarp();
 #pragma unroll
-            for (int i = 0; i < NB; i++) {
-                const uint32_t j = NB * lane + i;
-                const uint32_t k = MAXB - 1 - j;
-                if (k < p.beam && k < degree) {
-                    const float c = s.cand_dist[k];
-                    if (bk[i] > c) {
-                        bk[i] = c;
-                        bv[i] = s.cand_id[k];
+                for (int i = 0; i < NC; i++) {
+                    const uint32_t j = NC * lane + i;
+                    if (j < degree && j < p.beam) {
+                        s.cand_dist[j] = ck[i];
+                        s.cand_id[j] = cv[i];
                     }
                 }
+                __syncwarp();
             }
-            warp_merge_final<NB>(bk, bv);
+        }
+        if (state != kMergeDone) {
+            // -- merge into the beam (search_kernel.cuh:97-147) --
+            if (iter == 0) {
 #pragma unroll
-            for (int i = 0; i < NB; i++) {
-                const uint32_t j = NB * lane + i;
-                if (j >= p.beam) {  // the reference keeps only `beam` slots between iterations
-                    bk[i] = FLT_MAX;
-                    bv[i] = kInvalid;
+                for (int i = 0; i < NB; i++) {
+                    const uint32_t j = NB * lane + i;
+                    const bool take = (j < p.beam) && (j < degree);
+                    bk[i] = take ? s.cand_dist[j] : FLT_MAX;
+                    bv[i] = take ? s.cand_id[j] : kInvalid;
+                }
+            } else if constexpr (NB == 16) {
+                merge_beam_two_warps(bk, bv, p.beam, degree, s.cand_dist, s.cand_id, reinterpret_cast<float *>(s.tail), s.tail + 512);
+            } else {
+#pragma unroll
+                for (int i = 0; i < NB; i++) {
+                    const uint32_t j = NB * lane + i;
+                    const uint32_t k = MAXB - 1 - j;
+                    if (k < p.beam && k < degree) {
+                        const float c = s.cand_dist[k];
+                        if (bk[i] > c) {
+                            bk[i] = c;
+                            bv[i] = s.cand_id[k];
+                        }
+                    }
+                }
+                warp_merge_final<NB>(bk, bv);
+#pragma unroll
+                for (int i = 0; i < NB; i++) {
+                    const uint32_t j = NB * lane + i;
+                    if (j >= p.beam) {  // the reference keeps only `beam` slots between iterations
+                        bk[i] = FLT_MAX;
+                        bv[i] = kInvalid;
+                    }
                 }
             }
         }
@@ -545,59 +723,71 @@ __device__ __forceinline__ uint32_t beam_loop_lanes(float (&bk)[NB], uint32_t (&
     bool terminate = false;
     uint32_t rows = 0;
     while (true) {
-        // -- sort the candidates (search_kernel.cuh:9-37): afterwards lane j holds the j-th --
-        if (wide_first_sort && iter == 0) {
-            float k2[2] = {ck, FLT_MAX};          // slot j = lane + 32*i
-            uint32_t v2[2] = {cv, kInvalid};
-            warp_sort<2>(k2, v2);                 // sorted position e = 2*lane + i
-            const float a = __shfl_sync(kFullMask, k2[0], lane >> 1), b = __shfl_sync(kFullMask, k2[1], lane >> 1);
-            const uint32_t c = __shfl_sync(kFullMask, v2[0], lane >> 1), d = __shfl_sync(kFullMask, v2[1], lane >> 1);
-            ck = (lane & 1u) ? b : a;
-            cv = (lane & 1u) ? d : c;
-        } else {
+        MergeState state = kMergeSort;
+        if (iter != 0) {
             float k1[1] = {ck};
             uint32_t v1[1] = {cv};
-            warp_sort<1>(k1, v1);
+            state = merge_few<NB, 1>(bk, bv, p.beam, k1, v1, wide_first_sort);
             ck = k1[0];
             cv = v1[0];
         }
-        // -- merge into the beam (search_kernel.cuh:97-147) --
-        if (iter == 0) {
-#pragma unroll
-            for (int i = 0; i < NB; i++) {
-                const uint32_t j = NB * lane + i;
-                const float c = __shfl_sync(kFullMask, ck, j & 31u);
-                const uint32_t id = __shfl_sync(kFullMask, cv, j & 31u);
-                const bool take = (j < p.beam) && (j < degree);
-                bk[i] = take ? c : FLT_MAX;
-                bv[i] = take ? id : kInvalid;
+        if (state == kMergeSort) {
+            // -- sort the candidates (search_kernel.cuh:9-37): afterwards lane j holds the j-th --
+            if (wide_first_sort && iter == 0) {
+                float k2[2] = {ck, FLT_MAX};          // slot j = lane + 32*i
+                uint32_t v2[2] = {cv, kInvalid};
+                warp_sort<2>(k2, v2);                 // sorted position e = 2*lane + i
+                const float a = __shfl_sync(kFullMask, k2[0], lane >> 1), b = __shfl_sync(kFullMask, k2[1], lane >> 1);
+                const uint32_t c = __shfl_sync(kFullMask, v2[0], lane >> 1), d = __shfl_sync(kFullMask, v2[1], lane >> 1);
+                ck = (lane & 1u) ? b : a;
+                cv = (lane & 1u) ? d : c;
+            } else {
+                float k1[1] = {ck};
+                uint32_t v1[1] = {cv};
+                warp_sort<1>(k1, v1);
+                ck = k1[0];
+                cv = v1[0];
             }
-        } else if constexpr (NB == 16) {
-            float *row_k = reinterpret_cast<float *>(s.tail + 1024);
-            uint32_t *row_v = s.tail + 1024 + 32;
-            row_k[lane] = ck;          // the sorted candidate row, slot = lane
-            row_v[lane] = cv;
-            __syncwarp();
-            merge_beam_two_warps(bk, bv, p.beam, degree, row_k, row_v, reinterpret_cast<float *>(s.tail), s.tail + 512);
-        } else {
+        }
+        if (state != kMergeDone) {
+            // -- merge into the beam (search_kernel.cuh:97-147) --
+            if (iter == 0) {
 #pragma unroll
-            for (int i = 0; i < NB; i++) {
-                const uint32_t j = NB * lane + i;
-                const uint32_t k = MAXB - 1 - j;
-                const float c = __shfl_sync(kFullMask, ck, k & 31u);
-                const uint32_t id = __shfl_sync(kFullMask, cv, k & 31u);
-                if (k < p.beam && k < degree && bk[i] > c) {
-                    bk[i] = c;
-                    bv[i] = id;
+                for (int i = 0; i < NB; i++) {
+                    const uint32_t j = NB * lane + i;
+                    const float c = __shfl_sync(kFullMask, ck, j & 31u);
+                    const uint32_t id = __shfl_sync(kFullMask, cv, j & 31u);
+                    const bool take = (j < p.beam) && (j < degree);
+                    bk[i] = take ? c : FLT_MAX;
+                    bv[i] = take ? id : kInvalid;
                 }
-            }
-            warp_merge_final<NB>(bk, bv);
+            } else if constexpr (NB == 16) {
+                float *row_k = reinterpret_cast<float *>(s.tail + 1024);
+                uint32_t *row_v = s.tail + 1024 + 32;
+                row_k[lane] = ck;          // the sorted candidate row, slot = lane
+                row_v[lane] = cv;
+                __syncwarp();
+                merge_beam_two_warps(bk, bv, p.beam, degree, row_k, row_v, reinterpret_cast<float *>(s.tail), s.tail + 512);
+            } else {
 #pragma unroll
-            for (int i = 0; i < NB; i++) {
-                const uint32_t j = NB * lane + i;
-                if (j >= p.beam) {  // the reference keeps only `beam` slots between iterations
-                    bk[i] = FLT_MAX;
-                    bv[i] = kInvalid;
+                for (int i = 0; i < NB; i++) {
+                    const uint32_t j = NB * lane + i;
+                    const uint32_t k = MAXB - 1 - j;
+                    const float c = __shfl_sync(kFullMask, ck, k & 31u);
+                    const uint32_t id = __shfl_sync(kFullMask, cv, k & 31u);
+                    if (k < p.beam && k < degree && bk[i] > c) {
+                        bk[i] = c;
+                        bv[i] = id;
+                    }
+                }
+                warp_merge_final<NB>(bk, bv);
+#pragma unroll
+                for (int i = 0; i < NB; i++) {
+                    const uint32_t j = NB * lane + i;
+                    if (j >= p.beam) {  // the reference keeps only `beam` slots between iterations
+                        bk[i] = FLT_MAX;
+                        bv[i] = kInvalid;
+                    }
                 }
             }
         }
