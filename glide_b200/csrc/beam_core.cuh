@@ -34,8 +34,10 @@ struct WarpStrip {
     float *cand_dist;    // 32*NC
     uint32_t *visited;   // visited_words(hash_bit)
     uint32_t *work;      // 32*NC: slots of the candidates to score
-    uint32_t *work_id;   // 32*NC: their ids
+    uint32_t *work_id;   // 32*NC: their ids (TEAM: an adjacency row's ids, slot by slot)
+    float *work_dist;    // TEAM: their distances (the place of `work`, which teams do not use)
     uint32_t *extra;     // mode-specific scratch (pool, rows, merge buffers)
+    struct TeamCall *team;   // only in kernels whose CTA shares one search (TEAM): the master's calls to the other warps
     uint32_t *tail;      // the last kTwoWarpScratch words of the strip: present (and set by the kernel) only for beams
                          // above 256 slots, whose merge runs on shared arrays (merge_beam_two_warps)
 };
@@ -58,9 +60,82 @@ __device__ __forceinline__ WarpStrip make_strip(uint32_t *base, uint32_t dim, ui
     s.visited = s.cand_id + 2 * max_cand;
     s.work = s.visited + visited_words(hash_bit);
     s.work_id = s.work + max_cand;
+    s.work_dist = reinterpret_cast<float *>(s.work);
     s.extra = s.work_id + max_cand;
+    s.team = nullptr;
     s.tail = nullptr;
     return s;
+}
+
+// ---------------------------------------------------------------------------
+// Teams: for batches too small to fill the device with a warp per search, a CTA of several warps shares
+// one. Warp 0 (the master) runs the search as a lone warp would: beam, visited set, merges; the others
+// (helpers) score rows. Each row is still read and summed by one whole warp, so the results are those of a
+// lone warp bit for bit. What it buys is latency: a lone warp has eight rows in flight (four of more than
+// 128 values) and pays a trip to memory per batch, a team one per expansion. The helpers also ask for the
+// adjacency rows of the candidates they score, one of which the next expansion reads.
+//   rows that fit the lanes   the helpers score a whole adjacency row while the master puts its ids into the
+//                             visited set, a chain as long as a trip to memory; the distances of the ids that
+//                             were not new (about a tenth) are dropped. Four helpers, beam 64, one query:
+//                             207 us alone, 162 with the set in front of the scoring, 120 beside it.
+//   wider rows                the set comes first and the master scores its share too: rows that are dropped
+//                             and a warp that does not read cost more than the set's chain (960 values,
+//                             degree 64, 300 queries: 274 us this way, 378 the other).
+// ---------------------------------------------------------------------------
+struct TeamCall {
+    const float *data;
+    const uint32_t *graph;
+    uint32_t n;         // rows to score, or kTeamQuit
+    uint32_t pad[3];
+};
+constexpr uint32_t kTeamQuit = 0xffffffffu;
+constexpr uint32_t kTeamCallWords = sizeof(TeamCall) / 4;
+
+__device__ __forceinline__ void team_barrier() { __syncthreads(); }
+
+// The master's calls. work_id[0..n) holds ids (kInvalid: none); between a call and the wait that follows it the team
+// writes work_dist[0..n).
+__device__ __forceinline__ void team_call(const WarpStrip &s, const float *__restrict__ data, const uint32_t *__restrict__ graph, uint32_t n) {
+    if (lane_id() == 0) {
+        s.team->data = data;
+        s.team->graph = graph;
+        s.team->n = n;
+    }
+    team_barrier();
+}
+__device__ __forceinline__ void team_wait() { team_barrier(); }
+
+// What one warp of the team scores of a call.
+template<typename D>
+__device__ __forceinline__ void team_share(const WarpStrip &s, const float *__restrict__ data, uint32_t n, D dim, int metric) {
+    const uint32_t warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    auto id_at = [&](uint32_t i) { const uint32_t id = s.work_id[i]; return id != kInvalid ? id : 0u; };
+    auto sink = [&](uint32_t i, float d) { s.work_dist[i] = d; };
+    if (dim_fits(dim)) warp_rows_v4<1>(s.query, data, dim, metric, n, id_at, sink, 8u * (warp - 1u), 8u * (warps - 1u));
+    else warp_rows_generic(s.query, data, dim, metric, n, id_at, sink, kWideRows * warp, kWideRows * warps);
+}
+
+// The helpers: serve calls until the master quits.
+template<typename D>
+__device__ __forceinline__ void team_serve(const WarpStrip &s, D dim, uint32_t degree, int metric) {
+    const uint32_t lane = lane_id(), helper = (threadIdx.x >> 5) - 1u, helpers = (blockDim.x >> 5) - 1u;
+    while (true) {
+        team_barrier();
+        const uint32_t n = s.team->n;
+        if (n == kTeamQuit) return;
+        const uint32_t *graph = s.team->graph;
+        for (uint32_t i = helper + helpers * lane; i < n; i += 32u * helpers) {
+            const uint32_t id = s.work_id[i];
+            if (id != kInvalid) asm volatile("prefetch.global.L2 [%0];" ::"l"(graph + (uint64_t) id * degree));
+        }
+        team_share(s, s.team->data, n, dim, metric);
+        team_barrier();
+    }
+}
+
+__device__ __forceinline__ void team_quit(const WarpStrip &s) {
+    if (lane_id() == 0) s.team->n = kTeamQuit;
+    team_barrier();
 }
 
 __device__ __forceinline__ void load_query(float *q_smem, const float *q_global, uint32_t dim) {
@@ -81,8 +156,9 @@ __device__ __forceinline__ void load_query(float *q_smem, const float *q_global,
 // compacted into the strip's work list and scored by warp_rows (whole-warp row loads,
 // several rows in flight). Returns the number of rows read by this warp
 // (for the traffic counters).
+template<typename D>
 __device__ __forceinline__ uint32_t score_candidates(const WarpStrip &s, uint32_t count, uint32_t skip_id,
-                                                     const float *__restrict__ data, uint32_t dim, int metric) {
+                                                     const float *__restrict__ data, D dim, int metric) {
     const uint32_t lane = lane_id();
     uint32_t n = 0;
     for (uint32_t base = 0; base < count; base += 32) {
@@ -106,12 +182,87 @@ __device__ __forceinline__ uint32_t score_candidates(const WarpStrip &s, uint32_
     return n;
 }
 
+// TEAM: an adjacency row of `degree` entries scored by the team (see above). Ids that are not new (or are
+// `skip_insert`) leave empty candidate slots, `skip_score` keeps its slot with distance FLT_MAX. Returns the number
+// of candidates that got a distance; *skip_kept: skip_score was new.
+template<typename D>
+__device__ __forceinline__ uint32_t team_expand(const WarpStrip &s, const uint32_t *__restrict__ row, bool have_row, uint32_t skip_insert,
+                                                uint32_t skip_score, const uint32_t *__restrict__ graph, uint32_t degree,
+                                                uint32_t hash_bit, const float *__restrict__ data, D dim, int metric, bool *skip_kept) {
+    const uint32_t lane = lane_id();
+    if (dim_fits(dim)) {
+        for (uint32_t i = lane; i < degree; i += 32) s.work_id[i] = have_row ? __ldg(row + i) : kInvalid;
+        __syncwarp();
+        team_call(s, data, graph, degree);
+    }
+    uint32_t rows = 0;
+    bool kept = false;
+    for (uint32_t base = 0; base < degree; base += 32) {
+        const uint32_t i = base + lane;
+        uint32_t nb = kInvalid;
+        if (i < degree && have_row) nb = dim_fits(dim) ? s.work_id[i] : __ldg(row + i);
+        const uint32_t flag = visited_insert(s.visited, hash_bit, nb, nb != kInvalid && nb != skip_insert);
+        if (i < degree) s.cand_id[i] = flag ? nb : kInvalid;
+        const bool scored = flag && nb != skip_score;
+        const uint32_t mask = __ballot_sync(kFullMask, scored);
+        if (!dim_fits(dim) && scored) s.work_id[rows + __popc(mask & ((1u << lane) - 1u))] = nb;
+        rows += __popc(mask);
+        kept = kept || __any_sync(kFullMask, flag && nb == skip_score);
+    }
+    if (!dim_fits(dim)) {
+        __syncwarp();
+        team_call(s, data, graph, rows);
+        team_share(s, data, rows, dim, metric);
+    }
+    team_wait();
+    uint32_t at = 0;
+    for (uint32_t base = 0; base < degree; base += 32) {
+        const uint32_t i = base + lane;
+        const uint32_t id = i < degree ? s.cand_id[i] : kInvalid;
+        const bool scored = id != kInvalid && id != skip_score;
+        const uint32_t mask = __ballot_sync(kFullMask, scored);
+        if (i < degree) s.cand_dist[i] = scored ? s.work_dist[dim_fits(dim) ? i : at + __popc(mask & ((1u << lane) - 1u))] : FLT_MAX;
+        at += __popc(mask);
+    }
+    if (skip_kept) *skip_kept = kept;
+    __syncwarp();
+    return rows;
+}
+
+// The same for lane-resident candidates: `nb` is this lane's adjacency entry.
+template<typename D>
+__device__ __forceinline__ uint32_t team_expand_lanes(const WarpStrip &s, uint32_t nb, uint32_t skip_insert, uint32_t skip_score,
+                                                      const uint32_t *__restrict__ graph, uint32_t degree, uint32_t hash_bit,
+                                                      const float *__restrict__ data, D dim, int metric, float &ck, uint32_t &cv) {
+    const uint32_t lane = lane_id();
+    if (dim_fits(dim)) {
+        if (lane < degree) s.work_id[lane] = nb;
+        __syncwarp();
+        team_call(s, data, graph, degree);
+    }
+    cv = visited_insert(s.visited, hash_bit, nb, nb != kInvalid && nb != skip_insert) ? nb : kInvalid;
+    const bool scored = cv != kInvalid && cv != skip_score;
+    const uint32_t mask = __ballot_sync(kFullMask, scored), rank = __popc(mask & ((1u << lane) - 1u));
+    if (!dim_fits(dim)) {
+        if (scored) s.work_id[rank] = nb;
+        __syncwarp();
+        team_call(s, data, graph, __popc(mask));
+        team_share(s, data, __popc(mask), dim, metric);
+    }
+    team_wait();
+    ck = scored ? s.work_dist[dim_fits(dim) ? lane : rank] : FLT_MAX;
+    return __popc(mask);
+}
+
 // search_kernel.cuh:362-391: read the parent's adjacency row, keep ids that are new
 // to the visited set (and are not own_id), then score them.
+template<bool TEAM = false, typename D>
 __device__ __forceinline__ uint32_t expand_parent(const WarpStrip &s, uint32_t parent, uint32_t own_id,
                                                   const uint32_t *__restrict__ graph, uint32_t degree,
                                                   uint32_t hash_bit, const float *__restrict__ data,
-                                                  uint32_t dim, int metric) {
+                                                  D dim, int metric) {
+    if constexpr (TEAM)
+        return team_expand(s, graph + (uint64_t) parent * degree, parent != kInvalid, own_id, kInvalid, graph, degree, hash_bit, data, dim, metric, nullptr);
     for (uint32_t base = 0; base < degree; base += 32) {
         const uint32_t i = base + lane_id();
         uint32_t nb = kInvalid;
@@ -127,10 +278,13 @@ __device__ __forceinline__ uint32_t expand_parent(const WarpStrip &s, uint32_t p
 // slot but gets distance FLT_MAX.
 // *excluded_kept is set when the excluded id occurs: that slot then holds a valid id with distance
 // FLT_MAX, the one input the narrow candidate sort of beam_loop cannot take.
+template<bool TEAM = false, typename D>
 __device__ __forceinline__ uint32_t seed_from_row(const WarpStrip &s, uint32_t start_point, uint32_t exclude_id,
                                                   const uint32_t *__restrict__ graph, uint32_t degree,
                                                   uint32_t hash_bit, const float *__restrict__ data,
-                                                  uint32_t dim, int metric, bool *excluded_kept = nullptr) {
+                                                  D dim, int metric, bool *excluded_kept = nullptr) {
+    if constexpr (TEAM)
+        return team_expand(s, graph + (uint64_t) start_point * degree, true, kInvalid, exclude_id, graph, degree, hash_bit, data, dim, metric, excluded_kept);
     bool kept = false;
     for (uint32_t base = 0; base < degree; base += 32) {
         const uint32_t i = base + lane_id();
@@ -506,11 +660,11 @@ __device__ __forceinline__ MergeState merge_few(float (&bk)[NB], uint32_t (&bv)[
 // The search loop proper. On return bk/bv hold the beam (ascending, position
 // j = NB*lane + i, ids still carrying the explored flag). Returns the number of
 // expansions; *rows_read accumulates data rows fetched.
-template<int NB, int NC, bool NARROW_SORT = false>
+template<int NB, int NC, bool NARROW_SORT = false, bool TEAM = false, typename D>
 __device__ __forceinline__ uint32_t beam_loop(float (&bk)[NB], uint32_t (&bv)[NB], const WarpStrip &s,
                                               const BeamParams &p, uint32_t own_id,
                                               const uint32_t *__restrict__ graph, uint32_t degree,
-                                              const float *__restrict__ data, uint32_t dim, int metric,
+                                              const float *__restrict__ data, D dim, int metric,
                                               uint32_t *rows_read, bool wide_first_sort = false) {
     const uint32_t lane = lane_id();
     constexpr uint32_t MAXB = 32u * NB;
@@ -659,7 +813,7 @@ __device__ __forceinline__ uint32_t beam_loop(float (&bk)[NB], uint32_t (&bv)[NB
             __syncwarp();
         }
         if (terminate && iter >= p.min_iterations) break;
-        rows += expand_parent(s, parent, own_id, graph, degree, p.hash_bit, data, dim, metric);
+        rows += expand_parent<TEAM>(s, parent, own_id, graph, degree, p.hash_bit, data, dim, metric);
         iter++;
     }
     if (rows_read) *rows_read += rows;
@@ -678,13 +832,19 @@ __device__ __forceinline__ uint32_t beam_loop(float (&bk)[NB], uint32_t (&bv)[NB
 //  * for beam <= 32 the 64-position merge network splits, after its first stride-32 step, into
 //    two independent halves of which only the lower one is kept, so NB = 1 gives the same beam.
 // ---------------------------------------------------------------------------
+template<bool TEAM = false, typename D>
 __device__ __forceinline__ uint32_t seed_lanes(const WarpStrip &s, uint32_t start_point, uint32_t exclude_id,
                                                const uint32_t *__restrict__ graph, uint32_t degree, uint32_t hash_bit,
-                                               const float *__restrict__ data, uint32_t dim, int metric, float &ck,
+                                               const float *__restrict__ data, D dim, int metric, float &ck,
                                                uint32_t &cv, bool *excluded_kept = nullptr) {
     const uint32_t lane = lane_id();
     uint32_t index = kInvalid;
     if (lane < degree) index = __ldg(graph + (uint64_t) start_point * degree + lane);
+    if constexpr (TEAM) {
+        const uint32_t rows = team_expand_lanes(s, index, kInvalid, exclude_id, graph, degree, hash_bit, data, dim, metric, ck, cv);
+        if (excluded_kept) *excluded_kept = __any_sync(kFullMask, cv != kInvalid && cv == exclude_id);
+        return rows;
+    }
     const uint32_t flag = visited_insert(s.visited, hash_bit, index, index != kInvalid);
     cv = flag ? index : kInvalid;
     if (excluded_kept) *excluded_kept = __ballot_sync(kFullMask, flag && index == exclude_id) != 0;
@@ -694,13 +854,15 @@ __device__ __forceinline__ uint32_t seed_lanes(const WarpStrip &s, uint32_t star
     return __popc(mask);
 }
 
+template<bool TEAM = false, typename D>
 __device__ __forceinline__ uint32_t expand_lanes(const WarpStrip &s, uint32_t parent, uint32_t own_id,
                                                  const uint32_t *__restrict__ graph, uint32_t degree, uint32_t hash_bit,
-                                                 const float *__restrict__ data, uint32_t dim, int metric, float &ck,
+                                                 const float *__restrict__ data, D dim, int metric, float &ck,
                                                  uint32_t &cv) {
     const uint32_t lane = lane_id();
     uint32_t nb = kInvalid;
     if (lane < degree && parent != kInvalid) nb = __ldg(graph + (uint64_t) parent * degree + lane);
+    if constexpr (TEAM) return team_expand_lanes(s, nb, own_id, kInvalid, graph, degree, hash_bit, data, dim, metric, ck, cv);
     const uint32_t flag = visited_insert(s.visited, hash_bit, nb, nb != kInvalid && nb != own_id);
     cv = flag ? nb : kInvalid;
     const uint32_t mask = __ballot_sync(kFullMask, flag != 0);
@@ -710,11 +872,11 @@ __device__ __forceinline__ uint32_t expand_lanes(const WarpStrip &s, uint32_t pa
 }
 
 // (ck, cv): the seed step's candidates, slot = lane. Otherwise as beam_loop.
-template<int NB>
+template<int NB, bool TEAM = false, typename D>
 __device__ __forceinline__ uint32_t beam_loop_lanes(float (&bk)[NB], uint32_t (&bv)[NB], const WarpStrip &s,
                                                     const BeamParams &p, uint32_t own_id,
                                                     const uint32_t *__restrict__ graph, uint32_t degree,
-                                                    const float *__restrict__ data, uint32_t dim, int metric,
+                                                    const float *__restrict__ data, D dim, int metric,
                                                     uint32_t *rows_read, float ck, uint32_t cv,
                                                     bool wide_first_sort = false) {
     const uint32_t lane = lane_id();
@@ -831,7 +993,7 @@ __device__ __forceinline__ uint32_t beam_loop_lanes(float (&bk)[NB], uint32_t (&
             __syncwarp();
         }
         if (terminate && iter >= p.min_iterations) break;
-        rows += expand_lanes(s, parent, own_id, graph, degree, p.hash_bit, data, dim, metric, ck, cv);
+        rows += expand_lanes<TEAM>(s, parent, own_id, graph, degree, p.hash_bit, data, dim, metric, ck, cv);
         iter++;
     }
     if (rows_read) *rows_read += rows;

@@ -119,7 +119,8 @@ template<> struct Log2<1> { static constexpr int v = 0; };
 // by one lane per row). QR = number of 16-byte chunks each lane owns (dim <= 128*QR).
 template<int QR, typename IdAt, typename Sink>
 __device__ __forceinline__ void warp_rows_v4(const float *q_smem, const float *__restrict__ data, uint32_t dim,
-                                             int metric, uint32_t n, IdAt id_at, Sink sink) {
+                                             int metric, uint32_t n, IdAt id_at, Sink sink, uint32_t first = 0,
+                                             uint32_t step = 8 / QR) {
     constexpr int R = 8 / QR;
     const uint32_t lane = lane_id();
     const uint32_t chunks = dim >> 2;
@@ -129,7 +130,7 @@ __device__ __forceinline__ void warp_rows_v4(const float *q_smem, const float *_
         const uint32_t c = lane + 32u * j;
         q[j] = (c < chunks) ? reinterpret_cast<const float4 *>(q_smem)[c] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    for (uint32_t g = 0; g < n; g += R) {
+    for (uint32_t g = first; g < n; g += step) {
         float4 v[R][QR];
 #pragma unroll
         for (int r = 0; r < R; r++) {
@@ -156,57 +157,107 @@ __device__ __forceinline__ void warp_rows_v4(const float *q_smem, const float *_
     }
 }
 
-// Lane partial sum of one row for any dim. dim % 4 == 0: the chunk ownership of warp_rows_v4;
-// otherwise scalar elements l, l+32, ... (the reference's order).
-__device__ __forceinline__ float lane_row_partial(const float *q_smem, const float *__restrict__ row, uint32_t dim) {
+// Lane partial sums of kWideRows rows of any dim at once. dim % 4 == 0: the chunk ownership of
+// warp_rows_v4 (chunks l, l+32, ... in ascending order); otherwise scalar elements l, l+32, ... (the
+// reference's order). Bound by the latency of the row loads: a warp that reads one row at a time has
+// dim / 128 loads per lane in flight (two at dim 256) and pays a trip to L2 and a five-step fold per row.
+// With four rows there are eight 16-byte loads (or sixteen 4-byte ones) in flight and one fold of eight
+// shuffles for the four; two chunks a step because that is what 64-register kernels hold. A row's own
+// order of sums is the same, so the distances are.
+constexpr int kWideRows = 4;
+
+__device__ __forceinline__ void wide_rows_partial(const float *q_smem, const float *__restrict__ data, uint32_t dim,
+                                                  const uint32_t (&id)[kWideRows], float (&p)[kWideRows]) {
     const uint32_t lane = lane_id();
-    float acc = 0.0f;
+#pragma unroll
+    for (int r = 0; r < kWideRows; r++) p[r] = 0.0f;
     if ((dim & 3u) == 0) {
-        const float4 *q4 = reinterpret_cast<const float4 *>(q_smem);
-        const float4 *r4 = reinterpret_cast<const float4 *>(row);
+        const float4 *q4 = reinterpret_cast<const float4 *>(q_smem), *row[kWideRows];
+#pragma unroll
+        for (int r = 0; r < kWideRows; r++) row[r] = reinterpret_cast<const float4 *>(data + (uint64_t) id[r] * dim);
         const uint32_t chunks = dim >> 2;
-        // eight 16-byte loads in flight per lane (a 960-dim row is 7.5 of them), accumulated in chunk order
-        for (uint32_t c = lane; c < chunks; c += 256) {
-            float4 b[8];
+        for (uint32_t c = lane; c < chunks; c += 64) {
+            const bool two = c + 32u < chunks;
+            float4 v[kWideRows][2];
 #pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const uint32_t ck = c + 32u * k;
-                b[k] = ck < chunks ? __ldg(r4 + ck) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int r = 0; r < kWideRows; r++) {
+                v[r][0] = __ldg(row[r] + c);
+                v[r][1] = two ? __ldg(row[r] + c + 32) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
+            const float4 q0 = q4[c];
 #pragma unroll
-            for (int k = 0; k < 8; k++) {
-                const uint32_t ck = c + 32u * k;
-                if (ck < chunks) acc = sq_acc4(q4[ck], b[k], acc);
+            for (int r = 0; r < kWideRows; r++) p[r] = sq_acc4(q0, v[r][0], p[r]);
+            if (two) {
+                const float4 q1 = q4[c + 32u];
+#pragma unroll
+                for (int r = 0; r < kWideRows; r++) p[r] = sq_acc4(q1, v[r][1], p[r]);
             }
         }
     } else {
-        for (uint32_t i = lane; i < dim; i += 32) {
-            const float d = q_smem[i] - __ldg(row + i);
-            acc = __fmaf_rn(d, d, acc);
+        const float *row[kWideRows];
+#pragma unroll
+        for (int r = 0; r < kWideRows; r++) row[r] = data + (uint64_t) id[r] * dim;
+        for (uint32_t i0 = lane; i0 < dim; i0 += 128) {
+            float v[kWideRows][4];
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+#pragma unroll
+                for (int r = 0; r < kWideRows; r++) v[r][k] = i0 + 32u * k < dim ? __ldg(row[r] + i0 + 32u * k) : 0.0f;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                if (i0 + 32u * k < dim) {
+                    const float q = q_smem[i0 + 32u * k];
+#pragma unroll
+                    for (int r = 0; r < kWideRows; r++) {
+                        const float d = q - v[r][k];
+                        p[r] = __fmaf_rn(d, d, p[r]);
+                    }
+                }
+            }
         }
     }
-    return acc;
 }
 
-// Any dim: one row at a time.
+// Any dim, kWideRows rows at a time; slots past the last row re-read the batch's first one.
 template<typename IdAt, typename Sink>
 __device__ __forceinline__ void warp_rows_generic(const float *q_smem, const float *__restrict__ data, uint32_t dim,
-                                                  int metric, uint32_t n, IdAt id_at, Sink sink) {
+                                                  int metric, uint32_t n, IdAt id_at, Sink sink, uint32_t first = 0,
+                                                  uint32_t step = kWideRows) {
     const uint32_t lane = lane_id();
-    for (uint32_t g = 0; g < n; g++) {
-        float p[1] = {lane_row_partial(q_smem, data + (uint64_t) id_at(g) * dim, dim)};
-        const float sum = fold_rows<1>(p);
-        if (lane == 0) sink(g, metric == kEuclidean ? sqrtf(sum) : sum);
+    for (uint32_t g = first; g < n; g += step) {
+        uint32_t id[kWideRows];
+#pragma unroll
+        for (int r = 0; r < kWideRows; r++) id[r] = id_at(g + r < n ? g + r : g);
+        float p[kWideRows];
+        wide_rows_partial(q_smem, data, dim, id, p);
+        const float sum = fold_rows<kWideRows>(p);   // row r of the batch sits in lanes 8r .. 8r+7
+        const uint32_t my_row = lane >> 3;
+        if ((lane & 7u) == 0 && g + my_row < n) sink(g + my_row, metric == kEuclidean ? sqrtf(sum) : sum);
     }
 }
 
-template<typename IdAt, typename Sink>
-__device__ __forceinline__ void warp_rows(const float *q_smem, const float *__restrict__ data, uint32_t dim, int metric,
+// Rows of at most 128 values, a multiple of four: a 16-byte chunk per lane.
+__host__ __device__ __forceinline__ bool rows_fit_lanes(uint32_t dim) { return (dim & 3u) == 0 && dim <= 128; }
+
+// Search and build kernels are compiled apart for rows that fit the lanes and for the others, by the type of the
+// dim that they hand down: with both forms in one kernel the wide one's registers cost the other its occupancy
+// or spills (10,000 queries of 128 values 621 to 657 us, the large path's 2,785 to 3,042 us), and a call that is
+// not inlined costs both (960 values: search kernel 600 to 1,257 us for one query). A plain uint32_t keeps both.
+template<bool FIT> struct DimOf {
+    uint32_t value;
+    __device__ __forceinline__ operator uint32_t() const { return value; }
+};
+__device__ __forceinline__ bool dim_fits(uint32_t dim) { return rows_fit_lanes(dim); }
+template<bool FIT> __device__ __forceinline__ constexpr bool dim_fits(DimOf<FIT>) { return FIT; }
+// CTAs per SM that a kernel asks for: `wide` for kernels of wide rows, whose four rows in flight spill at 64 registers
+template<typename D> __host__ __device__ constexpr int ctas_per_sm(int others, int) { return others; }
+template<> __host__ __device__ constexpr int ctas_per_sm<DimOf<false>>(int, int wide) { return wide; }
+
+template<typename D, typename IdAt, typename Sink>
+__device__ __forceinline__ void warp_rows(const float *q_smem, const float *__restrict__ data, D dim, int metric,
                                           uint32_t n, IdAt id_at, Sink sink) {
-    // register budget (a third variant pushes the search kernels from 64 to 100 registers):
-    // the query-in-registers path serves dim <= 128, wider rows stream chunk by chunk against
-    // the query in shared memory
-    if ((dim & 3u) == 0 && dim <= 128) warp_rows_v4<1>(q_smem, data, dim, metric, n, id_at, sink);
+    // the query in registers for rows that fit the lanes; wider rows stream against the query in shared memory
+    if (dim_fits(dim)) warp_rows_v4<1>(q_smem, data, dim, metric, n, id_at, sink);
     else warp_rows_generic(q_smem, data, dim, metric, n, id_at, sink);
 }
 
@@ -307,26 +358,34 @@ __device__ __forceinline__ float score_lanes_q4(const float4 q, bool own, const 
     return mine;
 }
 
-__device__ __forceinline__ bool rows_fit_lanes(uint32_t dim) { return (dim & 3u) == 0 && dim <= 128; }
-
-__device__ __forceinline__ float score_lanes(const float *q_smem, const float *__restrict__ data, uint32_t dim,
+template<typename D>
+__device__ __forceinline__ float score_lanes(const float *q_smem, const float *__restrict__ data, D dim,
                                              int metric, uint32_t mask, uint32_t cv, uint32_t *ids_smem = nullptr) {
     const uint32_t lane = lane_id();
-    if (rows_fit_lanes(dim)) {
+    if (dim_fits(dim)) {
         const bool own = lane < (dim >> 2);
         const float4 q = own ? reinterpret_cast<const float4 *>(q_smem)[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
         return score_lanes_q4(q, own, data, dim, metric, mask, cv, ids_smem);
     }
     float mine = FLT_MAX;
     uint32_t m = mask;
-    while (m != 0) {
-        const uint32_t src = (uint32_t) __ffs(m) - 1u;
-        m &= m - 1u;
-        const uint32_t id = __shfl_sync(kFullMask, cv, src);
-        float p[1] = {lane_row_partial(q_smem, data + (uint64_t) id * dim, dim)};
-        const float sum = fold_rows<1>(p);
-        if (lane == src) mine = metric == kEuclidean ? sqrtf(sum) : sum;
+    const uint32_t my_rank = __popc(mask & ((1u << lane) - 1u));
+    const bool valid = ((mask >> lane) & 1u) != 0;
+    for (uint32_t g = 0; m != 0; g++) {
+        uint32_t id[kWideRows];
+#pragma unroll
+        for (int r = 0; r < kWideRows; r++) {   // slots past the last row re-read the batch's first one
+            const uint32_t got = __shfl_sync(kFullMask, cv, m != 0 ? (uint32_t) __ffs(m) - 1u : 0u);
+            id[r] = m != 0 ? got : id[0];
+            m &= m - 1u;
+        }
+        float p[kWideRows];
+        wide_rows_partial(q_smem, data, dim, id, p);
+        const float sum = fold_rows<kWideRows>(p);   // row r of the batch sits in lanes 8r .. 8r+7
+        const float got = __shfl_sync(kFullMask, sum, (my_rank & 3u) * 8u);
+        mine = (valid && (my_rank >> 2) == g) ? got : mine;
     }
+    if (metric == kEuclidean) mine = valid ? sqrtf(mine) : mine;
     return mine;
 }
 

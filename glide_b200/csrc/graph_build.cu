@@ -54,11 +54,11 @@ __device__ __forceinline__ PruneStrip make_prune_strip(uint32_t *extra, uint32_t
 // picks[0..limit) receives pool-relative ids, unused slots kInvalid. Returns rows read;
 // *pool_size = entries that were filled.
 // ---------------------------------------------------------------------------
-template<int NB>
+template<int NB, typename D>
 __device__ __forceinline__ uint32_t prune_lanes(const float (&bk)[NB], const uint32_t (&bv)[NB], uint32_t beam,
                                                 const PruneStrip &ps, float *q_smem, uint32_t *ids_smem,
                                                 const float *__restrict__ data,
-                                                uint32_t dim, uint32_t degree, uint32_t max_degree, uint32_t limit,
+                                                D dim, uint32_t degree, uint32_t max_degree, uint32_t limit,
                                                 float alpha, int metric, bool refine, uint32_t point_id,
                                                 uint32_t *pool_size) {
     const uint32_t lane = lane_id();
@@ -81,7 +81,7 @@ __device__ __forceinline__ uint32_t prune_lanes(const float (&bk)[NB], const uin
     }
     *pool_size = P;
     __syncwarp();
-    const bool fast = rows_fit_lanes(dim);
+    const bool fast = dim_fits(dim);
     const bool own = lane < (dim >> 2);
     uint32_t nsize = 0, rows = 0;
     while (nsize < limit) {
@@ -193,8 +193,8 @@ __device__ __forceinline__ void boundary_merge(const PruneStrip &ps, const uint3
 
 // LANES: adjacency rows searched have at most 32 entries; candidates stay in registers
 // (beam_loop_lanes) and the strip holds no candidate arrays.
-template<int NB, int NC, bool LANES>
-__global__ void __launch_bounds__(256, NB <= 4 ? 4 : 2) build_kernel(const BuildDev d) {
+template<int NB, int NC, bool LANES, typename D>
+__global__ void __launch_bounds__(256, NB <= 4 ? ctas_per_sm<D>(4, 3) : 2) build_kernel(const BuildDev d) {
     extern __shared__ __align__(16) uint32_t smem[];
     const BuildArgs &a = d.a;
     const uint32_t warps_per_cta = blockDim.x >> 5;
@@ -207,6 +207,7 @@ __global__ void __launch_bounds__(256, NB <= 4 ? 4 : 2) build_kernel(const Build
     if constexpr (NB == 16) s.tail = smem + (size_t) (warp + 1) * d.strip_words - kTwoWarpScratch;
     PruneStrip ps = make_prune_strip(s.extra, d.max_degree);
     const uint32_t degree = a.out_degree;
+    const D dim{a.dim};
 
     uint32_t rows = 0, prune_rows = 0, iters = 0;
     bool short_pool = false;
@@ -238,17 +239,17 @@ __global__ void __launch_bounds__(256, NB <= 4 ? 4 : 2) build_kernel(const Build
         if constexpr (LANES) {
             float ck;
             uint32_t cv;
-            rows += seed_lanes(s, a.start_points[seg], point, pknn, a.in_degree, p.hash_bit, pdata, a.dim, a.metric, ck, cv,
+            rows += seed_lanes(s, a.start_points[seg], point, pknn, a.in_degree, p.hash_bit, pdata, dim, a.metric, ck, cv,
                                &wide);
-            iters = beam_loop_lanes<NB>(bk, bv, s, p, point - seg_start, pknn, a.in_degree, pdata, a.dim, a.metric, &rows,
+            iters = beam_loop_lanes<NB>(bk, bv, s, p, point - seg_start, pknn, a.in_degree, pdata, dim, a.metric, &rows,
                                         ck, cv, wide);
         } else {
-            rows += seed_from_row(s, a.start_points[seg], point, pknn, a.in_degree, p.hash_bit, pdata, a.dim, a.metric, &wide);
-            iters = beam_loop<NB, NC, true>(bk, bv, s, p, point - seg_start, pknn, a.in_degree, pdata, a.dim, a.metric, &rows,
+            rows += seed_from_row(s, a.start_points[seg], point, pknn, a.in_degree, p.hash_bit, pdata, dim, a.metric, &wide);
+            iters = beam_loop<NB, NC, true>(bk, bv, s, p, point - seg_start, pknn, a.in_degree, pdata, dim, a.metric, &rows,
                                             wide);
         }
         uint32_t P;
-        prune_rows = prune_lanes<NB>(bk, bv, p.beam, ps, s.query, LANES ? s.cand_id : nullptr, pdata, a.dim, degree, d.max_degree, degree, a.alpha, a.metric,
+        prune_rows = prune_lanes<NB>(bk, bv, p.beam, ps, s.query, LANES ? s.cand_id : nullptr, pdata, dim, degree, d.max_degree, degree, a.alpha, a.metric,
                                      false, kInvalid, &P);
         short_pool = P < p.beam;
         const uint32_t orig = a.map ? a.map[point] : point;
@@ -300,14 +301,14 @@ __global__ void __launch_bounds__(256, NB <= 4 ? 4 : 2) build_kernel(const Build
         if constexpr (LANES) {
             float ck;
             uint32_t cv;
-            rows += seed_lanes(s, start, exclude, a.graph_in, degree, p.hash_bit, a.data, a.dim, a.metric, ck, cv, &wide);
-            iters = beam_loop_lanes<NB>(bk, bv, s, p, point, a.graph_in, degree, a.data, a.dim, a.metric, &rows, ck, cv, wide);
+            rows += seed_lanes(s, start, exclude, a.graph_in, degree, p.hash_bit, a.data, dim, a.metric, ck, cv, &wide);
+            iters = beam_loop_lanes<NB>(bk, bv, s, p, point, a.graph_in, degree, a.data, dim, a.metric, &rows, ck, cv, wide);
         } else {
-            rows += seed_from_row(s, start, exclude, a.graph_in, degree, p.hash_bit, a.data, a.dim, a.metric, &wide);
-            iters = beam_loop<NB, NC, true>(bk, bv, s, p, point, a.graph_in, degree, a.data, a.dim, a.metric, &rows, wide);
+            rows += seed_from_row(s, start, exclude, a.graph_in, degree, p.hash_bit, a.data, dim, a.metric, &wide);
+            iters = beam_loop<NB, NC, true>(bk, bv, s, p, point, a.graph_in, degree, a.data, dim, a.metric, &rows, wide);
         }
         uint32_t P;
-        prune_rows = prune_lanes<NB>(bk, bv, p.beam, ps, s.query, LANES ? s.cand_id : nullptr, a.data, a.dim, degree, d.max_degree, need, a.alpha, a.metric,
+        prune_rows = prune_lanes<NB>(bk, bv, p.beam, ps, s.query, LANES ? s.cand_id : nullptr, a.data, dim, degree, d.max_degree, need, a.alpha, a.metric,
                                      true, point, &P);
         short_pool = P < p.beam;
         uint32_t pos_num = 0;  // :660-671: holes, front to back
@@ -335,7 +336,9 @@ uint32_t pow2_at_least(uint32_t x, uint32_t lo) {
 
 template<int NB, int NC, bool LANES = false>
 cudaError_t launch_build_t(const BuildDev &d, uint32_t warps_per_cta, size_t smem_bytes, cudaStream_t stream) {
-    auto kernel = build_kernel<NB, NC, LANES>;
+    void (*kernel)(const BuildDev);
+    if constexpr (NC == 2) kernel = rows_fit_lanes(d.a.dim) ? build_kernel<NB, NC, LANES, DimOf<true>> : build_kernel<NB, NC, LANES, DimOf<false>>;
+    else kernel = build_kernel<NB, NC, LANES, uint32_t>;   // adjacency rows above 64 entries
     if (smem_bytes > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem_bytes);
         if (e != cudaSuccess) return e;
@@ -575,10 +578,10 @@ cudaError_t launch_build(const BuildArgs &a, cudaStream_t stream) {
 // find no work (count = 0: every warp returns at once).
 cudaError_t preload_build_kernels(cudaStream_t stream) {
     BuildDev d{};
-    build_kernel<2, 2, true><<<1, 32, 0, stream>>>(d);
-    build_kernel<4, 2, true><<<1, 32, 0, stream>>>(d);
-    build_kernel<2, 2, false><<<1, 32, 0, stream>>>(d);
-    build_kernel<4, 2, false><<<1, 32, 0, stream>>>(d);
+    build_kernel<2, 2, true, DimOf<true>><<<1, 32, 0, stream>>>(d);
+    build_kernel<4, 2, true, DimOf<true>><<<1, 32, 0, stream>>>(d);
+    build_kernel<2, 2, false, DimOf<false>><<<1, 32, 0, stream>>>(d);
+    build_kernel<4, 2, false, DimOf<false>><<<1, 32, 0, stream>>>(d);
     return cudaGetLastError();
 }
 
