@@ -578,9 +578,17 @@ int glide_bruteforce_knn(glide_ctx *ctx, const float *d_base, uint32_t n, const 
     GL_REQUIRE(ctx, k >= 1 && k <= 128 && k <= n, GLIDE_ERR_UNSUPPORTED, "bruteforce_knn: k must be in [1, min(128, n)]");
     GL_CUDA(ctx, cudaSetDevice(ctx->device));
     const uint32_t splits = bruteforce_default_splits(n, q);
-    int rc = ensure_ws(ctx, bruteforce_scratch_bytes(q, k, splits) + 256);
+    const bool tc = q > 0 && truth_tc_eligible(n, q, dim, k);
+    size_t need = bruteforce_scratch_bytes(q, k, splits) + 256;
+    if (tc) need = std::max(need, truth_tc_scratch_bytes(d_base, d_queries, n, q, dim, k));
+    int rc = ensure_ws(ctx, need);
     if (rc) return rc;
     Timed timer(ctx);
+    if (tc) {
+        uint32_t failed = 1;
+        GL_CUDA(ctx, launch_truth_tc(d_base, n, d_queries, q, dim, k, metric, ctx->ws, d_out_ids, d_out_dists, &failed, ctx->stream));
+        if (!failed) return timer.finish();
+    }
     GL_CUDA(ctx, launch_bruteforce(d_base, n, d_queries, q, dim, k, metric, splits, ctx->ws, d_out_ids, d_out_dists, ctx->stream));
     return timer.finish();
 }

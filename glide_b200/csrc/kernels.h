@@ -172,6 +172,11 @@ cudaError_t launch_count_changed(const uint32_t *a, const uint32_t *b, uint32_t 
 // ---- bruteforce.cu -------------------------------------------------------
 size_t bruteforce_scratch_bytes(uint32_t Q, uint32_t k, uint32_t splits);
 uint32_t bruteforce_default_splits(uint32_t n, uint32_t Q);
+// The same results from the tensor cores' candidates (truth_tc.cu); *h_failed != 0: use launch_bruteforce.
+bool truth_tc_eligible(uint32_t n, uint32_t Q, uint32_t dim, uint32_t k);
+size_t truth_tc_scratch_bytes(const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k);
+cudaError_t launch_truth_tc(const float *base, uint32_t n, const float *queries, uint32_t Q, uint32_t dim, uint32_t k, int metric, void *scratch,
+                            uint32_t *out_ids, float *out_dists, uint32_t *h_failed, cudaStream_t stream);
 cudaError_t launch_bruteforce(const float *base, uint32_t n, const float *queries, uint32_t Q, uint32_t dim,
                               uint32_t k, int metric, uint32_t splits, void *scratch, uint32_t *out_ids,
                               float *out_dists, cudaStream_t stream);

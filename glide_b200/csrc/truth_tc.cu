@@ -1,0 +1,528 @@
+// Exact brute-force kNN on the tensor cores: ground truth for large query or base sets. What comes out is
+// what bruteforce_tile_kernel gives bit for bit: the tensor cores only decide which rows are looked at.
+//
+//   norms      |b|^2 of every base row, and the largest |b| and |b - tf32(b)|.
+//   contract   a CTA owns 128 queries and every slices-th tile of 128 base rows. Operand blocks of 32 values
+//              arrive by TMA (128-byte swizzle) into a ring of shared-memory stages; the queries' blocks stay
+//              in shared memory where they fit (up to 256 values a row), otherwise they ride along with the
+//              rows'. tcgen05.mma kind::tf32 accumulates the 128 x 128 dot products in tensor memory (two
+//              buffers), sixteen epilogue warps turn them into a = |b|^2 - 2 q.b (thread (query, part): 32 columns).
+//   threshold  a pass over every stride-th tile keeps the minima of runs of columns; the k-th smallest of
+//              them, t, is an upper bound of the k-th smallest a. The true k nearest then have a <= t + 2E, where E
+//              bounds |a + |q|^2 - d| for the fp32 distance d (tf32 rounding by Cauchy's inequality from the
+//              norms of what it drops, which is nothing for integers below 2048; sums by their length).
+//   select     the pass over all tiles stores every column with a <= t + 2E.
+//   re-rank    their fp32 distances in the order of bruteforce_tile_kernel, sorted by (distance, id).
+//
+// A query with more candidates than its buffer holds (or fewer than k), a value that is no finite number, a tensor map
+// that cannot be made or a wait that runs out makes the caller fall back to bruteforce_tile_kernel.
+// Bound by the tensor pipe and, below it, by the trip of the row tiles from L2 (once per 128 queries).
+// bruteforce_tile_kernel against this: 1M x 128 rows, 1,000 queries, k = 10: 22.5 to 1.14 ms (0.22 of measured bf16
+// peak is what tf32 gives at best: 0.36 ms of it), k = 100: 39.1 to 2.29 ms; 100,000 x 960, 333 queries 6.5 to 0.55 ms;
+// 1M x 64, 10 queries 1.79 to 0.28 ms; 4,000 x 32, 10 queries 122 to 71 us. Where the norms are far above the distances
+// (values around 1,000, spread 1) nearly every row is a candidate and the attempt is lost: 0.39 to 0.81 ms at 50,000 x 64.
+#include "common.cuh"
+#include "kernels.h"
+#include "umma.cuh"
+
+namespace glide {
+
+namespace {
+
+using namespace umma;
+
+constexpr uint32_t kTile = 128;              // queries per CTA, base rows per tile
+constexpr uint32_t kBlock = 32;              // values of a row per operand block
+constexpr uint32_t kBlockBytes = kTile * kBlock * 4;
+constexpr uint32_t kParts = 4;               // epilogue threads per query
+constexpr uint32_t kEpi = 4 * kParts;        // epilogue warps
+constexpr uint32_t kTruthThreads = (kEpi + 2) * 32;
+constexpr uint32_t kResidentBlocks = 8;      // query blocks kept in shared memory
+constexpr uint32_t kCap = 3968;              // candidates per query; with up to 128 earlier results 4,096 sort keys
+constexpr uint32_t kBaseRows = 1u << 21;     // base rows per pass (bounds the scratch)
+constexpr uint32_t kQueryRows = 8192;        // queries per pass
+
+struct TruthStats {
+    uint32_t max_norm, max_rest;             // bits of the largest |b|^2 and |b - tf32(b)|^2 (non-negative floats order as integers)
+    uint32_t failed;
+    uint32_t pad;
+};
+
+struct TruthArgs {
+    uint32_t n, Q, dim, kblocks, stages;
+    uint32_t slices, stride;                 // CTA (query tile, slice) takes sampled tiles slice, slice + slices, ...; tile = index * stride
+    uint32_t group, groups;                  // columns per minimum, minima per query (sample pass)
+    bool sample;
+    const float *norms;
+    const float *thr;                        // per query (select pass)
+    float *gmin;                             // Q x groups
+    uint32_t *count;                         // per query
+    uint32_t *cand;                          // Q x kCap
+    TruthStats *stats;
+};
+
+__device__ __forceinline__ float tf32_rest(float x) { return x - __uint_as_float(__float_as_uint(x) & 0xffffe000u); }
+
+// A warp per row: |x|^2, |x - tf32(x)|^2 (two floats per row if `rest` is given), the maxima, and the row padded to `pitch`.
+__global__ void truth_rows_kernel(const float *__restrict__ data, uint32_t rows, uint32_t dim, float *norms, float *rest, uint32_t pitch,
+                                  float *padded, TruthStats *stats) {
+    __shared__ uint32_t top[2];
+    if (threadIdx.x < 2) top[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t lane = lane_id(), warps = blockDim.x >> 5;
+    uint32_t best_n = 0, best_r = 0;
+    for (uint64_t r = (uint64_t) blockIdx.x * warps + (threadIdx.x >> 5); r < rows; r += (uint64_t) gridDim.x * warps) {
+        const float *row = data + r * dim;
+        float s = 0.0f, t = 0.0f;
+        if (padded == nullptr) {
+            const float4 *row4 = reinterpret_cast<const float4 *>(row);   // dim % 4 == 0 and aligned, or a padded copy would be wanted
+            for (uint32_t k = lane; k < (dim >> 2); k += 32) {
+                const float4 v = __ldg(row4 + k);
+                const float4 l = make_float4(tf32_rest(v.x), tf32_rest(v.y), tf32_rest(v.z), tf32_rest(v.w));
+                s += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+                t += l.x * l.x + l.y * l.y + l.z * l.z + l.w * l.w;
+            }
+        } else {
+            for (uint32_t k = lane; k < pitch; k += 32) {
+                const float v = k < dim ? __ldg(row + k) : 0.0f, l = tf32_rest(v);
+                padded[r * pitch + k] = v;
+                s += v * v;
+                t += l * l;
+            }
+        }
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) {
+            s += __shfl_xor_sync(kFullMask, s, off);
+            t += __shfl_xor_sync(kFullMask, t, off);
+        }
+        if (lane == 0) {
+            norms[r] = s;
+            if (rest) rest[r] = t;
+        }
+        best_n = max(best_n, __float_as_uint(s));   // a NaN or an infinity is larger than any number and is caught with it
+        best_r = max(best_r, __float_as_uint(fabsf(t)));
+    }
+    if (lane == 0) {
+        atomicMax(&top[0], best_n);
+        atomicMax(&top[1], best_r);
+    }
+    __syncthreads();
+    if (stats && threadIdx.x == 0) {
+        atomicMax(&stats->max_norm, top[0]);
+        atomicMax(&stats->max_rest, top[1]);
+    }
+}
+
+template<int GS>
+__device__ __forceinline__ void run_minima(const float (&e)[32], float *out) {
+    float m = FLT_MAX;
+#pragma unroll
+    for (int j = 0; j < 32; j++) {
+        m = fminf(m, e[j]);
+        if ((j + 1) % GS == 0) {
+            out[j / GS] = m;
+            m = FLT_MAX;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthArgs a, const __grid_constant__ CUtensorMap tm_q,
+                                                                   const __grid_constant__ CUtensorMap tm_b) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t) 1023);
+    const uint32_t kblocks = a.kblocks, stages = a.stages;
+    const bool resident = kblocks <= kResidentBlocks;
+    const uint32_t stage_bytes = resident ? kBlockBytes : 2 * kBlockBytes;   // a block of rows, then one of queries
+    uint8_t *As = base, *ring = base + (resident ? kblocks * kBlockBytes : 0u);
+    float *cn_w = reinterpret_cast<float *>(ring + stages * stage_bytes);     // a warp's column norms
+    uint64_t *bars = reinterpret_cast<uint64_t *>(cn_w + kEpi * 32);
+    uint64_t *a_full = bars, *full = bars + 1, *freed = full + stages, *mma_done = freed + stages, *tmem_free = mma_done + 2;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_free + 2);
+    volatile uint32_t *failed = tmem_slot + 1;
+
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t qtiles = (a.Q + kTile - 1) / kTile;
+    const uint32_t q0 = (blockIdx.x % qtiles) * kTile, slice = blockIdx.x / qtiles;
+    const uint32_t all = (a.n + kTile - 1) / kTile, taken = (all + a.stride - 1) / a.stride;
+    const uint32_t tiles = slice < taken ? (taken - slice + a.slices - 1) / a.slices : 0u;   // of this CTA
+
+    if (tid == 0) {
+        mbar_init(a_full, 1);
+        for (uint32_t s = 0; s < stages; s++) { mbar_init(full + s, 1); mbar_init(freed + s, 1); }
+        for (int c = 0; c < 2; c++) { mbar_init(mma_done + c, 1); mbar_init(tmem_free + c, kEpi); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        *failed = 0;
+    }
+    if (warp == kEpi) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2 * kTile) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == kEpi + 1) {
+        // ================= copies: one thread =================
+        if (lane == 0 && tiles > 0) {
+            if (resident) {
+                mbar_expect_tx(a_full, kblocks * kBlockBytes);
+                for (uint32_t kb = 0; kb < kblocks; kb++) tma_load_2d(As + kb * kBlockBytes, &tm_q, kb * kBlock, q0, a_full);
+            }
+            uint32_t s = 0, use = 0;
+            bool ok = true;
+            for (uint32_t t = 0; t < tiles && ok; t++) {
+                const uint32_t row0 = (slice + t * a.slices) * a.stride * kTile;
+                for (uint32_t kb = 0; kb < kblocks; kb++) {
+                    if (use > 0 && !mbar_wait(freed + s, (use - 1) & 1u, failed)) { ok = false; break; }
+                    uint8_t *dst = ring + s * stage_bytes;
+                    mbar_expect_tx(full + s, stage_bytes);
+                    tma_load_2d(dst, &tm_b, kb * kBlock, row0, full + s);
+                    if (!resident) tma_load_2d(dst + kBlockBytes, &tm_q, kb * kBlock, q0, full + s);
+                    if (++s == stages) { s = 0; use++; }
+                }
+            }
+        }
+    } else if (warp == kEpi) {
+        // ================= MMAs: one thread =================
+        if (lane == 0 && tiles > 0) {
+            const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((kTile >> 3) << 17) | ((kTile >> 4) << 24);
+            const uint32_t a_addr = smem_u32(As), r_addr = smem_u32(ring);
+            bool ok = !resident || mbar_wait(a_full, 0, failed);
+            uint32_t s = 0, use = 0;
+            for (uint32_t t = 0; t < tiles && ok; t++) {
+                const uint32_t acc = t & 1u;
+                if (t >= 2) ok = mbar_wait(tmem_free + acc, ((t >> 1) - 1) & 1u, failed);
+                for (uint32_t kb = 0; kb < kblocks && ok; kb++) {
+                    ok = mbar_wait(full + s, use & 1u, failed);
+                    if (!ok) break;
+                    fence_after();
+                    const uint32_t b = r_addr + s * stage_bytes, q = resident ? a_addr + kb * kBlockBytes : b + kBlockBytes;
+#pragma unroll
+                    for (uint32_t k = 0; k < kBlock / 8; k++)
+                        mma_tf32(tmem_base + acc * kTile, desc_sw128(q + k * 32u), desc_sw128(b + k * 32u), idesc, kb + k > 0 ? 1u : 0u);
+                    commit_to(freed + s);
+                    if (++s == stages) { s = 0; use++; }
+                }
+                if (ok) commit_to(mma_done + acc);
+            }
+        }
+    } else {
+        // ================= epilogue: thread (query, part) owns 32 columns of every tile =================
+        const uint32_t quad = warp & 3u, part = warp >> 2, q = q0 + quad * 32u + lane;
+        const bool active = q < a.Q;
+        const float thr = (active && !a.sample) ? __ldg(a.thr + q) : 0.0f;
+        float *cn = cn_w + warp * 32u;
+        auto norm_of = [&](uint32_t t) {
+            const uint32_t c = (slice + t * a.slices) * a.stride * kTile + part * 32u + lane;
+            return t < tiles && c < a.n ? __ldg(a.norms + c) : 0.0f;
+        };
+        float ahead = norm_of(0);
+        for (uint32_t t = 0; t < tiles; t++) {
+            __syncwarp();
+            cn[lane] = ahead;
+            ahead = norm_of(t + 1);
+            __syncwarp();
+            const uint32_t acc = t & 1u, index = slice + t * a.slices, c0 = index * a.stride * kTile + part * 32u;
+            bool ok = !*failed && mbar_wait(mma_done + acc, (t >> 1) & 1u, failed);
+            ok = __all_sync(kFullMask, ok);
+            if (!ok) break;
+            fence_after();
+            uint32_t r[32];
+            tmem_load32(tmem_base + ((quad * 32u) << 16) + acc * kTile + part * 32u, r);
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tmem_free + acc);
+            float e[32];
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+                const float4 c4 = *reinterpret_cast<const float4 *>(cn + j);
+                e[j] = __fmaf_rn(-2.0f, __uint_as_float(r[j]), c4.x);
+                e[j + 1] = __fmaf_rn(-2.0f, __uint_as_float(r[j + 1]), c4.y);
+                e[j + 2] = __fmaf_rn(-2.0f, __uint_as_float(r[j + 2]), c4.z);
+                e[j + 3] = __fmaf_rn(-2.0f, __uint_as_float(r[j + 3]), c4.w);
+            }
+            if (c0 + 32u > a.n) {
+#pragma unroll
+                for (int j = 0; j < 32; j++)
+                    if (c0 + j >= a.n) e[j] = FLT_MAX;
+            }
+            if (!active) continue;
+            if (a.sample) {
+                float *out = a.gmin + (uint64_t) q * a.groups + (index * kTile + part * 32u) / a.group;
+                switch (a.group) {
+                    case 1: run_minima<1>(e, out); break;
+                    case 2: run_minima<2>(e, out); break;
+                    case 4: run_minima<4>(e, out); break;
+                    case 8: run_minima<8>(e, out); break;
+                    case 16: run_minima<16>(e, out); break;
+                    default: run_minima<32>(e, out); break;
+                }
+            } else {
+                float m = e[0];
+#pragma unroll
+                for (int j = 1; j < 32; j++) m = fminf(m, e[j]);
+                if (m <= thr) {   // rare
+#pragma unroll
+                    for (int j = 0; j < 32; j++) {
+                        if (e[j] <= thr && c0 + j < a.n) {
+                            const uint32_t at = atomicAdd(a.count + q, 1u);
+                            if (at < kCap) a.cand[(uint64_t) q * kCap + at] = c0 + j;
+                        }
+                    }
+                }
+            }
+        }
+        if (*failed && lane == 0) atomicExch(&a.stats->failed, 1u);
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == kEpi) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * kTile) : "memory");
+}
+
+__device__ __forceinline__ uint32_t ordered(float x) {   // ascending floats as ascending integers
+    const uint32_t u = __float_as_uint(x);
+    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ float from_ordered(uint32_t o) { return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o); }
+
+// A CTA per query: the k-th smallest of its group minima (or, on later base passes, its k-th result so far) plus the error
+// bounds. Also clears the query's candidate counter.
+__global__ void __launch_bounds__(128) truth_threshold_kernel(const float *__restrict__ gmin, uint32_t groups, uint32_t k, const u64 *__restrict__ best,
+                                                              const float *__restrict__ q_norm, const float *__restrict__ q_rest, uint32_t dim,
+                                                              TruthStats *stats, float *thr, uint32_t *count) {
+    extern __shared__ uint32_t keys[];
+    __shared__ uint32_t below;
+    const uint32_t q = blockIdx.x, tid = threadIdx.x;
+    float kth;
+    if (best == nullptr) {
+        for (uint32_t i = tid; i < groups; i += 128) keys[i] = ordered(gmin[(uint64_t) q * groups + i]);
+        uint32_t lo = 0, hi = 0xffffffffu;   // smallest key with at least k keys at or below it
+        while (lo < hi) {
+            const uint32_t mid = lo + ((hi - lo) >> 1);
+            if (tid == 0) below = 0;
+            __syncthreads();
+            uint32_t c = 0;
+            for (uint32_t i = tid; i < groups; i += 128) c += keys[i] <= mid ? 1u : 0u;
+            c = __reduce_add_sync(kFullMask, c);
+            if ((tid & 31u) == 0) atomicAdd(&below, c);
+            __syncthreads();
+            if (below >= k) hi = mid; else lo = mid + 1;
+            __syncthreads();
+        }
+        kth = from_ordered(lo);
+    } else {
+        kth = __uint_as_float((uint32_t) (best[(uint64_t) q * k + k - 1] >> 32)) - q_norm[q];
+    }
+    if (tid != 0) return;
+    const float qn = sqrtf(q_norm[q]), ql = sqrtf(q_rest[q]);
+    const float bn = sqrtf(__uint_as_float(stats->max_norm)), bl = sqrtf(__uint_as_float(stats->max_rest));
+    // |2 q.b - 2 tf32(q).tf32(b)| <= 2 (|q| |b - tf32(b)| + |q - tf32(q)| |b|); every sum (the two norms, the MMA's, the
+    // fp32 distance) is within dim + 8 steps of 2^-23 of its terms' magnitudes, all below (|q| + |b|)^2
+    const float sums = (float) (dim + 64u) * 4.0f * 1.1920929e-7f * (qn + bn) * (qn + bn);
+    const float E = 1.001f * 2.0f * (qn * bl + ql * bn) + sums + 1e-30f;
+    const float t = kth + 2.0f * E;
+    if (!(fabsf(t) < FLT_MAX) || !(bn < 1e18f) || !(qn < 1e18f)) atomicExch(&stats->failed, 1u);
+    thr[q] = t;
+    count[q] = 0;
+}
+
+// A CTA per query: exact distances of the candidates (and the earlier passes' results), sorted by (distance, id).
+__global__ void __launch_bounds__(128) truth_rerank_kernel(const float *__restrict__ base, uint32_t first_row, const float *__restrict__ queries, uint32_t dim,
+                                                           const uint32_t *__restrict__ cand, const uint32_t *__restrict__ count, uint32_t k, u64 *best,
+                                                           bool earlier, int metric, uint32_t *out_ids, float *out_dists, TruthStats *stats) {
+    extern __shared__ __align__(16) uint32_t smem[];
+    u64 *keys = reinterpret_cast<u64 *>(smem);                      // 4096
+    float *query = reinterpret_cast<float *>(keys + 4096);          // dim
+    const uint32_t q = blockIdx.x, tid = threadIdx.x;
+    const uint32_t found = count[q], n = min(found, kCap);
+    const uint32_t total = n + (earlier ? k : 0u);
+    if (tid == 0 && (found > kCap || total < k)) atomicExch(&stats->failed, 1u);
+    for (uint32_t d = tid; d < dim; d += 128) query[d] = queries[(uint64_t) q * dim + d];
+    __syncthreads();
+    const bool vec = (dim & 3u) == 0 && (reinterpret_cast<uintptr_t>(base) & 15u) == 0;
+    for (uint32_t i = tid; i < n; i += 128) {
+        const uint32_t id = first_row + cand[(uint64_t) q * kCap + i];
+        const float *row = base + (uint64_t) id * dim;
+        float acc = 0.0f;   // ascending dimensions, one fused multiply-add each: the order of bruteforce_tile_kernel
+        if (vec) {
+#pragma unroll 8
+            for (uint32_t d = 0; d < dim; d += 4) {
+                const float4 b = __ldg(reinterpret_cast<const float4 *>(row + d));
+                const float4 x = *reinterpret_cast<const float4 *>(query + d);
+                const float dx = x.x - b.x, dy = x.y - b.y, dz = x.z - b.z, dw = x.w - b.w;
+                acc = __fmaf_rn(dx, dx, acc);
+                acc = __fmaf_rn(dy, dy, acc);
+                acc = __fmaf_rn(dz, dz, acc);
+                acc = __fmaf_rn(dw, dw, acc);
+            }
+        } else {
+#pragma unroll 8
+            for (uint32_t d = 0; d < dim; d++) {
+                const float df = query[d] - __ldg(row + d);
+                acc = __fmaf_rn(df, df, acc);
+            }
+        }
+        keys[i] = ((u64) __float_as_uint(acc) << 32) | id;
+    }
+    if (earlier)
+        for (uint32_t i = tid; i < k; i += 128) keys[n + i] = best[(uint64_t) q * k + i];
+    uint32_t size = 1;
+    while (size < total) size <<= 1;
+    for (uint32_t i = total + tid; i < size; i += 128) keys[i] = ~0ull;
+    for (uint32_t span = 2; span <= size; span <<= 1)
+        for (uint32_t step = span >> 1; step >= 1; step >>= 1) {
+            __syncthreads();
+            for (uint32_t p = tid; p < size / 2; p += 128) {
+                const uint32_t i = 2 * (p & ~(step - 1u)) + (p & (step - 1u)), j = i + step;
+                const u64 x = keys[i], y = keys[j];
+                if ((x > y) == ((i & span) == 0)) { keys[i] = y; keys[j] = x; }
+            }
+        }
+    __syncthreads();
+    for (uint32_t i = tid; i < k && i < total; i += 128) {
+        best[(uint64_t) q * k + i] = keys[i];
+        if (out_ids) out_ids[(uint64_t) q * k + i] = (uint32_t) keys[i];
+        if (out_dists) out_dists[(uint64_t) q * k + i] = finish_metric(__uint_as_float((uint32_t) (keys[i] >> 32)), metric);
+    }
+}
+
+size_t up256(size_t x) { return (x + 255) & ~(size_t) 255; }
+
+// The sample of a pass over n rows for k neighbours: every stride-th tile, minima over `group` columns. The select
+// pass lets about stride x k columns through, the sample costs 1 / stride of it: 16 where at least 64 k rows remain,
+// less for smaller sets; groups as wide as leaves 8 k of them, so that few of the k smallest share one.
+struct Sample {
+    uint32_t stride, group, groups;
+};
+Sample sample_of(uint32_t n, uint32_t k) {
+    Sample s;
+    s.stride = n / (64u * k);
+    s.stride = s.stride < 1 ? 1 : (s.stride > 16 ? 16 : s.stride);
+    const uint32_t tiles = (n + kTile - 1) / kTile, taken = (tiles + s.stride - 1) / s.stride;
+    s.group = 32;
+    while (s.group > 1 && taken * kTile / s.group < 8u * k) s.group >>= 1;
+    s.groups = taken * (kTile / s.group);
+    return s;
+}
+
+struct TruthPlan {
+    uint32_t nb, qb, pitch;     // rows and queries per pass, padded row length
+    bool pad;
+    Sample sample;
+    size_t norms, rows, q_rows, q_norm, q_rest, thr, count, cand, gmin, best, stats, total;
+};
+
+TruthPlan truth_plan(const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k) {
+    TruthPlan p;
+    p.pad = (dim & 3u) != 0 || ((reinterpret_cast<uintptr_t>(base) | reinterpret_cast<uintptr_t>(queries)) & 15u) != 0;
+    p.pitch = (dim + 3u) & ~3u;
+    p.nb = n < kBaseRows ? n : kBaseRows;
+    if (p.pad && (uint64_t) p.nb * p.pitch > (1u << 28)) p.nb = (1u << 28) / p.pitch;   // a padded copy of 1 GB at most
+    p.nb = (p.nb + 3u) & ~3u;
+    p.qb = Q < kQueryRows ? Q : kQueryRows;
+    p.sample = sample_of(p.nb < n ? p.nb : n, k);
+    size_t at = 0;
+    auto take = [&](size_t bytes) { const size_t o = at; at += up256(bytes); return o; };
+    p.stats = take(sizeof(TruthStats));
+    p.norms = take((size_t) p.nb * 4);
+    p.q_norm = take((size_t) p.qb * 4);
+    p.q_rest = take((size_t) p.qb * 4);
+    p.thr = take((size_t) p.qb * 4);
+    p.count = take((size_t) p.qb * 4);
+    p.cand = take((size_t) p.qb * kCap * 4);
+    p.gmin = take((size_t) p.qb * p.sample.groups * 4);
+    p.best = take((size_t) p.qb * k * 8);
+    p.rows = take(p.pad ? (size_t) p.nb * p.pitch * 4 : 0);
+    p.q_rows = take(p.pad ? (size_t) p.qb * p.pitch * 4 : 0);
+    p.total = at;
+    return p;
+}
+
+// row-major rows of `pitch` floats as TMA boxes of 32 values x 128 rows (make_row_map takes the row length as the pitch)
+bool row_map(CUtensorMap *tm, const float *ptr, uint32_t rows, uint32_t pitch) { return make_row_map(tm, ptr, rows, pitch, kTile); }
+
+}  // namespace
+
+// Below 2^20 products of values a dozen launches cost what the tiles do (the smallest size timed is 1.3 x 2^20: 122 to 71 us).
+bool truth_tc_eligible(uint32_t n, uint32_t Q, uint32_t dim, uint32_t k) {
+    return dim >= 16 && dim <= 4096 && k >= 1 && k <= 128 && n >= 1 && (uint64_t) n * Q * dim >= (1ull << 20) && encode_tiled_fn() != nullptr;
+}
+
+size_t truth_tc_scratch_bytes(const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k) {
+    return truth_plan(base, queries, n, Q, dim, k).total;
+}
+
+// *h_failed != 0: the caller computes the results by other means. Synchronises the stream.
+cudaError_t launch_truth_tc(const float *base, uint32_t n, const float *queries, uint32_t Q, uint32_t dim, uint32_t k, int metric, void *scratch,
+                            uint32_t *out_ids, float *out_dists, uint32_t *h_failed, cudaStream_t stream) {
+    const TruthPlan p = truth_plan(base, queries, n, Q, dim, k);
+    char *w = static_cast<char *>(scratch);
+    auto at = [&](size_t o) { return reinterpret_cast<float *>(w + o); };
+    TruthStats *stats = reinterpret_cast<TruthStats *>(w + p.stats);
+    float *norms = at(p.norms), *q_norm = at(p.q_norm), *q_rest = at(p.q_rest), *thr = at(p.thr), *gmin = at(p.gmin);
+    uint32_t *count = reinterpret_cast<uint32_t *>(w + p.count), *cand = reinterpret_cast<uint32_t *>(w + p.cand);
+    u64 *best = reinterpret_cast<u64 *>(w + p.best);
+    *h_failed = 1;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaMemsetAsync(stats, 0, sizeof(TruthStats), stream);
+    if (e != cudaSuccess) return e;
+
+    TruthArgs a{};
+    a.dim = dim; a.kblocks = (p.pitch + kBlock - 1) / kBlock;
+    const bool resident = a.kblocks <= kResidentBlocks;
+    a.stages = resident ? 12u - a.kblocks : 6u;    // 192 KB of operand blocks
+    a.norms = norms; a.thr = thr; a.gmin = gmin; a.count = count; a.cand = cand; a.stats = stats;
+    const size_t smem = 1024 + 12u * (size_t) kBlockBytes + kEpi * 32 * 4 + (1 + 2 * a.stages + 4) * 8 + 16;
+    if ((e = cudaFuncSetAttribute(truth_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
+    const size_t rr_smem = 4096 * 8 + (size_t) p.pitch * 4;
+    if (rr_smem > 48 * 1024 && (e = cudaFuncSetAttribute(truth_rerank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) rr_smem)) != cudaSuccess) return e;
+
+    for (uint32_t qa = 0; qa < Q; qa += p.qb) {
+        const uint32_t nq = Q - qa < p.qb ? Q - qa : p.qb;
+        const float *qrows = queries + (size_t) qa * dim;
+        float *q_padded = p.pad ? at(p.q_rows) : nullptr;
+        truth_rows_kernel<<<(nq + 7) / 8, 256, 0, stream>>>(qrows, nq, dim, q_norm, q_rest, p.pitch, q_padded, nullptr);
+        CUtensorMap tm_q, tm_b;
+        if (!row_map(&tm_q, p.pad ? q_padded : qrows, nq, p.pitch)) return cudaSuccess;
+        a.Q = nq;
+        const uint32_t qtiles = (nq + kTile - 1) / kTile;
+        for (uint32_t ba = 0; ba < n; ba += p.nb) {
+            const uint32_t nr = n - ba < p.nb ? n - ba : p.nb;
+            const float *brows = base + (size_t) ba * dim;
+            float *b_padded = p.pad ? at(p.rows) : nullptr;
+            const uint32_t blocks = (nr + 7) / 8 < 8u * (uint32_t) sms ? (nr + 7) / 8 : 8u * (uint32_t) sms;
+            truth_rows_kernel<<<blocks, 256, 0, stream>>>(brows, nr, dim, norms, nullptr, p.pitch, b_padded, stats);
+            if (!row_map(&tm_b, p.pad ? b_padded : brows, nr, p.pitch)) return cudaSuccess;
+            a.n = nr;
+            auto launch = [&](uint32_t taken) {   // the CTAs of a pass over `taken` tiles: a full wave where the tiles suffice
+                a.slices = (uint32_t) sms / qtiles;
+                if (a.slices < 1) a.slices = 1;
+                if (a.slices > taken) a.slices = taken;
+                truth_umma_kernel<<<qtiles * a.slices, kTruthThreads, smem, stream>>>(a, tm_q, tm_b);
+            };
+            const uint32_t tiles = (nr + kTile - 1) / kTile;
+            if (ba == 0) {
+                a.sample = true;
+                a.stride = p.sample.stride; a.group = p.sample.group; a.groups = p.sample.groups;
+                launch((tiles + a.stride - 1) / a.stride);
+                truth_threshold_kernel<<<nq, 128, (size_t) a.groups * 4, stream>>>(gmin, a.groups, k, nullptr, q_norm, q_rest, dim, stats, thr, count);
+            } else {
+                truth_threshold_kernel<<<nq, 128, 0, stream>>>(nullptr, 0, k, best, q_norm, q_rest, dim, stats, thr, count);
+            }
+            a.sample = false;
+            a.stride = 1;
+            launch(tiles);
+            const bool last = ba + nr == n;
+            truth_rerank_kernel<<<nq, 128, rr_smem, stream>>>(base, ba, qrows, dim, cand, count, k, best, ba > 0, metric,
+                                                              last ? out_ids + (size_t) qa * k : nullptr, last && out_dists ? out_dists + (size_t) qa * k : nullptr, stats);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        }
+    }
+    if ((e = cudaMemcpyAsync(h_failed, &stats->failed, 4, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
+    return cudaStreamSynchronize(stream);
+}
+
+}  // namespace glide

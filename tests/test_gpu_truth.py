@@ -1,0 +1,50 @@
+"""bruteforce_knn through the tensor cores' candidates against bruteforce_tile_kernel, which takes what is too small for
+them: one call over all queries, then slices of few queries, whose products of values are below the line between the two.
+Bit for bit, ties by id included."""
+import numpy as np
+import pytest
+import torch
+
+from glide_b200 import api
+from glide_b200.params import Metric
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(kind, rng, n, dim):
+    if kind == "ties":
+        return rng.integers(0, 3, (n, dim)).astype(np.float32)
+    x = rng.random((n, dim), dtype=np.float32)
+    if kind == "unit":
+        x -= np.float32(0.5)
+        x /= np.linalg.norm(x, axis=1, keepdims=True)
+    if kind == "offset":          # norms far above the distances: the candidates overflow and the other kernel answers
+        x += np.float32(500)
+    if kind == "nan":
+        x[n // 2, 0] = np.nan
+    return x
+
+
+@pytest.mark.parametrize("kind", ["uniform", "ties", "unit", "offset", "nan"])
+@pytest.mark.parametrize("n,dim,q,k", [
+    (4097, 128, 129, 10),      # a tile and one more on both sides, four operand blocks
+    (3000, 33, 128, 128),      # padded rows, the longest lists
+    (127, 100, 200, 127),      # fewer rows than a tile, nearly all of them wanted
+    (2000, 256, 40, 1),        # the most blocks that stay in shared memory
+    (1500, 260, 70, 50),       # blocks of queries stream with the rows'
+    (700, 961, 33, 10),        # wide and padded
+    (20000, 16, 64, 10),       # one block, half of it filled; a sample of every other stride
+])
+def test_candidates_from_the_tensor_cores_give_the_tile_kernels_results(gpu_ctx, kind, n, dim, q, k):
+    rng = np.random.default_rng(n + dim)
+    base = torch.from_numpy(_rows(kind, rng, n, dim)).to(gpu_ctx.torch_device)
+    queries = torch.from_numpy(_rows("uniform" if kind == "nan" else kind, rng, q, dim)).to(gpu_ctx.torch_device)
+    assert n * q * dim >= 1 << 20
+    metric = Metric.Cosine if kind == "unit" else Metric.Euclidean
+    ids, dists = api.bruteforce_knn(gpu_ctx, base, queries, k, metric)
+    few = max(1, ((1 << 20) - 1) // (n * dim))
+    assert n * dim < 1 << 20
+    for lo in range(0, q, few):
+        want_ids, want = api.bruteforce_knn(gpu_ctx, base, queries[lo:lo + few].contiguous(), k, metric)
+        assert torch.equal(ids[lo:lo + few], want_ids)
+        assert torch.equal(dists[lo:lo + few].view(torch.int32), want.view(torch.int32))
