@@ -542,12 +542,15 @@ static int build_nnd_simt(glide_ctx *ctx, const float *d_reorder_data, uint32_t 
     bool need_nnd = false;
     for (uint32_t s = 0; s < S; s++) need_nnd = need_nnd || h_segment_length[s] > exact_max_rows;
     const size_t nnd_bytes = need_nnd ? nnd_workspace_bytes(rows, K, sample, S) : 0;
-    int rc = ensure_ws(ctx, nnd_bytes + 2 * align256((size_t) S * 4) + align256((size_t) tile_count * 12) + 256);
+    const bool tc = tile_count != 0 && segment_tc_eligible(d_reorder_data, rows, dim, h_segment_length, S, exact_max_rows, knn_degree);
+    const size_t tc_bytes = tc ? segment_tc_scratch_bytes(d_reorder_data, rows, dim, h_segment_length, S, exact_max_rows, knn_degree) : 0;
+    const size_t work_bytes = std::max(nnd_bytes, tc_bytes);   // one after the other
+    int rc = ensure_ws(ctx, work_bytes + 2 * align256((size_t) S * 4) + align256((size_t) tile_count * 12) + 256);
     if (rc) return rc;
     Bump b(ctx->ws);
     uint32_t *d_start = b.take<uint32_t>(S), *d_len = b.take<uint32_t>(S);
     uint32_t *d_tiles = b.take<uint32_t>((size_t) tile_count * 3 + 1);
-    void *work = b.take<char>(nnd_bytes);
+    void *work = b.take<char>(work_bytes);
     std::vector<uint32_t> h_tiles((size_t) tile_count * 3 + 1);
     if (tile_count) segment_knn_fill_tiles(h_segment_start, h_segment_length, S, exact_max_rows, h_tiles.data());
     // empty segments (C == 1 leaves the boundary segment empty, partition_kernel.cuh:58) need no launch
@@ -555,7 +558,14 @@ static int build_nnd_simt(glide_ctx *ctx, const float *d_reorder_data, uint32_t 
     GL_CUDA(ctx, cudaMemcpyAsync(d_start, h_segment_start, (size_t) S * 4, cudaMemcpyHostToDevice, ctx->stream));
     GL_CUDA(ctx, cudaMemcpyAsync(d_len, h_segment_length, (size_t) S * 4, cudaMemcpyHostToDevice, ctx->stream));
     if (iterations_run) *iterations_run = 0;
-    if (tile_count) {
+    uint32_t by_tiles = tile_count;
+    if (tc) {
+        uint32_t failed = 1;
+        GL_CUDA(ctx, launch_segment_tc(d_reorder_data, rows, dim, h_segment_start, h_segment_length, S, exact_max_rows, knn_degree, row_base, work, d_knn,
+                                       &failed, ctx->stream));
+        if (!failed) by_tiles = 0;
+    }
+    if (by_tiles) {
         GL_CUDA(ctx, cudaMemcpyAsync(d_tiles, h_tiles.data(), (size_t) tile_count * 12, cudaMemcpyHostToDevice, ctx->stream));
         GL_CUDA(ctx, launch_segment_knn(d_reorder_data, dim, d_tiles, tile_count, knn_degree, row_base, d_knn, ctx->stream));
     }

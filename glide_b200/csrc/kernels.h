@@ -187,6 +187,11 @@ uint32_t segment_knn_tile_count(const uint32_t *h_seg_len, uint32_t S, uint32_t 
 void segment_knn_fill_tiles(const uint32_t *h_seg_start, const uint32_t *h_seg_len, uint32_t S, uint32_t max_len,
                             uint32_t *h_tiles);
 // row_base: index of data's row 0 within the whole reordered set (enters the padding hash of short partitions)
+// The same rows from the tensor cores' candidates (truth_tc.cu); *h_failed != 0: use launch_segment_knn.
+bool segment_tc_eligible(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree);
+size_t segment_tc_scratch_bytes(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree);
+cudaError_t launch_segment_tc(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len, uint32_t S, uint32_t max_len,
+                              uint32_t out_degree, uint32_t row_base, void *scratch, int32_t *out, uint32_t *h_failed, cudaStream_t stream);
 cudaError_t launch_segment_knn(const float *data, uint32_t dim, const uint32_t *d_tiles, uint32_t tile_count,
                                uint32_t out_degree, uint32_t row_base, int32_t *out, cudaStream_t stream);
 

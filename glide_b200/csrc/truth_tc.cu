@@ -21,6 +21,8 @@
 // peak is what tf32 gives at best: 0.36 ms of it), k = 100: 39.1 to 2.29 ms; 100,000 x 960, 333 queries 6.5 to 0.55 ms;
 // 1M x 64, 10 queries 1.79 to 0.28 ms; 4,000 x 32, 10 queries 122 to 71 us. Where the norms are far above the distances
 // (values around 1,000, spread 1) nearly every row is a candidate and the attempt is lost: 0.39 to 0.81 ms at 50,000 x 64.
+#include <vector>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "umma.cuh"
@@ -39,6 +41,7 @@ constexpr uint32_t kEpi = 4 * kParts;        // epilogue warps
 constexpr uint32_t kTruthThreads = (kEpi + 2) * 32;
 constexpr uint32_t kResidentBlocks = 8;      // query blocks kept in shared memory
 constexpr uint32_t kCap = 3968;              // candidates per query; with up to 128 earlier results 4,096 sort keys
+constexpr uint32_t kSegCap = 2048;           // candidates per row of a segment call
 constexpr uint32_t kBaseRows = 1u << 21;     // base rows per pass (bounds the scratch)
 constexpr uint32_t kQueryRows = 8192;        // queries per pass
 
@@ -48,8 +51,15 @@ struct TruthStats {
     uint32_t pad;
 };
 
+// A CTA's share of a partition's own kNN graph (segment form): rows [first, first + 128) of the partition are the
+// queries, all of its rows the base; `stride`, `group` and `groups` are the sample's, as in TruthArgs.
+struct SegmentTile {
+    uint32_t seg_start, seg_len, first, stride, group, groups;
+};
+
 struct TruthArgs {
-    uint32_t n, Q, dim, kblocks, stages;
+    uint32_t n, Q, dim, kblocks, stages, cap;
+    const SegmentTile *segments;             // segment form: one per CTA; per-query arrays are indexed by CTA * 128 + row
     uint32_t slices, stride;                 // CTA (query tile, slice) takes sampled tiles slice, slice + slices, ...; tile = index * stride
     uint32_t group, groups;                  // columns per minimum, minima per query (sample pass)
     bool sample;
@@ -57,7 +67,7 @@ struct TruthArgs {
     const float *thr;                        // per query (select pass)
     float *gmin;                             // Q x groups
     uint32_t *count;                         // per query
-    uint32_t *cand;                          // Q x kCap
+    uint32_t *cand;                          // Q x cap
     TruthStats *stats;
 };
 
@@ -141,10 +151,15 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
     volatile uint32_t *failed = tmem_slot + 1;
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t qtiles = (a.Q + kTile - 1) / kTile;
-    const uint32_t q0 = (blockIdx.x % qtiles) * kTile, slice = blockIdx.x / qtiles;
-    const uint32_t all = (a.n + kTile - 1) / kTile, taken = (all + a.stride - 1) / a.stride;
-    const uint32_t tiles = slice < taken ? (taken - slice + a.slices - 1) / a.slices : 0u;   // of this CTA
+    const bool seg = a.segments != nullptr;
+    const SegmentTile part_of = seg ? a.segments[blockIdx.x] : SegmentTile{0, a.n, 0, a.stride, a.group, a.groups};
+    const uint32_t qtiles = seg ? 1u : (a.Q + kTile - 1) / kTile;
+    const uint32_t q0 = seg ? blockIdx.x * kTile : (blockIdx.x % qtiles) * kTile;      // index of the first query's results
+    const uint32_t q_row = seg ? part_of.seg_start + part_of.first : q0;                // its row in the query map
+    const uint32_t slice = seg ? 0u : blockIdx.x / qtiles, slices = seg ? 1u : a.slices;
+    const uint32_t n = part_of.seg_len, b_row = part_of.seg_start, stride = a.sample ? part_of.stride : 1u;
+    const uint32_t all = (n + kTile - 1) / kTile, taken = (all + stride - 1) / stride;
+    const uint32_t tiles = slice < taken ? (taken - slice + slices - 1) / slices : 0u;   // of this CTA
 
     if (tid == 0) {
         mbar_init(a_full, 1);
@@ -167,18 +182,18 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
         if (lane == 0 && tiles > 0) {
             if (resident) {
                 mbar_expect_tx(a_full, kblocks * kBlockBytes);
-                for (uint32_t kb = 0; kb < kblocks; kb++) tma_load_2d(As + kb * kBlockBytes, &tm_q, kb * kBlock, q0, a_full);
+                for (uint32_t kb = 0; kb < kblocks; kb++) tma_load_2d(As + kb * kBlockBytes, &tm_q, kb * kBlock, q_row, a_full);
             }
             uint32_t s = 0, use = 0;
             bool ok = true;
             for (uint32_t t = 0; t < tiles && ok; t++) {
-                const uint32_t row0 = (slice + t * a.slices) * a.stride * kTile;
+                const uint32_t row0 = b_row + (slice + t * slices) * stride * kTile;
                 for (uint32_t kb = 0; kb < kblocks; kb++) {
                     if (use > 0 && !mbar_wait(freed + s, (use - 1) & 1u, failed)) { ok = false; break; }
                     uint8_t *dst = ring + s * stage_bytes;
                     mbar_expect_tx(full + s, stage_bytes);
                     tma_load_2d(dst, &tm_b, kb * kBlock, row0, full + s);
-                    if (!resident) tma_load_2d(dst + kBlockBytes, &tm_q, kb * kBlock, q0, full + s);
+                    if (!resident) tma_load_2d(dst + kBlockBytes, &tm_q, kb * kBlock, q_row, full + s);
                     if (++s == stages) { s = 0; use++; }
                 }
             }
@@ -210,12 +225,12 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
     } else {
         // ================= epilogue: thread (query, part) owns 32 columns of every tile =================
         const uint32_t quad = warp & 3u, part = warp >> 2, q = q0 + quad * 32u + lane;
-        const bool active = q < a.Q;
+        const bool active = seg ? part_of.first + quad * 32u + lane < n : q < a.Q;
         const float thr = (active && !a.sample) ? __ldg(a.thr + q) : 0.0f;
         float *cn = cn_w + warp * 32u;
         auto norm_of = [&](uint32_t t) {
-            const uint32_t c = (slice + t * a.slices) * a.stride * kTile + part * 32u + lane;
-            return t < tiles && c < a.n ? __ldg(a.norms + c) : 0.0f;
+            const uint32_t c = (slice + t * slices) * stride * kTile + part * 32u + lane;
+            return t < tiles && c < n ? __ldg(a.norms + b_row + c) : 0.0f;
         };
         float ahead = norm_of(0);
         for (uint32_t t = 0; t < tiles; t++) {
@@ -223,7 +238,7 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
             cn[lane] = ahead;
             ahead = norm_of(t + 1);
             __syncwarp();
-            const uint32_t acc = t & 1u, index = slice + t * a.slices, c0 = index * a.stride * kTile + part * 32u;
+            const uint32_t acc = t & 1u, index = slice + t * slices, c0 = index * stride * kTile + part * 32u;
             bool ok = !*failed && mbar_wait(mma_done + acc, (t >> 1) & 1u, failed);
             ok = __all_sync(kFullMask, ok);
             if (!ok) break;
@@ -242,15 +257,15 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
                 e[j + 2] = __fmaf_rn(-2.0f, __uint_as_float(r[j + 2]), c4.z);
                 e[j + 3] = __fmaf_rn(-2.0f, __uint_as_float(r[j + 3]), c4.w);
             }
-            if (c0 + 32u > a.n) {
+            if (c0 + 32u > n) {
 #pragma unroll
                 for (int j = 0; j < 32; j++)
-                    if (c0 + j >= a.n) e[j] = FLT_MAX;
+                    if (c0 + j >= n) e[j] = FLT_MAX;
             }
             if (!active) continue;
             if (a.sample) {
-                float *out = a.gmin + (uint64_t) q * a.groups + (index * kTile + part * 32u) / a.group;
-                switch (a.group) {
+                float *out = a.gmin + (uint64_t) q * a.groups + (index * kTile + part * 32u) / part_of.group;
+                switch (part_of.group) {
                     case 1: run_minima<1>(e, out); break;
                     case 2: run_minima<2>(e, out); break;
                     case 4: run_minima<4>(e, out); break;
@@ -265,9 +280,9 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
                 if (m <= thr) {   // rare
 #pragma unroll
                     for (int j = 0; j < 32; j++) {
-                        if (e[j] <= thr && c0 + j < a.n) {
+                        if (e[j] <= thr && c0 + j < n) {
                             const uint32_t at = atomicAdd(a.count + q, 1u);
-                            if (at < kCap) a.cand[(uint64_t) q * kCap + at] = c0 + j;
+                            if (at < a.cap) a.cand[(uint64_t) q * a.cap + at] = c0 + j;
                         }
                     }
                 }
@@ -290,13 +305,22 @@ __device__ __forceinline__ float from_ordered(uint32_t o) { return __uint_as_flo
 // bounds. Also clears the query's candidate counter.
 __global__ void __launch_bounds__(128) truth_threshold_kernel(const float *__restrict__ gmin, uint32_t groups, uint32_t k, const u64 *__restrict__ best,
                                                               const float *__restrict__ q_norm, const float *__restrict__ q_rest, uint32_t dim,
-                                                              TruthStats *stats, float *thr, uint32_t *count) {
+                                                              const SegmentTile *segments, TruthStats *stats, float *thr, uint32_t *count) {
     extern __shared__ uint32_t keys[];
     __shared__ uint32_t below;
     const uint32_t q = blockIdx.x, tid = threadIdx.x;
+    uint32_t row = q, pitch = groups;   // the query's row in q_norm and q_rest, minima per query in gmin
+    if (segments != nullptr) {
+        const SegmentTile t = segments[q / kTile];
+        const uint32_t r = t.first + q % kTile;
+        if (r >= t.seg_len) return;
+        row = t.seg_start + r;
+        groups = t.groups;
+        k = min(k, t.seg_len);
+    }
     float kth;
     if (best == nullptr) {
-        for (uint32_t i = tid; i < groups; i += 128) keys[i] = ordered(gmin[(uint64_t) q * groups + i]);
+        for (uint32_t i = tid; i < groups; i += 128) keys[i] = ordered(gmin[(uint64_t) q * pitch + i]);
         uint32_t lo = 0, hi = 0xffffffffu;   // smallest key with at least k keys at or below it
         while (lo < hi) {
             const uint32_t mid = lo + ((hi - lo) >> 1);
@@ -312,10 +336,10 @@ __global__ void __launch_bounds__(128) truth_threshold_kernel(const float *__res
         }
         kth = from_ordered(lo);
     } else {
-        kth = __uint_as_float((uint32_t) (best[(uint64_t) q * k + k - 1] >> 32)) - q_norm[q];
+        kth = __uint_as_float((uint32_t) (best[(uint64_t) q * k + k - 1] >> 32)) - q_norm[row];
     }
     if (tid != 0) return;
-    const float qn = sqrtf(q_norm[q]), ql = sqrtf(q_rest[q]);
+    const float qn = sqrtf(q_norm[row]), ql = sqrtf(q_rest[row]);
     const float bn = sqrtf(__uint_as_float(stats->max_norm)), bl = sqrtf(__uint_as_float(stats->max_rest));
     // |2 q.b - 2 tf32(q).tf32(b)| <= 2 (|q| |b - tf32(b)| + |q - tf32(q)| |b|); every sum (the two norms, the MMA's, the
     // fp32 distance) is within dim + 8 steps of 2^-23 of its terms' magnitudes, all below (|q| + |b|)^2
@@ -325,6 +349,48 @@ __global__ void __launch_bounds__(128) truth_threshold_kernel(const float *__res
     if (!(fabsf(t) < FLT_MAX) || !(bn < 1e18f) || !(qn < 1e18f)) atomicExch(&stats->failed, 1u);
     thr[q] = t;
     count[q] = 0;
+}
+
+// Ascending dimensions, one fused multiply-add each: the order of bruteforce_tile_kernel and segment_knn_kernel.
+__device__ __forceinline__ float direct_distance(const float *query, const float *__restrict__ row, uint32_t dim) {
+    float acc = 0.0f;
+    if ((dim & 3u) == 0 && (reinterpret_cast<uintptr_t>(row) & 15u) == 0) {
+#pragma unroll 8
+        for (uint32_t d = 0; d < dim; d += 4) {
+            const float4 b = __ldg(reinterpret_cast<const float4 *>(row + d));
+            const float4 x = *reinterpret_cast<const float4 *>(query + d);
+            const float dx = x.x - b.x, dy = x.y - b.y, dz = x.z - b.z, dw = x.w - b.w;
+            acc = __fmaf_rn(dx, dx, acc);
+            acc = __fmaf_rn(dy, dy, acc);
+            acc = __fmaf_rn(dz, dz, acc);
+            acc = __fmaf_rn(dw, dw, acc);
+        }
+    } else {
+#pragma unroll 8
+        for (uint32_t d = 0; d < dim; d++) {
+            const float df = query[d] - __ldg(row + d);
+            acc = __fmaf_rn(df, df, acc);
+        }
+    }
+    return acc;
+}
+
+// Sorts `total` keys in shared memory (room for the next power of two) by a CTA of 128 threads.
+__device__ __forceinline__ void sort_keys(u64 *keys, uint32_t total) {
+    const uint32_t tid = threadIdx.x;
+    uint32_t size = 1;
+    while (size < total) size <<= 1;
+    for (uint32_t i = total + tid; i < size; i += 128) keys[i] = ~0ull;
+    for (uint32_t span = 2; span <= size; span <<= 1)
+        for (uint32_t step = span >> 1; step >= 1; step >>= 1) {
+            __syncthreads();
+            for (uint32_t p = tid; p < size / 2; p += 128) {
+                const uint32_t i = 2 * (p & ~(step - 1u)) + (p & (step - 1u)), j = i + step;
+                const u64 x = keys[i], y = keys[j];
+                if ((x > y) == ((i & span) == 0)) { keys[i] = y; keys[j] = x; }
+            }
+        }
+    __syncthreads();
 }
 
 // A CTA per query: exact distances of the candidates (and the earlier passes' results), sorted by (distance, id).
@@ -340,50 +406,48 @@ __global__ void __launch_bounds__(128) truth_rerank_kernel(const float *__restri
     if (tid == 0 && (found > kCap || total < k)) atomicExch(&stats->failed, 1u);
     for (uint32_t d = tid; d < dim; d += 128) query[d] = queries[(uint64_t) q * dim + d];
     __syncthreads();
-    const bool vec = (dim & 3u) == 0 && (reinterpret_cast<uintptr_t>(base) & 15u) == 0;
     for (uint32_t i = tid; i < n; i += 128) {
         const uint32_t id = first_row + cand[(uint64_t) q * kCap + i];
-        const float *row = base + (uint64_t) id * dim;
-        float acc = 0.0f;   // ascending dimensions, one fused multiply-add each: the order of bruteforce_tile_kernel
-        if (vec) {
-#pragma unroll 8
-            for (uint32_t d = 0; d < dim; d += 4) {
-                const float4 b = __ldg(reinterpret_cast<const float4 *>(row + d));
-                const float4 x = *reinterpret_cast<const float4 *>(query + d);
-                const float dx = x.x - b.x, dy = x.y - b.y, dz = x.z - b.z, dw = x.w - b.w;
-                acc = __fmaf_rn(dx, dx, acc);
-                acc = __fmaf_rn(dy, dy, acc);
-                acc = __fmaf_rn(dz, dz, acc);
-                acc = __fmaf_rn(dw, dw, acc);
-            }
-        } else {
-#pragma unroll 8
-            for (uint32_t d = 0; d < dim; d++) {
-                const float df = query[d] - __ldg(row + d);
-                acc = __fmaf_rn(df, df, acc);
-            }
-        }
-        keys[i] = ((u64) __float_as_uint(acc) << 32) | id;
+        keys[i] = ((u64) __float_as_uint(direct_distance(query, base + (uint64_t) id * dim, dim)) << 32) | id;
     }
     if (earlier)
         for (uint32_t i = tid; i < k; i += 128) keys[n + i] = best[(uint64_t) q * k + i];
-    uint32_t size = 1;
-    while (size < total) size <<= 1;
-    for (uint32_t i = total + tid; i < size; i += 128) keys[i] = ~0ull;
-    for (uint32_t span = 2; span <= size; span <<= 1)
-        for (uint32_t step = span >> 1; step >= 1; step >>= 1) {
-            __syncthreads();
-            for (uint32_t p = tid; p < size / 2; p += 128) {
-                const uint32_t i = 2 * (p & ~(step - 1u)) + (p & (step - 1u)), j = i + step;
-                const u64 x = keys[i], y = keys[j];
-                if ((x > y) == ((i & span) == 0)) { keys[i] = y; keys[j] = x; }
-            }
-        }
-    __syncthreads();
+    sort_keys(keys, total);
     for (uint32_t i = tid; i < k && i < total; i += 128) {
         best[(uint64_t) q * k + i] = keys[i];
         if (out_ids) out_ids[(uint64_t) q * k + i] = (uint32_t) keys[i];
         if (out_dists) out_dists[(uint64_t) q * k + i] = finish_metric(__uint_as_float((uint32_t) (keys[i] >> 32)), metric);
+    }
+}
+
+// Segment form, a CTA per row: its candidates without itself, nearest first, as partition-local ids; a row with fewer
+// than out_degree others is padded with xorshift32(flat index) % partition size (nn_descent.cuh:1384-1391).
+__global__ void __launch_bounds__(128) segment_rerank_kernel(const float *__restrict__ data, uint32_t dim, const SegmentTile *__restrict__ segments,
+                                                             const uint32_t *__restrict__ cand, const uint32_t *__restrict__ count, uint32_t out_degree,
+                                                             uint32_t row_base, int32_t *out, TruthStats *stats) {
+    extern __shared__ __align__(16) uint32_t smem[];
+    u64 *keys = reinterpret_cast<u64 *>(smem);                      // kSegCap
+    float *query = reinterpret_cast<float *>(keys + kSegCap);       // dim
+    const uint32_t q = blockIdx.x, tid = threadIdx.x;
+    const SegmentTile t = segments[q / kTile];
+    const uint32_t r = t.first + q % kTile;
+    if (r >= t.seg_len) return;
+    const float *seg = data + (uint64_t) t.seg_start * dim;
+    const uint32_t found = count[q], n = min(found, kSegCap);
+    const uint32_t want = min(out_degree, t.seg_len - 1u);
+    if (tid == 0 && (found > kSegCap || n < want + 1u)) atomicExch(&stats->failed, 1u);
+    for (uint32_t d = tid; d < dim; d += 128) query[d] = seg[(uint64_t) r * dim + d];
+    __syncthreads();
+    for (uint32_t i = tid; i < n; i += 128) {
+        const uint32_t id = cand[(uint64_t) q * kSegCap + i];
+        keys[i] = id == r ? ~0ull : ((u64) __float_as_uint(direct_distance(query, seg + (uint64_t) id * dim, dim)) << 32) | id;
+    }
+    sort_keys(keys, n);
+    for (uint32_t j = tid; j < out_degree; j += 128) {
+        const uint64_t flat = (uint64_t) (t.seg_start + r) * out_degree + j;
+        uint32_t u = (uint32_t) (flat + (uint64_t) row_base * out_degree);  // xorshift32, utils.cuh:14-19
+        u ^= u >> 13; u ^= u << 27; u ^= u >> 5; u *= 0x9E3779B9u;
+        out[flat] = (int32_t) (j < want && j < n ? (uint32_t) keys[j] : u % t.seg_len);
     }
 }
 
@@ -439,6 +503,9 @@ TruthPlan truth_plan(const float *base, const float *queries, uint32_t n, uint32
     return p;
 }
 
+uint32_t ring_stages(uint32_t kblocks) { return kblocks <= kResidentBlocks ? 12u - kblocks : 6u; }    // 192 KB of operand blocks
+size_t umma_smem(uint32_t stages) { return 1024 + 12u * (size_t) kBlockBytes + kEpi * 32 * 4 + (1 + 2 * stages + 4) * 8 + 16; }
+
 // row-major rows of `pitch` floats as TMA boxes of 32 values x 128 rows (make_row_map takes the row length as the pitch)
 bool row_map(CUtensorMap *tm, const float *ptr, uint32_t rows, uint32_t pitch) { return make_row_map(tm, ptr, rows, pitch, kTile); }
 
@@ -471,11 +538,10 @@ cudaError_t launch_truth_tc(const float *base, uint32_t n, const float *queries,
     if (e != cudaSuccess) return e;
 
     TruthArgs a{};
-    a.dim = dim; a.kblocks = (p.pitch + kBlock - 1) / kBlock;
-    const bool resident = a.kblocks <= kResidentBlocks;
-    a.stages = resident ? 12u - a.kblocks : 6u;    // 192 KB of operand blocks
+    a.dim = dim; a.cap = kCap; a.kblocks = (p.pitch + kBlock - 1) / kBlock;
+    a.stages = ring_stages(a.kblocks);
     a.norms = norms; a.thr = thr; a.gmin = gmin; a.count = count; a.cand = cand; a.stats = stats;
-    const size_t smem = 1024 + 12u * (size_t) kBlockBytes + kEpi * 32 * 4 + (1 + 2 * a.stages + 4) * 8 + 16;
+    const size_t smem = umma_smem(a.stages);
     if ((e = cudaFuncSetAttribute(truth_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
     const size_t rr_smem = 4096 * 8 + (size_t) p.pitch * 4;
     if (rr_smem > 48 * 1024 && (e = cudaFuncSetAttribute(truth_rerank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) rr_smem)) != cudaSuccess) return e;
@@ -508,9 +574,9 @@ cudaError_t launch_truth_tc(const float *base, uint32_t n, const float *queries,
                 a.sample = true;
                 a.stride = p.sample.stride; a.group = p.sample.group; a.groups = p.sample.groups;
                 launch((tiles + a.stride - 1) / a.stride);
-                truth_threshold_kernel<<<nq, 128, (size_t) a.groups * 4, stream>>>(gmin, a.groups, k, nullptr, q_norm, q_rest, dim, stats, thr, count);
+                truth_threshold_kernel<<<nq, 128, (size_t) a.groups * 4, stream>>>(gmin, a.groups, k, nullptr, q_norm, q_rest, dim, nullptr, stats, thr, count);
             } else {
-                truth_threshold_kernel<<<nq, 128, 0, stream>>>(nullptr, 0, k, best, q_norm, q_rest, dim, stats, thr, count);
+                truth_threshold_kernel<<<nq, 128, 0, stream>>>(nullptr, 0, k, best, q_norm, q_rest, dim, nullptr, stats, thr, count);
             }
             a.sample = false;
             a.stride = 1;
@@ -520,6 +586,118 @@ cudaError_t launch_truth_tc(const float *base, uint32_t n, const float *queries,
                                                               last ? out_ids + (size_t) qa * k : nullptr, last && out_dists ? out_dists + (size_t) qa * k : nullptr, stats);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
+    }
+    if ((e = cudaMemcpyAsync(h_failed, &stats->failed, 4, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
+    return cudaStreamSynchronize(stream);
+}
+
+// ---- every row's nearest rows of its own partition ----------------------------------------------
+namespace {
+
+constexpr uint32_t kSegTiles = 296;   // CTAs per launch (two per SM): bounds the candidates and minima kept
+
+struct SegPlan {
+    bool pad;
+    uint32_t pitch, groups;
+    size_t stats, tiles, norms, rest, thr, count, cand, gmin, rows, total;
+};
+
+SegPlan seg_plan(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree) {
+    SegPlan p;
+    p.pad = (dim & 3u) != 0 || (reinterpret_cast<uintptr_t>(data) & 15u) != 0;
+    p.pitch = (dim + 3u) & ~3u;
+    p.groups = 1;
+    size_t tiles = 0;
+    for (uint32_t s = 0; s < S; s++)
+        if (h_len[s] > 0 && h_len[s] <= max_len) {
+            const uint32_t g = sample_of(h_len[s], out_degree + 1).groups;
+            if (g > p.groups) p.groups = g;
+            tiles += (h_len[s] + kTile - 1) / kTile;
+        }
+    const size_t slots = (size_t) (tiles < kSegTiles ? tiles : kSegTiles) * kTile;
+    size_t at = 0;
+    auto take = [&](size_t bytes) { const size_t o = at; at += up256(bytes); return o; };
+    p.stats = take(sizeof(TruthStats));
+    p.tiles = take(tiles * sizeof(SegmentTile));
+    p.norms = take((size_t) rows * 4);
+    p.rest = take((size_t) rows * 4);
+    p.thr = take(slots * 4);
+    p.count = take(slots * 4);
+    p.cand = take(slots * kSegCap * 4);
+    p.gmin = take(slots * p.groups * 4);
+    p.rows = take(p.pad ? (size_t) rows * p.pitch * 4 : 0);
+    p.total = at;
+    return p;
+}
+
+}  // namespace
+
+// The padded copy of rows that TMA cannot read is bounded, and so are a partition's minima.
+bool segment_tc_eligible(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree) {
+    const bool pad = (dim & 3u) != 0 || (reinterpret_cast<uintptr_t>(data) & 15u) != 0;
+    if (dim < 16 || dim > 4096 || out_degree < 1 || out_degree > 64 || (pad && (uint64_t) rows * dim > (1ull << 30)) || encode_tiled_fn() == nullptr) return false;
+    uint64_t taken = 0, pairs = 0;
+    for (uint32_t s = 0; s < S; s++) {
+        if (h_len[s] > max_len) continue;
+        if (h_len[s] > kBaseRows) return false;
+        taken += h_len[s];
+        pairs += (uint64_t) h_len[s] * h_len[s];
+    }
+    // values a row meets: below 2^15 (about 1,000 rows of 32 values) the re-rank of a hundred candidates costs more than the pairs.
+    // segment_knn_kernel against this, ms: 60 partitions of 1,000 x 23 0.97 / 1.41; 2 of 2,000 x 20 0.36 / 0.28; 8 of 1,000 x 768
+    // 1.01 / 0.82; 4 of 15,000 x 50 9.8 / 7.0; 10 of 10,000 x 100 16.5 / 6.3; 15 of 4,000 x 960 (lists of 64) 34.0 / 10.3
+    return pairs * dim >= taken << 15;
+}
+
+size_t segment_tc_scratch_bytes(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree) {
+    return seg_plan(data, rows, dim, h_len, S, max_len, out_degree).total;
+}
+
+// Exact kNN rows of every partition of at most max_len rows: what segment_knn_kernel writes, bit for bit. *h_failed != 0: use
+// that kernel. Synchronises the stream.
+cudaError_t launch_segment_tc(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len, uint32_t S, uint32_t max_len,
+                              uint32_t out_degree, uint32_t row_base, void *scratch, int32_t *out, uint32_t *h_failed, cudaStream_t stream) {
+    const SegPlan p = seg_plan(data, rows, dim, h_len, S, max_len, out_degree);
+    std::vector<SegmentTile> tiles;
+    for (uint32_t s = 0; s < S; s++) {
+        if (h_len[s] == 0 || h_len[s] > max_len) continue;
+        const Sample m = sample_of(h_len[s], out_degree + 1);
+        for (uint32_t first = 0; first < h_len[s]; first += kTile) tiles.push_back(SegmentTile{h_start[s], h_len[s], first, m.stride, m.group, m.groups});
+    }
+    *h_failed = 0;
+    if (tiles.empty()) return cudaSuccess;
+    *h_failed = 1;
+    char *w = static_cast<char *>(scratch);
+    auto at = [&](size_t o) { return reinterpret_cast<float *>(w + o); };
+    TruthStats *stats = reinterpret_cast<TruthStats *>(w + p.stats);
+    SegmentTile *d_tiles = reinterpret_cast<SegmentTile *>(w + p.tiles);
+    uint32_t *count = reinterpret_cast<uint32_t *>(w + p.count), *cand = reinterpret_cast<uint32_t *>(w + p.cand);
+    float *padded = p.pad ? at(p.rows) : nullptr;
+    CUtensorMap tm;
+    if (!row_map(&tm, p.pad ? padded : data, rows, p.pitch)) return cudaSuccess;
+    cudaError_t e = cudaMemsetAsync(stats, 0, sizeof(TruthStats), stream);
+    // the table is pageable host memory: the copy has read it when the call returns
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_tiles, tiles.data(), tiles.size() * sizeof(SegmentTile), cudaMemcpyHostToDevice, stream);
+    if (e != cudaSuccess) return e;
+    const uint32_t blocks = (rows + 7) / 8 < 1184u ? (rows + 7) / 8 : 1184u;
+    truth_rows_kernel<<<blocks, 256, 0, stream>>>(data, rows, dim, at(p.norms), at(p.rest), p.pitch, padded, stats);
+    TruthArgs a{};
+    a.dim = dim; a.cap = kSegCap; a.kblocks = (p.pitch + kBlock - 1) / kBlock; a.stages = ring_stages(a.kblocks);
+    a.groups = p.groups;
+    a.norms = at(p.norms); a.thr = at(p.thr); a.gmin = at(p.gmin); a.count = count; a.cand = cand; a.stats = stats;
+    const size_t smem = umma_smem(a.stages), rr_smem = (size_t) kSegCap * 8 + (size_t) p.pitch * 4;
+    if ((e = cudaFuncSetAttribute(truth_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
+    for (size_t first = 0; first < tiles.size(); first += kSegTiles) {
+        const uint32_t n = (uint32_t) (tiles.size() - first < kSegTiles ? tiles.size() - first : kSegTiles);
+        a.segments = d_tiles + first;
+        a.sample = true;
+        truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm);
+        truth_threshold_kernel<<<n * kTile, 128, (size_t) p.groups * 4, stream>>>(a.gmin, p.groups, out_degree + 1, nullptr, a.norms, at(p.rest), dim, a.segments,
+                                                                                  stats, at(p.thr), count);
+        a.sample = false;
+        truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm);
+        segment_rerank_kernel<<<n * kTile, 128, rr_smem, stream>>>(data, dim, a.segments, cand, count, out_degree, row_base, out, stats);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     if ((e = cudaMemcpyAsync(h_failed, &stats->failed, 4, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
     return cudaStreamSynchronize(stream);

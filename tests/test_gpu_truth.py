@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from glide_b200 import api
-from glide_b200.params import Metric
+from glide_b200.params import Metric, NNDescentParameter
 
 pytestmark = pytest.mark.gpu
 
@@ -48,3 +48,31 @@ def test_candidates_from_the_tensor_cores_give_the_tile_kernels_results(gpu_ctx,
         want_ids, want = api.bruteforce_knn(gpu_ctx, base, queries[lo:lo + few].contiguous(), k, metric)
         assert torch.equal(ids[lo:lo + few], want_ids)
         assert torch.equal(dists[lo:lo + few].view(torch.int32), want.view(torch.int32))
+
+
+@pytest.mark.parametrize("kind", ["uniform", "ties", "offset", "nan"])
+@pytest.mark.parametrize("dim", [16, 33, 100, 256, 260, 961])
+@pytest.mark.parametrize("degree", [8, 32, 64])
+def test_partition_graphs_from_the_tensor_cores_are_the_tile_kernels(gpu_ctx, kind, dim, degree):
+    lens = np.array([1, 2, 40, 128, 129, 1000, 4200], np.uint32)   # padding, one tile, a tile and a row, several
+    start = np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.uint32)
+    rng = np.random.default_rng(dim + degree)
+    rows = torch.from_numpy(_rows(kind, rng, int(lens.sum()), dim)).to(gpu_ctx.torch_device)
+    got, _, _ = api.build_nnd(gpu_ctx, NNDescentParameter(degree), rows, start, lens, exact_max_rows=16384)
+    got = got.cpu().numpy()
+    for lo, n in zip(start, lens):
+        lo, n = int(lo), int(n)
+        part = rows[lo:lo + n].contiguous()
+        if kind == "nan" and bool(torch.isnan(part).any()):
+            continue      # a row that is no number is nobody's neighbour; which pads fill its own row is checked by its sums' order only
+        k = min(degree, n - 1)
+        if k == 0:
+            continue
+        few = max(1, ((1 << 20) - 1) // (n * dim))     # below the line: bruteforce_tile_kernel
+        for q in range(0, n, max(few, n // 4)):
+            hi = min(n, q + few)
+            ids, _ = api.bruteforce_knn(gpu_ctx, part, part[q:hi].contiguous(), min(k + 1, n))
+            ids = ids.cpu().numpy()
+            for r in range(q, hi):
+                want = [i for i in ids[r - q] if i != r][:k]
+                assert list(got[lo + r][:k]) == want
