@@ -542,10 +542,17 @@ static int build_nnd_simt(glide_ctx *ctx, const float *d_reorder_data, uint32_t 
     bool need_nnd = false;
     for (uint32_t s = 0; s < S; s++) need_nnd = need_nnd || h_segment_length[s] > exact_max_rows;
     const size_t nnd_bytes = need_nnd ? nnd_workspace_bytes(rows, K, sample, S) : 0;
-    const bool tc = tile_count != 0 && segment_tc_eligible(d_reorder_data, rows, dim, h_segment_length, S, exact_max_rows, knn_degree);
+    bool tc = tile_count != 0 && segment_tc_eligible(d_reorder_data, rows, dim, h_segment_length, S, exact_max_rows, knn_degree);
     const size_t tc_bytes = tc ? segment_tc_scratch_bytes(d_reorder_data, rows, dim, h_segment_length, S, exact_max_rows, knn_degree) : 0;
-    const size_t work_bytes = std::max(nnd_bytes, tc_bytes);   // one after the other
-    int rc = ensure_ws(ctx, work_bytes + 2 * align256((size_t) S * 4) + align256((size_t) tile_count * 12) + 256);
+    size_t work_bytes = std::max(nnd_bytes, tc_bytes);   // one after the other
+    const size_t tables = 2 * align256((size_t) S * 4) + align256((size_t) tile_count * 12) + 256;
+    int rc = ensure_ws(ctx, work_bytes + tables);
+    if (tc && rc == GLIDE_ERR_NO_MEMORY) {   // the tile kernel needs none
+        cudaGetLastError();
+        tc = false;
+        work_bytes = nnd_bytes;
+        rc = ensure_ws(ctx, work_bytes + tables);
+    }
     if (rc) return rc;
     Bump b(ctx->ws);
     uint32_t *d_start = b.take<uint32_t>(S), *d_len = b.take<uint32_t>(S);
@@ -588,10 +595,14 @@ int glide_bruteforce_knn(glide_ctx *ctx, const float *d_base, uint32_t n, const 
     GL_REQUIRE(ctx, k >= 1 && k <= 128 && k <= n, GLIDE_ERR_UNSUPPORTED, "bruteforce_knn: k must be in [1, min(128, n)]");
     GL_CUDA(ctx, cudaSetDevice(ctx->device));
     const uint32_t splits = bruteforce_default_splits(n, q);
-    const bool tc = q > 0 && truth_tc_eligible(n, q, dim, k);
-    size_t need = bruteforce_scratch_bytes(q, k, splits) + 256;
-    if (tc) need = std::max(need, truth_tc_scratch_bytes(d_base, d_queries, n, q, dim, k));
-    int rc = ensure_ws(ctx, need);
+    bool tc = q > 0 && truth_tc_eligible(n, q, dim, k);
+    const size_t need = bruteforce_scratch_bytes(q, k, splits) + 256;
+    int rc = ensure_ws(ctx, tc ? std::max(need, truth_tc_scratch_bytes(d_base, d_queries, n, q, dim, k)) : need);
+    if (tc && rc == GLIDE_ERR_NO_MEMORY) {   // the tile kernel asks for less
+        cudaGetLastError();
+        tc = false;
+        rc = ensure_ws(ctx, need);
+    }
     if (rc) return rc;
     Timed timer(ctx);
     if (tc) {
