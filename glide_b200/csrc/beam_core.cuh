@@ -519,6 +519,10 @@ __device__ __forceinline__ void sort_candidates_two_warps(float *cand_k, uint32_
 // Bound by instruction issue and by the networks' chain of 20 dependent shuffles. Measured, networks
 // only against this: build of 1M x 128 rows (beams 64 and 128) 238 to 215 ms, 10,000 queries at beam 32
 // 655 to 627 us, 2,000 at beam 128 1136 to 1078 us.
+// All of this takes an ascending beam. The seed step alone can leave another one: an infinite distance (a row
+// that holds an infinity, a square beyond fp32) or one that is no number sorts behind the empty slots' FLT_MAX,
+// which follow it in the beam all the same. Such a search (kSeedNetworks) takes the networks at every merge, as they
+// move these entries. No later candidate brings one in: the merges take only what is smaller than a slot's key.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kFewSurvivors = 8;
 
@@ -629,8 +633,9 @@ __device__ __forceinline__ void trim_beam(float (&bk)[NB], uint32_t (&bv)[NB], u
 // Drops the candidates beyond the beam's last slot ((FLT_MAX, kInvalid), as an empty slot) and does as
 // much of the merge as few survivors allow. kMergeDone: the beam is merged. kMergeSorted: (ck[0], cv[0]) of lane j
 // is the j-th survivor, the merge is left to do. kMergeSort: both are.
-// open_seed: the seed row held a valid id with distance FLT_MAX; while such an entry may sit among the
+// open_seed (kSeedWide): the seed row held a valid id with distance FLT_MAX; while such an entry may sit among the
 // beam's empty slots, which of them a merge replaces is the network's business too.
+constexpr uint32_t kSeedWide = 1, kSeedNetworks = 2;   // what the seed step left behind, see above
 enum MergeState : int { kMergeDone = 0, kMergeSorted = 1, kMergeSort = 2 };
 
 template<int NB, int NC>
@@ -657,6 +662,21 @@ __device__ __forceinline__ MergeState merge_few(float (&bk)[NB], uint32_t (&bv)[
     return kMergeDone;
 }
 
+// A key above an empty slot's, or no number at all, in the beam that the seed step left.
+template<int NB>
+__device__ __forceinline__ bool beyond_empty(const float (&bk)[NB]) {
+    bool beyond = false;
+#pragma unroll
+    for (int i = 0; i < NB; i++) beyond = beyond || !(bk[i] <= FLT_MAX);
+    return __any_sync(kFullMask, beyond);
+}
+
+// An infinite distance among the seed candidates (a lane's own) that the 32-slot sort would leave in front of the empty
+// slots. With one that is no number beside it neither sort has an order to keep: the narrow one stays.
+__device__ __forceinline__ bool infinite_seed(float ck) {
+    return __any_sync(kFullMask, ck > FLT_MAX) && !__any_sync(kFullMask, ck != ck);
+}
+
 // The search loop proper. On return bk/bv hold the beam (ascending, position
 // j = NB*lane + i, ids still carrying the explored flag). Returns the number of
 // expansions; *rows_read accumulates data rows fetched.
@@ -668,12 +688,12 @@ __device__ __forceinline__ uint32_t beam_loop(float (&bk)[NB], uint32_t (&bv)[NB
                                               uint32_t *rows_read, bool wide_first_sort = false) {
     const uint32_t lane = lane_id();
     constexpr uint32_t MAXB = 32u * NB;
-    uint32_t iter = 0;
+    uint32_t iter = 0, seed = wide_first_sort ? kSeedWide : 0u;
     bool terminate = false;
     uint32_t rows = 0;
     while (true) {
         MergeState state = kMergeSort;
-        if (iter != 0) {
+        if (iter != 0 && !(seed & kSeedNetworks)) {
             float ck[NC];
             uint32_t cv[NC];
 #pragma unroll
@@ -682,7 +702,7 @@ __device__ __forceinline__ uint32_t beam_loop(float (&bk)[NB], uint32_t (&bv)[NB
                 ck[i] = (j < degree) ? s.cand_dist[j] : FLT_MAX;
                 cv[i] = (j < degree) ? s.cand_id[j] : kInvalid;
             }
-            state = merge_few<NB, NC>(bk, bv, p.beam, ck, cv, wide_first_sort);
+            state = merge_few<NB, NC>(bk, bv, p.beam, ck, cv, (seed & kSeedWide) != 0);
             if (state != kMergeDone) {   // back to the strip: the survivors at their slots, or sorted from slot 0 on
 #pragma unroll
                 for (int i = 0; i < NC; i++) {
@@ -700,10 +720,11 @@ __device__ __forceinline__ uint32_t beam_loop(float (&bk)[NB], uint32_t (&bv)[NB
             // first `degree` outputs of that network equal those of the 32-slot network on the real
             // slots alone, ties included (checked exhaustively-at-random in
             // tests/test_oracle_primitives.py); the only input that breaks this is the seed row's
-            // excluded id (valid id, FLT_MAX), flagged by wide_first_sort. Used by the build kernels
+            // excluded id (valid id, FLT_MAX), flagged by wide_first_sort, or an infinite distance. Used by the build kernels
             // (instruction bound); the query search kernel is bound by row gathers and measured
             // slower with it.
-            if (NARROW_SORT && NC == 2 && degree <= 32 && !(wide_first_sort && iter == 0)) {
+            if (NARROW_SORT && NC == 2 && degree <= 32 &&
+                !(iter == 0 && ((seed & kSeedWide) || infinite_seed(lane < degree ? s.cand_dist[lane] : FLT_MAX)))) {
                 float ck[1] = {lane < degree ? s.cand_dist[lane] : FLT_MAX};
                 uint32_t cv[1] = {lane < degree ? s.cand_id[lane] : kInvalid};
                 warp_sort<1>(ck, cv);
@@ -747,6 +768,7 @@ __device__ __forceinline__ uint32_t beam_loop(float (&bk)[NB], uint32_t (&bv)[NB
                     bk[i] = take ? s.cand_dist[j] : FLT_MAX;
                     bv[i] = take ? s.cand_id[j] : kInvalid;
                 }
+                if (beyond_empty<NB>(bk)) seed |= kSeedNetworks;
             } else if constexpr (NB == 16) {
                 merge_beam_two_warps(bk, bv, p.beam, degree, s.cand_dist, s.cand_id, reinterpret_cast<float *>(s.tail), s.tail + 512);
             } else {
@@ -827,8 +849,9 @@ __device__ __forceinline__ uint32_t beam_loop(float (&bk)[NB], uint32_t (&bv)[NB
 //  * the reference sorts MAX_CANDIDATE = 64 slots, the upper 32 being padding (FLT_MAX,
 //    0xffffffff); the first 32 outputs of that network equal those of the 32-slot network on the
 //    real slots alone as long as every FLT_MAX slot carries the padding id (checked at random in
-//    tests/test_oracle_primitives.py). The one input that breaks this is the seed row's excluded
-//    id (a valid id with FLT_MAX), which takes the 64-slot network once (wide_first_sort);
+//    tests/test_oracle_primitives.py). What breaks this is a seed row's excluded id (a valid id with
+//    FLT_MAX) or an infinite distance (it sorts behind the padding); a seed step with either takes the 64-slot
+//    network once. Later candidates of that kind enter no beam, wherever they sort;
 //  * for beam <= 32 the 64-position merge network splits, after its first stride-32 step, into
 //    two independent halves of which only the lower one is kept, so NB = 1 gives the same beam.
 // ---------------------------------------------------------------------------
@@ -881,21 +904,21 @@ __device__ __forceinline__ uint32_t beam_loop_lanes(float (&bk)[NB], uint32_t (&
                                                     bool wide_first_sort = false) {
     const uint32_t lane = lane_id();
     constexpr uint32_t MAXB = 32u * NB;
-    uint32_t iter = 0;
+    uint32_t iter = 0, seed = wide_first_sort ? kSeedWide : 0u;
     bool terminate = false;
     uint32_t rows = 0;
     while (true) {
         MergeState state = kMergeSort;
-        if (iter != 0) {
+        if (iter != 0 && !(seed & kSeedNetworks)) {
             float k1[1] = {ck};
             uint32_t v1[1] = {cv};
-            state = merge_few<NB, 1>(bk, bv, p.beam, k1, v1, wide_first_sort);
+            state = merge_few<NB, 1>(bk, bv, p.beam, k1, v1, (seed & kSeedWide) != 0);
             ck = k1[0];
             cv = v1[0];
         }
         if (state == kMergeSort) {
             // -- sort the candidates (search_kernel.cuh:9-37): afterwards lane j holds the j-th --
-            if (wide_first_sort && iter == 0) {
+            if (iter == 0 && ((seed & kSeedWide) || infinite_seed(ck))) {
                 float k2[2] = {ck, FLT_MAX};          // slot j = lane + 32*i
                 uint32_t v2[2] = {cv, kInvalid};
                 warp_sort<2>(k2, v2);                 // sorted position e = 2*lane + i
@@ -923,6 +946,7 @@ __device__ __forceinline__ uint32_t beam_loop_lanes(float (&bk)[NB], uint32_t (&
                     bk[i] = take ? c : FLT_MAX;
                     bv[i] = take ? id : kInvalid;
                 }
+                if (beyond_empty<NB>(bk)) seed |= kSeedNetworks;
             } else if constexpr (NB == 16) {
                 float *row_k = reinterpret_cast<float *>(s.tail + 1024);
                 uint32_t *row_v = s.tail + 1024 + 32;
