@@ -147,7 +147,7 @@ int glide_ctx_create(int device, glide_ctx **out) {
     // load the common kernel instances and let the driver size its local-memory reservation now,
     // not inside the first timed stage
     if (preload_build_kernels(ctx->stream) != cudaSuccess || preload_search_kernels(ctx->stream) != cudaSuccess ||
-        cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
+        preload_truth_kernels() != cudaSuccess || cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
         glide_ctx_destroy(ctx);
         return GLIDE_ERR_CUDA;
     }

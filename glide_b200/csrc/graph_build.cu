@@ -576,12 +576,18 @@ cudaError_t launch_build(const BuildArgs &a, cudaStream_t stream) {
 // First launches pay for loading the kernel and for growing the device's local-memory
 // reservation (tens of milliseconds); a context pays them once, at creation, with launches that
 // find no work (count = 0: every warp returns at once).
+template<typename D>
+static void preload_build_instances(const BuildDev &d, cudaStream_t stream) {
+    build_kernel<2, 2, true, D><<<1, 32, 0, stream>>>(d);
+    build_kernel<4, 2, true, D><<<1, 32, 0, stream>>>(d);
+    build_kernel<2, 2, false, D><<<1, 32, 0, stream>>>(d);
+    build_kernel<4, 2, false, D><<<1, 32, 0, stream>>>(d);
+}
+
 cudaError_t preload_build_kernels(cudaStream_t stream) {
-    BuildDev d{};
-    build_kernel<2, 2, true, DimOf<true>><<<1, 32, 0, stream>>>(d);
-    build_kernel<4, 2, true, DimOf<true>><<<1, 32, 0, stream>>>(d);
-    build_kernel<2, 2, false, DimOf<false>><<<1, 32, 0, stream>>>(d);
-    build_kernel<4, 2, false, DimOf<false>><<<1, 32, 0, stream>>>(d);
+    const BuildDev d{};
+    preload_build_instances<DimOf<true>>(d, stream);
+    preload_build_instances<DimOf<false>>(d, stream);
     return cudaGetLastError();
 }
 

@@ -53,6 +53,7 @@ struct SearchArgs {
 cudaError_t launch_search_team(const SearchArgs &a, cudaStream_t stream, bool *launched);
 cudaError_t launch_search(const SearchArgs &a, cudaStream_t stream);
 cudaError_t preload_search_kernels(cudaStream_t stream);
+void preload_search_team_kernels(cudaStream_t stream);
 
 struct SelectSegmentArgs {
     const float *queries;
@@ -172,6 +173,8 @@ cudaError_t launch_count_changed(const uint32_t *a, const uint32_t *b, uint32_t 
 // ---- bruteforce.cu -------------------------------------------------------
 size_t bruteforce_scratch_bytes(uint32_t Q, uint32_t k, uint32_t splits);
 uint32_t bruteforce_default_splits(uint32_t n, uint32_t Q);
+// Loads what exact kNN from tensor-core candidates launches.
+cudaError_t preload_truth_kernels();
 // The same results from the tensor cores' candidates (truth_tc.cu); *h_failed != 0: use launch_bruteforce.
 bool truth_tc_eligible(uint32_t n, uint32_t Q, uint32_t dim, uint32_t k);
 size_t truth_tc_scratch_bytes(const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k);

@@ -86,13 +86,21 @@ cudaError_t launch_search_t(const SearchDev &d, uint32_t warps_per_cta, size_t s
 
 }  // namespace
 
-// See preload_build_kernels: launches without work (Q = 0, no ticket) that load the common instances.
+// See preload_build_kernels: launches without work (Q = 0, no ticket) that load the common instances, for rows that fit
+// the lanes and for others.
+template<typename D>
+static void preload_search_instances(const SearchDev &d, cudaStream_t stream) {
+    search_kernel_32<2, true, D><<<1, 32, 0, stream>>>(d);
+    search_kernel<2, 2, true, D><<<1, 32, 0, stream>>>(d);
+    search_kernel<4, 2, true, D><<<1, 32, 0, stream>>>(d);
+    search_kernel<2, 2, false, D><<<1, 32, 0, stream>>>(d);
+}
+
 cudaError_t preload_search_kernels(cudaStream_t stream) {
-    SearchDev d{};
-    search_kernel_32<2, true, DimOf<true>><<<1, 32, 0, stream>>>(d);
-    search_kernel<2, 2, true, DimOf<true>><<<1, 32, 0, stream>>>(d);
-    search_kernel<4, 2, true, DimOf<true>><<<1, 32, 0, stream>>>(d);
-    search_kernel<2, 2, false, DimOf<false>><<<1, 32, 0, stream>>>(d);
+    const SearchDev d{};
+    preload_search_instances<DimOf<true>>(d, stream);
+    preload_search_instances<DimOf<false>>(d, stream);
+    preload_search_team_kernels(stream);
     return cudaGetLastError();
 }
 

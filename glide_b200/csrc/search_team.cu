@@ -62,6 +62,22 @@ cudaError_t launch_team_t(const SearchDev &given, size_t smem_bytes, int sms, cu
 
 }  // namespace
 
+template<typename D>
+static void preload_team_instances(const SearchDev &d, cudaStream_t stream) {
+    const size_t call = sizeof(TeamCall);   // all that the master's farewell to its helper touches
+    search_team_kernel<1, 2, true, false, D><<<1, 64, call, stream>>>(d);
+    search_team_kernel<2, 2, true, false, D><<<1, 64, call, stream>>>(d);
+    search_team_kernel<4, 2, true, false, D><<<1, 64, call, stream>>>(d);
+    search_team_kernel<2, 2, false, false, D><<<1, 64, call, stream>>>(d);
+}
+
+// The instances that small batches take, as preload_search_kernels: Q = 0, the master quits at once.
+void preload_search_team_kernels(cudaStream_t stream) {
+    const SearchDev d{};
+    preload_team_instances<DimOf<true>>(d, stream);
+    preload_team_instances<DimOf<false>>(d, stream);
+}
+
 // Beams above 256 slots and adjacency rows above 64 entries stay with a warp per query (their merges and sorts use
 // per-warp scratch of another layout), and so does the streamed large path, which skips most of its queries.
 cudaError_t launch_search_team(const SearchArgs &a, cudaStream_t stream, bool *launched) {

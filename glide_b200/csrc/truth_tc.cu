@@ -511,6 +511,19 @@ bool row_map(CUtensorMap *tm, const float *ptr, uint32_t rows, uint32_t pitch) {
 
 }  // namespace
 
+// A kernel is loaded when its attributes are first asked for; most builds whose rows knn_tc.cu does not take come here.
+cudaError_t preload_truth_kernels() {
+    cudaFuncAttributes f;
+    const void *kernels[] = {reinterpret_cast<const void *>(truth_rows_kernel), reinterpret_cast<const void *>(truth_umma_kernel),
+                             reinterpret_cast<const void *>(truth_threshold_kernel), reinterpret_cast<const void *>(truth_rerank_kernel),
+                             reinterpret_cast<const void *>(segment_rerank_kernel)};
+    for (const void *k : kernels) {
+        const cudaError_t e = cudaFuncGetAttributes(&f, k);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 // Below 2^20 products of values a dozen launches cost what the tiles do (the smallest size timed is 1.3 x 2^20: 122 to 71 us).
 bool truth_tc_eligible(uint32_t n, uint32_t Q, uint32_t dim, uint32_t k) {
     return dim >= 16 && dim <= 4096 && k >= 1 && k <= 128 && n >= 1 && (uint64_t) n * Q * dim >= (1ull << 20) && encode_tiled_fn() != nullptr;
