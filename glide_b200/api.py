@@ -93,6 +93,11 @@ class Context:
         return float(self.lib.glide_last_kernel_ms(self.handle)) / 1000.0
 
     @property
+    def last_team_warps(self) -> int:
+        """Warps of a query's CTA in the last search; 0: a warp per query."""
+        return int(self.lib.glide_last_search_team_warps(self.handle))
+
+    @property
     def tc_knn_fallbacks(self) -> int:
         """kNN stages the tensor-core kernel handed back to the fp32 kernels (0 in normal operation)."""
         return int(self.lib.glide_tc_knn_fallbacks(self.handle))
@@ -132,8 +137,9 @@ class Context:
         self.lib.glide_enable_counters(self.handle, 1 if on else 0)
 
     def read_counters(self) -> tuple[int, int, int, int]:
-        """(rows read while searching, expansions, rows read while pruning, points whose beam
-        ended unfilled) of the last search / build / refine call."""
+        """(rows scored while searching, expansions, rows read while pruning, points whose beam
+        ended unfilled) of the last build / refine call. After a search the third is the rows that teams
+        read beside the scored ones."""
         out = (C.c_uint64 * 4)()
         self.check(self.lib.glide_read_counters(self.handle, out))
         return int(out[0]), int(out[1]), int(out[2]), int(out[3])

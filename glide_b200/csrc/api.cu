@@ -183,6 +183,7 @@ void glide_last_search_split_ms(const glide_ctx *ctx, float out[2]) {
 }
 
 uint32_t glide_last_search_launches(const glide_ctx *ctx) { return ctx ? ctx->last_launches : 0; }
+uint32_t glide_last_search_team_warps(const glide_ctx *ctx) { return ctx ? ctx->last_team_warps : 0; }
 
 void glide_enable_counters(glide_ctx *ctx, int on) { if (ctx) ctx->counters_on = on != 0; }
 
@@ -981,7 +982,7 @@ int glide_search(glide_ctx *ctx, const float *d_data, uint32_t num, uint32_t dim
         launched += 1;
     }
     GL_CUDA(ctx, cudaEventRecord(ctx->ev_mid, ctx->stream));
-    GL_CUDA(ctx, launch_search(a, ctx->stream));
+    GL_CUDA(ctx, launch_search(a, ctx->stream, &ctx->last_team_warps));
     ctx->last_launches = launched + 1;
     rc = timer.finish();
     if (rc) return rc;
@@ -1135,7 +1136,7 @@ int glide_search_pipe_submit(glide_search_pipe *pipe, const float *d_data, uint3
         a.order = order;
         launched += 1;
     }
-    GL_CUDA(ctx, launch_search(a, ctx->stream));
+    GL_CUDA(ctx, launch_search(a, ctx->stream, &ctx->last_team_warps));
     ctx->last_launches = launched + 1;
     GL_CUDA(ctx, cudaEventRecord(sl.searched, ctx->stream));
     GL_CUDA(ctx, cudaStreamWaitEvent(pipe->down, sl.searched, 0));
@@ -1202,7 +1203,7 @@ int glide_search_static_scratch(glide_ctx *ctx, const float *d_data, uint32_t nu
     uint32_t launched = 0;
     GL_CUDA(ctx, launch_assign(r, ctx->stream, &launched));
     GL_CUDA(ctx, cudaEventRecord(ctx->ev_mid, ctx->stream));
-    GL_CUDA(ctx, launch_search(a, ctx->stream));
+    GL_CUDA(ctx, launch_search(a, ctx->stream, &ctx->last_team_warps));
     ctx->last_launches = launched + 1;
     rc = timer.finish();
     if (rc) return rc;
@@ -1244,7 +1245,7 @@ int glide_search_on_sub(glide_ctx *ctx, const float *d_data, uint32_t dim, const
     a.counters = counters_or_null(ctx);
     a.ticket = ctx->ticket;
     Timed timer(ctx);
-    GL_CUDA(ctx, launch_search(a, ctx->stream));
+    GL_CUDA(ctx, launch_search(a, ctx->stream, &ctx->last_team_warps));
     return timer.finish();
 }
 

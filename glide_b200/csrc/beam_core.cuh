@@ -184,7 +184,7 @@ __device__ __forceinline__ uint32_t score_candidates(const WarpStrip &s, uint32_
 
 // TEAM: an adjacency row of `degree` entries scored by the team (see above). Ids that are not new (or are
 // `skip_insert`) leave empty candidate slots, `skip_score` keeps its slot with distance FLT_MAX. Returns the number
-// of candidates that got a distance; *skip_kept: skip_score was new.
+// of candidates that got a distance (rows that fit the lanes: `degree` rows are read for them); *skip_kept: skip_score was new.
 template<typename D>
 __device__ __forceinline__ uint32_t team_expand(const WarpStrip &s, const uint32_t *__restrict__ row, bool have_row, uint32_t skip_insert,
                                                 uint32_t skip_score, const uint32_t *__restrict__ graph, uint32_t degree,

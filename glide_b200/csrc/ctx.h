@@ -21,6 +21,7 @@ struct glide_ctx {
     unsigned long long *counters = nullptr;  // 4 x u64 on the device
     uint32_t *ticket = nullptr;              // one word: the search kernel's query counter
     uint32_t *start_point_word = nullptr;    // one word: the start point of a per-partition refine
+    uint32_t last_team_warps = 0;            // of the last glide_search or resident large search
     uint32_t last_launches = 0;              // kernels enqueued by the last glide_search
     float *tc_norms = nullptr;               // centroid norms for the assignment's tensor-core prefilter (up to 4096 centroids)
     uint32_t tc_knn_fallbacks = 0;           // kNN stages the tensor-core kernel handed back to the fp32 kernels

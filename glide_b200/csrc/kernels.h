@@ -48,10 +48,11 @@ struct SearchArgs {
     uint32_t *ticket;            // one word, zeroed by launch_search: warps draw their next query from it;
                                  // nullptr: query q runs on warp q of the grid
 };
-// A CTA of several warps per query, where the batch leaves the device idle otherwise; *launched = false: nothing
+// A CTA of several warps per query, where the batch leaves the device idle otherwise; *team_warps = 0: nothing
 // was launched, a warp per query is the better form.
-cudaError_t launch_search_team(const SearchArgs &a, cudaStream_t stream, bool *launched);
-cudaError_t launch_search(const SearchArgs &a, cudaStream_t stream);
+cudaError_t launch_search_team(const SearchArgs &a, cudaStream_t stream, uint32_t *team_warps);
+// *team_warps: the warps of a query's CTA, 0 with a warp per query
+cudaError_t launch_search(const SearchArgs &a, cudaStream_t stream, uint32_t *team_warps = nullptr);
 cudaError_t preload_search_kernels(cudaStream_t stream);
 void preload_search_team_kernels(cudaStream_t stream);
 

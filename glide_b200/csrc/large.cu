@@ -667,7 +667,7 @@ int glide_large_search(glide_large *L, const float *d_queries, uint32_t q, const
         LG_CUDA(ctx, cudaEventCreate(&k0));
         LG_CUDA(ctx, cudaEventCreate(&k1));
         LG_CUDA(ctx, cudaEventRecord(k0, ctx->stream));
-        LG_CUDA(ctx, glide::launch_search(a, ctx->stream));
+        LG_CUDA(ctx, glide::launch_search(a, ctx->stream, &ctx->last_team_warps));
         LG_CUDA(ctx, cudaEventRecord(k1, ctx->stream));
         LG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         float ms = 0;

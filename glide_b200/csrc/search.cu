@@ -104,11 +104,13 @@ cudaError_t preload_search_kernels(cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_search(const SearchArgs &a, cudaStream_t stream) {
+cudaError_t launch_search(const SearchArgs &a, cudaStream_t stream, uint32_t *team_warps) {
+    uint32_t team = 0;
+    if (team_warps) *team_warps = 0;
     if (a.Q == 0) return cudaSuccess;
-    bool launched = false;
-    const cudaError_t te = launch_search_team(a, stream, &launched);
-    if (te != cudaSuccess || launched) return te;
+    const cudaError_t te = launch_search_team(a, stream, &team);
+    if (team_warps) *team_warps = team;
+    if (te != cudaSuccess || team) return te;
     SearchDev d;
     d.a = a;
     d.max_centroid = pow2_at_least(a.C, 32);

@@ -140,6 +140,8 @@ __device__ __forceinline__ void search_one(const SearchDev &d, const WarpStrip &
     if (a.counters && lane == 0) {
         atomicAdd(a.counters + 0, (unsigned long long) rows);
         atomicAdd(a.counters + 1, (unsigned long long) iters);
+        // a team's calls read whole adjacency rows where the rows fit the lanes (team_expand): what they read beside `rows`
+        if (TEAM && dim_fits(dim)) atomicAdd(a.counters + 2, (unsigned long long) (iters + 1u) * a.degree - rows);
     }
 }
 

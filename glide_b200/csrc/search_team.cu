@@ -45,7 +45,7 @@ void (*team_instance(const SearchArgs &a))(const SearchDev) {
 }
 
 template<int NB, int NC, bool LANES>
-cudaError_t launch_team_t(const SearchDev &given, size_t smem_bytes, int sms, cudaStream_t stream, bool *launched) {
+cudaError_t launch_team_t(const SearchDev &given, size_t smem_bytes, int sms, cudaStream_t stream, uint32_t *team_warps_out) {
     SearchDev d = given;
     void (*kernel)(const SearchDev) = rows_fit_lanes(d.a.dim) ? team_instance<NB, NC, LANES, DimOf<true>>(d.a) : team_instance<NB, NC, LANES, DimOf<false>>(d.a);
     if (smem_bytes > 48 * 1024) {
@@ -56,7 +56,7 @@ cudaError_t launch_team_t(const SearchDev &given, size_t smem_bytes, int sms, cu
     if (warps == 0) return cudaSuccess;
     d.a.ticket = nullptr;   // every query has its CTA
     kernel<<<d.a.Q, warps * 32, smem_bytes, stream>>>(d);
-    *launched = true;
+    *team_warps_out = warps;
     return cudaGetLastError();
 }
 
@@ -80,8 +80,8 @@ void preload_search_team_kernels(cudaStream_t stream) {
 
 // Beams above 256 slots and adjacency rows above 64 entries stay with a warp per query (their merges and sorts use
 // per-warp scratch of another layout), and so does the streamed large path, which skips most of its queries.
-cudaError_t launch_search_team(const SearchArgs &a, cudaStream_t stream, bool *launched) {
-    *launched = false;
+cudaError_t launch_search_team(const SearchArgs &a, cudaStream_t stream, uint32_t *team_warps_out) {
+    *team_warps_out = 0;
     if (a.p.beam > 256 || a.degree > 64 || (a.segment_ids != nullptr && a.parts == nullptr)) return cudaSuccess;
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -97,14 +97,14 @@ cudaError_t launch_search_team(const SearchArgs &a, cudaStream_t stream, bool *l
     const size_t bytes = (size_t) d.strip_words * 4;
     if (bytes > 200 * 1024) return cudaSuccess;   // refused by the other form too
     if (a.degree <= 32) {
-        if (a.p.beam <= 32 && a.parts == nullptr) return launch_team_t<1, 2, true>(d, bytes, sms, stream, launched);
-        if (a.p.beam <= 64) return launch_team_t<2, 2, true>(d, bytes, sms, stream, launched);
-        if (a.p.beam <= 128) return launch_team_t<4, 2, true>(d, bytes, sms, stream, launched);
-        return launch_team_t<8, 2, true>(d, bytes, sms, stream, launched);
+        if (a.p.beam <= 32 && a.parts == nullptr) return launch_team_t<1, 2, true>(d, bytes, sms, stream, team_warps_out);
+        if (a.p.beam <= 64) return launch_team_t<2, 2, true>(d, bytes, sms, stream, team_warps_out);
+        if (a.p.beam <= 128) return launch_team_t<4, 2, true>(d, bytes, sms, stream, team_warps_out);
+        return launch_team_t<8, 2, true>(d, bytes, sms, stream, team_warps_out);
     }
-    if (a.p.beam <= 64) return launch_team_t<2, 2, false>(d, bytes, sms, stream, launched);
-    if (a.p.beam <= 128) return launch_team_t<4, 2, false>(d, bytes, sms, stream, launched);
-    return launch_team_t<8, 2, false>(d, bytes, sms, stream, launched);
+    if (a.p.beam <= 64) return launch_team_t<2, 2, false>(d, bytes, sms, stream, team_warps_out);
+    if (a.p.beam <= 128) return launch_team_t<4, 2, false>(d, bytes, sms, stream, team_warps_out);
+    return launch_team_t<8, 2, false>(d, bytes, sms, stream, team_warps_out);
 }
 
 }  // namespace glide

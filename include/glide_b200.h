@@ -288,8 +288,12 @@ int glide_search_static_scratch(glide_ctx *ctx, const float *d_data, uint32_t nu
 void glide_last_search_split_ms(const glide_ctx *ctx, float out[2]);
 /* Number of kernels the last glide_search enqueued (routing kernels + the search kernel). */
 uint32_t glide_last_search_launches(const glide_ctx *ctx);
-/* Counters of the last search/build/refine/define_partition call when enabled: rows read during
- * search, expansions, rows read during pruning, and a fourth that depends on the call: build and
+/* Warps of the CTA that each query of the context's last search (small path, or resident partitions of the
+ * large one) was given, where the batch was small enough for that; 0: a warp per query. */
+uint32_t glide_last_search_team_warps(const glide_ctx *ctx);
+/* Counters of the last search/build/refine/define_partition call when enabled: rows scored during
+ * search, expansions, rows read during pruning (after a search: rows that teams of warps read beside
+ * the scored ones), and a fourth that depends on the call: build and
  * refine count the points whose beam ended with fewer than `beam` entries; search and
  * define_partition count the points whose nearest centroid was settled by the exact
  * warp-per-point kernel (a tie, or too many candidates after the tensor-core prefilter). */
