@@ -102,6 +102,18 @@ class Context:
         """kNN stages the tensor-core kernel handed back to the fp32 kernels (0 in normal operation)."""
         return int(self.lib.glide_tc_knn_fallbacks(self.handle))
 
+    @property
+    def exact_knn_counts(self) -> tuple[int, int, int, int]:
+        """Queries of bruteforce_knn calls given to tensor-core candidates, those of them that the fp32 tile kernel
+        answered after all, and the same two for the rows of kNN stages."""
+        out = (C.c_uint64 * 4)()
+        self.lib.glide_exact_knn_counts(self.handle, out)
+        return tuple(int(x) for x in out)
+
+    def limit_exact_knn(self, base_rows: int = 0, queries: int = 0, padded_values: int = 0, tiles: int = 0):
+        """Bounds the scratch of exact kNN from tensor-core candidates by the size of its passes (0: the default)."""
+        self.check(self.lib.glide_limit_exact_knn(self.handle, base_rows, queries, padded_values, tiles))
+
     def empty(self, shape, dtype) -> torch.Tensor:
         return torch.empty(shape, dtype=dtype, device=self.torch_device)
 

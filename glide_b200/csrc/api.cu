@@ -532,6 +532,21 @@ int glide_build_nnd_range(glide_ctx *ctx, const float *d_reorder_data, uint32_t 
 
 uint32_t glide_tc_knn_fallbacks(const glide_ctx *ctx) { return ctx ? ctx->tc_knn_fallbacks : 0; }
 
+void glide_exact_knn_counts(const glide_ctx *ctx, uint64_t out[4]) {
+    if (!ctx || !out) return;
+    for (int i = 0; i < 4; i++) out[i] = ctx->exact_knn[i];
+}
+
+int glide_limit_exact_knn(glide_ctx *ctx, uint32_t base_rows, uint32_t queries, uint32_t padded_values, uint32_t tiles) {
+    if (!ctx) return GLIDE_ERR_BAD_ARG;
+    const TcPasses usual;
+    ctx->tc_passes.base_rows = base_rows ? base_rows : usual.base_rows;
+    ctx->tc_passes.queries = queries ? std::min(queries, usual.queries) : usual.queries;
+    ctx->tc_passes.padded_values = padded_values ? padded_values : usual.padded_values;
+    ctx->tc_passes.tiles = tiles ? std::min(tiles, usual.tiles) : usual.tiles;
+    return GLIDE_OK;
+}
+
 // The fp32 kernels of the kNN stage: the register-tile all-pairs kernel for partitions of at most
 // exact_max_rows rows (unless skip_exact: the tensor-core kernel has done them) and NN-descent for the rest.
 static int build_nnd_simt(glide_ctx *ctx, const float *d_reorder_data, uint32_t rows, uint32_t dim,
@@ -544,7 +559,7 @@ static int build_nnd_simt(glide_ctx *ctx, const float *d_reorder_data, uint32_t 
     for (uint32_t s = 0; s < S; s++) need_nnd = need_nnd || h_segment_length[s] > exact_max_rows;
     const size_t nnd_bytes = need_nnd ? nnd_workspace_bytes(rows, K, sample, S) : 0;
     bool tc = tile_count != 0 && segment_tc_eligible(d_reorder_data, rows, dim, h_segment_length, S, exact_max_rows, knn_degree);
-    const size_t tc_bytes = tc ? segment_tc_scratch_bytes(d_reorder_data, rows, dim, h_segment_length, S, exact_max_rows, knn_degree) : 0;
+    const size_t tc_bytes = tc ? segment_tc_scratch_bytes(ctx->tc_passes, d_reorder_data, rows, dim, h_segment_length, S, exact_max_rows, knn_degree) : 0;
     size_t work_bytes = std::max(nnd_bytes, tc_bytes);   // one after the other
     const size_t tables = 2 * align256((size_t) S * 4) + align256((size_t) tile_count * 12) + 256;
     int rc = ensure_ws(ctx, work_bytes + tables);
@@ -569,9 +584,14 @@ static int build_nnd_simt(glide_ctx *ctx, const float *d_reorder_data, uint32_t 
     uint32_t by_tiles = tile_count;
     if (tc) {
         uint32_t failed = 1;
-        GL_CUDA(ctx, launch_segment_tc(d_reorder_data, rows, dim, h_segment_start, h_segment_length, S, exact_max_rows, knn_degree, row_base, work, d_knn,
+        GL_CUDA(ctx, launch_segment_tc(ctx->tc_passes, d_reorder_data, rows, dim, h_segment_start, h_segment_length, S, exact_max_rows, knn_degree, row_base, work, d_knn,
                                        &failed, ctx->stream));
         if (!failed) by_tiles = 0;
+        for (uint32_t s = 0; s < S; s++)
+            if (h_segment_length[s] <= exact_max_rows) {
+                ctx->exact_knn[2] += h_segment_length[s];
+                if (failed) ctx->exact_knn[3] += h_segment_length[s];
+            }
     }
     if (by_tiles) {
         GL_CUDA(ctx, cudaMemcpyAsync(d_tiles, h_tiles.data(), (size_t) tile_count * 12, cudaMemcpyHostToDevice, ctx->stream));
@@ -598,7 +618,7 @@ int glide_bruteforce_knn(glide_ctx *ctx, const float *d_base, uint32_t n, const 
     const uint32_t splits = bruteforce_default_splits(n, q);
     bool tc = q > 0 && truth_tc_eligible(n, q, dim, k);
     const size_t need = bruteforce_scratch_bytes(q, k, splits) + 256;
-    int rc = ensure_ws(ctx, tc ? std::max(need, truth_tc_scratch_bytes(d_base, d_queries, n, q, dim, k)) : need);
+    int rc = ensure_ws(ctx, tc ? std::max(need, truth_tc_scratch_bytes(ctx->tc_passes, d_base, d_queries, n, q, dim, k)) : need);
     if (tc && rc == GLIDE_ERR_NO_MEMORY) {   // the tile kernel asks for less
         cudaGetLastError();
         tc = false;
@@ -608,8 +628,10 @@ int glide_bruteforce_knn(glide_ctx *ctx, const float *d_base, uint32_t n, const 
     Timed timer(ctx);
     if (tc) {
         uint32_t failed = 1;
-        GL_CUDA(ctx, launch_truth_tc(d_base, n, d_queries, q, dim, k, metric, ctx->ws, d_out_ids, d_out_dists, &failed, ctx->stream));
+        GL_CUDA(ctx, launch_truth_tc(ctx->tc_passes, d_base, n, d_queries, q, dim, k, metric, ctx->ws, d_out_ids, d_out_dists, &failed, ctx->stream));
+        ctx->exact_knn[0] += q;
         if (!failed) return timer.finish();
+        ctx->exact_knn[1] += q;
     }
     GL_CUDA(ctx, launch_bruteforce(d_base, n, d_queries, q, dim, k, metric, splits, ctx->ws, d_out_ids, d_out_dists, ctx->stream));
     return timer.finish();

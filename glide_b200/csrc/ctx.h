@@ -7,6 +7,8 @@
 
 #include <cuda_runtime.h>
 
+#include "kernels.h"
+
 struct glide_comm_state;   // comm.cu
 
 struct glide_ctx {
@@ -25,6 +27,8 @@ struct glide_ctx {
     uint32_t last_launches = 0;              // kernels enqueued by the last glide_search
     float *tc_norms = nullptr;               // centroid norms for the assignment's tensor-core prefilter (up to 4096 centroids)
     uint32_t tc_knn_fallbacks = 0;           // kNN stages the tensor-core kernel handed back to the fp32 kernels
+    glide::TcPasses tc_passes;               // sizes of the passes of exact kNN from tensor-core candidates
+    uint64_t exact_knn[4] = {0, 0, 0, 0};    // glide_exact_knn_counts
     bool counters_on = false;
     glide_comm_state *comm = nullptr;        // NCCL communicator (glide_comm_init), or nullptr
 };

@@ -176,11 +176,18 @@ size_t bruteforce_scratch_bytes(uint32_t Q, uint32_t k, uint32_t splits);
 uint32_t bruteforce_default_splits(uint32_t n, uint32_t Q);
 // Loads what exact kNN from tensor-core candidates launches.
 cudaError_t preload_truth_kernels();
+// How much of its work that takes at a time (truth_tc.cu): the passes bound the scratch.
+struct TcPasses {
+    uint32_t base_rows = 1u << 21;      // base rows of a bruteforce call
+    uint32_t queries = 8192;            // its queries
+    uint32_t padded_values = 1u << 28;  // values in the padded copy of rows that TMA cannot read (1 GB)
+    uint32_t tiles = 296;               // CTAs of 128 rows of a launch over partitions
+};
 // The same results from the tensor cores' candidates (truth_tc.cu); *h_failed != 0: use launch_bruteforce.
 bool truth_tc_eligible(uint32_t n, uint32_t Q, uint32_t dim, uint32_t k);
-size_t truth_tc_scratch_bytes(const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k);
-cudaError_t launch_truth_tc(const float *base, uint32_t n, const float *queries, uint32_t Q, uint32_t dim, uint32_t k, int metric, void *scratch,
-                            uint32_t *out_ids, float *out_dists, uint32_t *h_failed, cudaStream_t stream);
+size_t truth_tc_scratch_bytes(const TcPasses &passes, const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k);
+cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t n, const float *queries, uint32_t Q, uint32_t dim, uint32_t k, int metric,
+                            void *scratch, uint32_t *out_ids, float *out_dists, uint32_t *h_failed, cudaStream_t stream);
 cudaError_t launch_bruteforce(const float *base, uint32_t n, const float *queries, uint32_t Q, uint32_t dim,
                               uint32_t k, int metric, uint32_t splits, void *scratch, uint32_t *out_ids,
                               float *out_dists, cudaStream_t stream);
@@ -193,8 +200,8 @@ void segment_knn_fill_tiles(const uint32_t *h_seg_start, const uint32_t *h_seg_l
 // row_base: index of data's row 0 within the whole reordered set (enters the padding hash of short partitions)
 // The same rows from the tensor cores' candidates (truth_tc.cu); *h_failed != 0: use launch_segment_knn.
 bool segment_tc_eligible(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree);
-size_t segment_tc_scratch_bytes(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree);
-cudaError_t launch_segment_tc(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len, uint32_t S, uint32_t max_len,
+size_t segment_tc_scratch_bytes(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree);
+cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len, uint32_t S, uint32_t max_len,
                               uint32_t out_degree, uint32_t row_base, void *scratch, int32_t *out, uint32_t *h_failed, cudaStream_t stream);
 cudaError_t launch_segment_knn(const float *data, uint32_t dim, const uint32_t *d_tiles, uint32_t tile_count,
                                uint32_t out_degree, uint32_t row_base, int32_t *out, cudaStream_t stream);

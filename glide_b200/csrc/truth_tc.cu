@@ -21,6 +21,7 @@
 // peak is what tf32 gives at best: 0.36 ms of it), k = 100: 39.1 to 2.29 ms; 100,000 x 960, 333 queries 6.5 to 0.55 ms;
 // 1M x 64, 10 queries 1.79 to 0.28 ms; 4,000 x 32, 10 queries 122 to 71 us. Where the norms are far above the distances
 // (values around 1,000, spread 1) nearly every row is a candidate and the attempt is lost: 0.39 to 0.81 ms at 50,000 x 64.
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -42,8 +43,7 @@ constexpr uint32_t kTruthThreads = (kEpi + 2) * 32;
 constexpr uint32_t kResidentBlocks = 8;      // query blocks kept in shared memory
 constexpr uint32_t kCap = 3968;              // candidates per query; with up to 128 earlier results 4,096 sort keys
 constexpr uint32_t kSegCap = 2048;           // candidates per row of a segment call
-constexpr uint32_t kBaseRows = 1u << 21;     // base rows per pass (bounds the scratch)
-constexpr uint32_t kQueryRows = 8192;        // queries per pass
+constexpr uint32_t kSegRows = 1u << 21;      // rows of the largest partition of a segment call
 
 struct TruthStats {
     uint32_t max_norm, max_rest;             // bits of the largest |b|^2 and |b - tf32(b)|^2 (non-negative floats order as integers)
@@ -477,14 +477,13 @@ struct TruthPlan {
     size_t norms, rows, q_rows, q_norm, q_rest, thr, count, cand, gmin, best, stats, total;
 };
 
-TruthPlan truth_plan(const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k) {
+TruthPlan truth_plan(const TcPasses &passes, const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k) {
     TruthPlan p;
     p.pad = (dim & 3u) != 0 || ((reinterpret_cast<uintptr_t>(base) | reinterpret_cast<uintptr_t>(queries)) & 15u) != 0;
     p.pitch = (dim + 3u) & ~3u;
-    p.nb = n < kBaseRows ? n : kBaseRows;
-    if (p.pad && (uint64_t) p.nb * p.pitch > (1u << 28)) p.nb = (1u << 28) / p.pitch;   // a padded copy of 1 GB at most
-    p.nb = (p.nb + 3u) & ~3u;
-    p.qb = Q < kQueryRows ? Q : kQueryRows;
+    p.nb = std::min(n, std::max(k, passes.base_rows));   // the first pass has k results
+    if (p.pad && (uint64_t) p.nb * p.pitch > passes.padded_values) p.nb = std::max(k, passes.padded_values / p.pitch);
+    p.qb = Q < passes.queries ? Q : passes.queries;
     p.sample = sample_of(p.nb < n ? p.nb : n, k);
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t o = at; at += up256(bytes); return o; };
@@ -529,14 +528,14 @@ bool truth_tc_eligible(uint32_t n, uint32_t Q, uint32_t dim, uint32_t k) {
     return dim >= 16 && dim <= 4096 && k >= 1 && k <= 128 && n >= 1 && (uint64_t) n * Q * dim >= (1ull << 20) && encode_tiled_fn() != nullptr;
 }
 
-size_t truth_tc_scratch_bytes(const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k) {
-    return truth_plan(base, queries, n, Q, dim, k).total;
+size_t truth_tc_scratch_bytes(const TcPasses &passes, const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k) {
+    return truth_plan(passes, base, queries, n, Q, dim, k).total;
 }
 
 // *h_failed != 0: the caller computes the results by other means. Synchronises the stream.
-cudaError_t launch_truth_tc(const float *base, uint32_t n, const float *queries, uint32_t Q, uint32_t dim, uint32_t k, int metric, void *scratch,
-                            uint32_t *out_ids, float *out_dists, uint32_t *h_failed, cudaStream_t stream) {
-    const TruthPlan p = truth_plan(base, queries, n, Q, dim, k);
+cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t n, const float *queries, uint32_t Q, uint32_t dim, uint32_t k, int metric,
+                            void *scratch, uint32_t *out_ids, float *out_dists, uint32_t *h_failed, cudaStream_t stream) {
+    const TruthPlan p = truth_plan(passes, base, queries, n, Q, dim, k);
     char *w = static_cast<char *>(scratch);
     auto at = [&](size_t o) { return reinterpret_cast<float *>(w + o); };
     TruthStats *stats = reinterpret_cast<TruthStats *>(w + p.stats);
@@ -607,15 +606,13 @@ cudaError_t launch_truth_tc(const float *base, uint32_t n, const float *queries,
 // ---- every row's nearest rows of its own partition ----------------------------------------------
 namespace {
 
-constexpr uint32_t kSegTiles = 296;   // CTAs per launch (two per SM): bounds the candidates and minima kept
-
 struct SegPlan {
     bool pad;
     uint32_t pitch, groups;
     size_t stats, tiles, norms, rest, thr, count, cand, gmin, rows, total;
 };
 
-SegPlan seg_plan(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree) {
+SegPlan seg_plan(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree) {
     SegPlan p;
     p.pad = (dim & 3u) != 0 || (reinterpret_cast<uintptr_t>(data) & 15u) != 0;
     p.pitch = (dim + 3u) & ~3u;
@@ -627,7 +624,7 @@ SegPlan seg_plan(const float *data, uint32_t rows, uint32_t dim, const uint32_t 
             if (g > p.groups) p.groups = g;
             tiles += (h_len[s] + kTile - 1) / kTile;
         }
-    const size_t slots = (size_t) (tiles < kSegTiles ? tiles : kSegTiles) * kTile;
+    const size_t slots = (size_t) (tiles < passes.tiles ? tiles : passes.tiles) * kTile;
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t o = at; at += up256(bytes); return o; };
     p.stats = take(sizeof(TruthStats));
@@ -652,7 +649,7 @@ bool segment_tc_eligible(const float *data, uint32_t rows, uint32_t dim, const u
     uint64_t taken = 0, pairs = 0;
     for (uint32_t s = 0; s < S; s++) {
         if (h_len[s] > max_len) continue;
-        if (h_len[s] > kBaseRows) return false;
+        if (h_len[s] > kSegRows) return false;
         taken += h_len[s];
         pairs += (uint64_t) h_len[s] * h_len[s];
     }
@@ -662,15 +659,16 @@ bool segment_tc_eligible(const float *data, uint32_t rows, uint32_t dim, const u
     return pairs * dim >= taken << 15;
 }
 
-size_t segment_tc_scratch_bytes(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree) {
-    return seg_plan(data, rows, dim, h_len, S, max_len, out_degree).total;
+size_t segment_tc_scratch_bytes(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len,
+                                uint32_t out_degree) {
+    return seg_plan(passes, data, rows, dim, h_len, S, max_len, out_degree).total;
 }
 
 // Exact kNN rows of every partition of at most max_len rows: what segment_knn_kernel writes, bit for bit. *h_failed != 0: use
 // that kernel. Synchronises the stream.
-cudaError_t launch_segment_tc(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len, uint32_t S, uint32_t max_len,
-                              uint32_t out_degree, uint32_t row_base, void *scratch, int32_t *out, uint32_t *h_failed, cudaStream_t stream) {
-    const SegPlan p = seg_plan(data, rows, dim, h_len, S, max_len, out_degree);
+cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len,
+                              uint32_t S, uint32_t max_len, uint32_t out_degree, uint32_t row_base, void *scratch, int32_t *out, uint32_t *h_failed, cudaStream_t stream) {
+    const SegPlan p = seg_plan(passes, data, rows, dim, h_len, S, max_len, out_degree);
     std::vector<SegmentTile> tiles;
     for (uint32_t s = 0; s < S; s++) {
         if (h_len[s] == 0 || h_len[s] > max_len) continue;
@@ -700,8 +698,8 @@ cudaError_t launch_segment_tc(const float *data, uint32_t rows, uint32_t dim, co
     a.norms = at(p.norms); a.thr = at(p.thr); a.gmin = at(p.gmin); a.count = count; a.cand = cand; a.stats = stats;
     const size_t smem = umma_smem(a.stages), rr_smem = (size_t) kSegCap * 8 + (size_t) p.pitch * 4;
     if ((e = cudaFuncSetAttribute(truth_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
-    for (size_t first = 0; first < tiles.size(); first += kSegTiles) {
-        const uint32_t n = (uint32_t) (tiles.size() - first < kSegTiles ? tiles.size() - first : kSegTiles);
+    for (size_t first = 0; first < tiles.size(); first += passes.tiles) {
+        const uint32_t n = (uint32_t) (tiles.size() - first < passes.tiles ? tiles.size() - first : passes.tiles);
         a.segments = d_tiles + first;
         a.sample = true;
         truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm);

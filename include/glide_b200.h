@@ -219,6 +219,14 @@ int glide_ctx_synchronize(glide_ctx *ctx);
  * tensor map, a bounded wait that ran out, or more candidates at a row's threshold than its buffers
  * hold): 0 in normal operation; the results are correct either way. */
 uint32_t glide_tc_knn_fallbacks(const glide_ctx *ctx);
+/* What the context's calls of exact kNN got from tensor-core candidates (truth_tc.cu) so far: [0] queries
+ * of glide_bruteforce_knn that were given to them, [1] of those, queries answered by the fp32 tile kernel
+ * after all; [2], [3] the same for the rows of kNN stages. */
+void glide_exact_knn_counts(const glide_ctx *ctx, uint64_t out[4]);
+/* Bounds the scratch that such calls take, by the size of their passes: base rows and queries of a
+ * glide_bruteforce_knn call, values in the padded copy of rows whose length or address TMA cannot read, and
+ * 128-row tiles of a kNN stage's launches. 0 leaves a bound at its default. Results do not depend on it. */
+int glide_limit_exact_knn(glide_ctx *ctx, uint32_t base_rows, uint32_t queries, uint32_t padded_values, uint32_t tiles);
 
 /* ---- matrix files ----------------------------------------------------------------------- */
 /* load_matrix_data, load.cuh:10-30 (u32 rows, u32 dim, then the rows; the reference reads row by

@@ -76,3 +76,81 @@ def test_partition_graphs_from_the_tensor_cores_are_the_tile_kernels(gpu_ctx, ki
             for r in range(q, hi):
                 want = [i for i in ids[r - q] if i != r][:k]
                 assert list(got[lo + r][:k]) == want
+
+
+@pytest.fixture
+def short_passes(gpu_ctx):
+    """Passes of a few hundred rows, so that small inputs take several of each kind."""
+    def set_passes(**sizes):
+        gpu_ctx.limit_exact_knn(**sizes)
+        return gpu_ctx
+    yield set_passes
+    gpu_ctx.limit_exact_knn()
+
+
+def _tile_kernel(ctx, base, queries, k, metric=Metric.Euclidean):
+    """bruteforce_tile_kernel on every query: slices below the line between it and the tensor cores."""
+    n, dim = base.shape
+    few = max(1, ((1 << 20) - 1) // (n * dim))
+    before = ctx.exact_knn_counts
+    got = [api.bruteforce_knn(ctx, base, queries[lo:lo + few].contiguous(), k, metric) for lo in range(0, queries.shape[0], few)]
+    assert ctx.exact_knn_counts == before      # none of them went through the tensor cores
+    return torch.cat([g[0] for g in got]), torch.cat([g[1] for g in got])
+
+
+@pytest.mark.parametrize("kind", ["uniform", "ties", "unit"])
+@pytest.mark.parametrize("dim", [64, 33])
+@pytest.mark.parametrize("k", [1, 10, 100])
+def test_several_passes_give_the_tile_kernels_results(short_passes, kind, dim, k):
+    """Three passes over the base rows (the last one ragged; equal rows on both sides of a boundary) times three over
+    the queries."""
+    rng = np.random.default_rng(dim + k)
+    base = _rows(kind, rng, 1409, dim)
+    base[512] = base[511]
+    base[1024:1030] = base[100]
+    queries = _rows(kind, rng, 300, dim)
+    queries[7], queries[299] = base[511], base[1024]
+    ctx = short_passes(base_rows=512, queries=128)
+    base, queries = (torch.from_numpy(x).to(ctx.torch_device) for x in (base, queries))
+    before = ctx.exact_knn_counts
+    ids, dists = api.bruteforce_knn(ctx, base, queries, k)
+    after = ctx.exact_knn_counts
+    assert after[0] - before[0] == 300 and after[1] == before[1]     # all from the tensor cores' candidates
+    want_ids, want = _tile_kernel(ctx, base, queries, k)
+    assert torch.equal(ids, want_ids)
+    assert torch.equal(dists.view(torch.int32), want.view(torch.int32))
+
+
+def test_passes_cut_by_the_padded_copy_give_the_tile_kernels_results(short_passes):
+    rng = np.random.default_rng(3)
+    ctx = short_passes(padded_values=36 * 500)
+    base = torch.from_numpy(_rows("uniform", rng, 1700, 35)).to(ctx.torch_device)
+    queries = torch.from_numpy(_rows("uniform", rng, 150, 35)).to(ctx.torch_device)
+    before = ctx.exact_knn_counts
+    ids, dists = api.bruteforce_knn(ctx, base, queries, 20)
+    after = ctx.exact_knn_counts
+    assert after[0] - before[0] == 150 and after[1] == before[1]
+    want_ids, want = _tile_kernel(ctx, base, queries, 20)
+    assert torch.equal(ids, want_ids) and torch.equal(dists, want)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "ties"])
+@pytest.mark.parametrize("dim,degree", [(36, 32), (33, 16)])
+def test_several_launches_over_partitions_give_the_tile_kernels_graph(short_passes, kind, dim, degree):
+    lens = np.array([2000, 129, 1400, 1, 600], np.uint32)
+    start = np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.uint32)
+    ctx = short_passes(tiles=4)
+    rows = torch.from_numpy(_rows(kind, np.random.default_rng(dim), int(lens.sum()), dim)).to(ctx.torch_device)
+    before = ctx.exact_knn_counts
+    got, _, _ = api.build_nnd(ctx, NNDescentParameter(degree), rows, start, lens, exact_max_rows=16384)
+    after = ctx.exact_knn_counts
+    assert after[2] - before[2] == int(lens.sum()) and after[3] == before[3]
+    got = got.cpu().numpy()
+    for lo, n in zip(start, lens):
+        k = min(degree, int(n) - 1)
+        if k == 0:
+            continue
+        part = rows[int(lo):int(lo) + int(n)].contiguous()
+        ids, _ = _tile_kernel(ctx, part, part, k + 1)
+        for r, row in enumerate(ids.cpu().numpy()):
+            assert list(got[int(lo) + r][:k]) == [i for i in row if i != r][:k]
