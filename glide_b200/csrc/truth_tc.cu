@@ -7,8 +7,9 @@
 //              in shared memory where they fit (up to 256 values a row), otherwise they ride along with the
 //              rows'. tcgen05.mma kind::tf32 accumulates the 128 x 128 dot products in tensor memory (two
 //              buffers), sixteen epilogue warps turn them into a = |b|^2 - 2 q.b (thread (query, part): 32 columns).
-//   threshold  a pass over every stride-th tile keeps the minima of runs of columns; the k-th smallest of
-//              them, t, is an upper bound of the k-th smallest a. The true k nearest then have a <= t + 2E, where E
+//   threshold  a pass over every stride-th row keeps minima over groups of rows that lie tiles apart (rows that are
+//              neighbours in the file are often neighbours in space; a group has few of a query's k nearest rows even
+//              where the file is sorted by cluster); the k-th smallest of them, t, is an upper bound of the k-th smallest a. The true k nearest then have a <= t + 2E, where E
 //              bounds |a + |q|^2 - d| for the fp32 distance d (tf32 rounding by Cauchy's inequality from the
 //              norms of what it drops, which is nothing for integers below 2048; sums by their length).
 //   select     the pass over all tiles stores every column with a <= t + 2E.
@@ -52,16 +53,18 @@ struct TruthStats {
 };
 
 // A CTA's share of a partition's own kNN graph (segment form): rows [first, first + 128) of the partition are the
-// queries, all of its rows the base; `stride`, `group` and `groups` are the sample's, as in TruthArgs.
+// queries, all of its rows the base; `stride`, `span` and `runs` are the sample's, as in TruthArgs.
 struct SegmentTile {
-    uint32_t seg_start, seg_len, first, stride, group, groups;
+    uint32_t seg_start, seg_len, first, stride, span, runs;
 };
 
 struct TruthArgs {
     uint32_t n, Q, dim, kblocks, stages, cap;
     const SegmentTile *segments;             // segment form: one per CTA; per-query arrays are indexed by CTA * 128 + row
-    uint32_t slices, stride;                 // CTA (query tile, slice) takes sampled tiles slice, slice + slices, ...; tile = index * stride
-    uint32_t group, groups;                  // columns per minimum, minima per query (sample pass)
+    uint32_t slices;                         // CTA (query tile, slice) takes tiles slice, slice + slices, ...
+    // sample pass: column c stands for row c * stride; a thread keeps the minima of its columns over `span` of its tiles,
+    // takes the minimum of every `fold` of them and stores those, for each of `runs` such spans; `groups` minima per query
+    uint32_t stride, span, runs, fold, groups;
     bool sample;
     const float *norms;
     const float *thr;                        // per query (select pass)
@@ -123,21 +126,35 @@ __global__ void truth_rows_kernel(const float *__restrict__ data, uint32_t rows,
     }
 }
 
-template<int GS>
-__device__ __forceinline__ void run_minima(const float (&e)[32], float *out) {
-    float m = FLT_MAX;
+// 32 / fold minima, 16-byte aligned; m is FLT_MAX again afterwards.
+__device__ __forceinline__ void store_minima(float (&m)[32], uint32_t fold, float *out) {
+    if (fold >= 2u) {
 #pragma unroll
-    for (int j = 0; j < 32; j++) {
-        m = fminf(m, e[j]);
-        if ((j + 1) % GS == 0) {
-            out[j / GS] = m;
-            m = FLT_MAX;
-        }
+        for (int j = 0; j < 16; j++) m[j] = fminf(m[j], m[j + 16]);
     }
+    if (fold >= 4u) {
+#pragma unroll
+        for (int j = 0; j < 8; j++) m[j] = fminf(m[j], m[j + 8]);
+    }
+    if (fold >= 8u) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) m[j] = fminf(m[j], m[j + 4]);
+    }
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+        if (out != nullptr && (uint32_t) j < 32u / fold) *reinterpret_cast<float4 *>(out + j) = make_float4(m[j], m[j + 1], m[j + 2], m[j + 3]);
+    }
+#pragma unroll
+    for (int j = 0; j < 32; j++) m[j] = FLT_MAX;
 }
 
+constexpr uint32_t kMaxStride = 16;
+struct SampleMaps {
+    CUtensorMap of[kMaxStride];              // by stride - 1
+};
+
 __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthArgs a, const __grid_constant__ CUtensorMap tm_q,
-                                                                   const __grid_constant__ CUtensorMap tm_b) {
+                                                                   const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ SampleMaps tm_s) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t) 1023);
     const uint32_t kblocks = a.kblocks, stages = a.stages;
@@ -152,14 +169,14 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const bool seg = a.segments != nullptr;
-    const SegmentTile part_of = seg ? a.segments[blockIdx.x] : SegmentTile{0, a.n, 0, a.stride, a.group, a.groups};
+    const SegmentTile part_of = seg ? a.segments[blockIdx.x] : SegmentTile{0, a.n, 0, a.stride, a.span, a.runs};
     const uint32_t qtiles = seg ? 1u : (a.Q + kTile - 1) / kTile;
     const uint32_t q0 = seg ? blockIdx.x * kTile : (blockIdx.x % qtiles) * kTile;      // index of the first query's results
     const uint32_t q_row = seg ? part_of.seg_start + part_of.first : q0;                // its row in the query map
     const uint32_t slice = seg ? 0u : blockIdx.x / qtiles, slices = seg ? 1u : a.slices;
-    const uint32_t n = part_of.seg_len, b_row = part_of.seg_start, stride = a.sample ? part_of.stride : 1u;
-    const uint32_t all = (n + kTile - 1) / kTile, taken = (all + stride - 1) / stride;
-    const uint32_t tiles = slice < taken ? (taken - slice + slices - 1) / slices : 0u;   // of this CTA
+    const uint32_t b_row = part_of.seg_start, stride = a.sample ? part_of.stride : 1u;
+    const uint32_t n = part_of.seg_len / stride, all = (n + kTile - 1) / kTile;             // columns, tiles of them
+    const uint32_t tiles = slice < all ? (all - slice + slices - 1) / slices : 0u;          // of this CTA
 
     if (tid == 0) {
         mbar_init(a_full, 1);
@@ -187,12 +204,13 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
             uint32_t s = 0, use = 0;
             bool ok = true;
             for (uint32_t t = 0; t < tiles && ok; t++) {
-                const uint32_t row0 = b_row + (slice + t * slices) * stride * kTile;
+                const uint32_t c0 = (slice + t * slices) * kTile;
                 for (uint32_t kb = 0; kb < kblocks; kb++) {
                     if (use > 0 && !mbar_wait(freed + s, (use - 1) & 1u, failed)) { ok = false; break; }
                     uint8_t *dst = ring + s * stage_bytes;
                     mbar_expect_tx(full + s, stage_bytes);
-                    tma_load_2d(dst, &tm_b, kb * kBlock, row0, full + s);
+                    if (a.sample) tma_load_3d(dst, &tm_s.of[stride - 1u], kb * kBlock, b_row % stride, b_row / stride + c0, full + s);
+                    else tma_load_2d(dst, &tm_b, kb * kBlock, b_row + c0, full + s);
                     if (!resident) tma_load_2d(dst + kBlockBytes, &tm_q, kb * kBlock, q_row, full + s);
                     if (++s == stages) { s = 0; use++; }
                 }
@@ -225,20 +243,25 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
     } else {
         // ================= epilogue: thread (query, part) owns 32 columns of every tile =================
         const uint32_t quad = warp & 3u, part = warp >> 2, q = q0 + quad * 32u + lane;
-        const bool active = seg ? part_of.first + quad * 32u + lane < n : q < a.Q;
+        const bool active = seg ? part_of.first + quad * 32u + lane < part_of.seg_len : q < a.Q;
         const float thr = (active && !a.sample) ? __ldg(a.thr + q) : 0.0f;
         float *cn = cn_w + warp * 32u;
         auto norm_of = [&](uint32_t t) {
-            const uint32_t c = (slice + t * slices) * stride * kTile + part * 32u + lane;
-            return t < tiles && c < n ? __ldg(a.norms + b_row + c) : 0.0f;
+            const uint32_t c = (slice + t * slices) * kTile + part * 32u + lane;
+            return t < tiles && c < n ? __ldg(a.norms + b_row + c * stride) : 0.0f;
         };
         float ahead = norm_of(0);
+        float m[32];
+#pragma unroll
+        for (int j = 0; j < 32; j++) m[j] = FLT_MAX;
+        uint32_t run = 0, left = part_of.span;
+        float *minima = active ? a.gmin + (uint64_t) q * a.groups + (slice * part_of.runs * kTile + part * 32u) / a.fold : nullptr;
         for (uint32_t t = 0; t < tiles; t++) {
             __syncwarp();
             cn[lane] = ahead;
             ahead = norm_of(t + 1);
             __syncwarp();
-            const uint32_t acc = t & 1u, index = slice + t * slices, c0 = index * stride * kTile + part * 32u;
+            const uint32_t acc = t & 1u, c0 = (slice + t * slices) * kTile + part * 32u;
             bool ok = !*failed && mbar_wait(mma_done + acc, (t >> 1) & 1u, failed);
             ok = __all_sync(kFullMask, ok);
             if (!ok) break;
@@ -262,22 +285,19 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
                 for (int j = 0; j < 32; j++)
                     if (c0 + j >= n) e[j] = FLT_MAX;
             }
-            if (!active) continue;
             if (a.sample) {
-                float *out = a.gmin + (uint64_t) q * a.groups + (index * kTile + part * 32u) / part_of.group;
-                switch (part_of.group) {
-                    case 1: run_minima<1>(e, out); break;
-                    case 2: run_minima<2>(e, out); break;
-                    case 4: run_minima<4>(e, out); break;
-                    case 8: run_minima<8>(e, out); break;
-                    case 16: run_minima<16>(e, out); break;
-                    default: run_minima<32>(e, out); break;
-                }
-            } else {
-                float m = e[0];
 #pragma unroll
-                for (int j = 1; j < 32; j++) m = fminf(m, e[j]);
-                if (m <= thr) {   // rare
+                for (int j = 0; j < 32; j++) m[j] = fminf(m[j], e[j]);
+                if (--left == 0 || t + 1 == tiles) {
+                    store_minima(m, a.fold, minima ? minima + run * (kTile / a.fold) : nullptr);
+                    run++;
+                    left = part_of.span;
+                }
+            } else if (active) {
+                float least = e[0];
+#pragma unroll
+                for (int j = 1; j < 32; j++) least = fminf(least, e[j]);
+                if (least <= thr) {   // rare
 #pragma unroll
                     for (int j = 0; j < 32; j++) {
                         if (e[j] <= thr && c0 + j < n) {
@@ -288,6 +308,8 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
                 }
             }
         }
+        if (a.sample)   // spans that this CTA has no tile for
+            for (; run < part_of.runs; run++) store_minima(m, a.fold, minima ? minima + run * (kTile / a.fold) : nullptr);
         if (*failed && lane == 0) atomicExch(&a.stats->failed, 1u);
     }
     fence_before();
@@ -315,7 +337,7 @@ __global__ void __launch_bounds__(128) truth_threshold_kernel(const float *__res
         const uint32_t r = t.first + q % kTile;
         if (r >= t.seg_len) return;
         row = t.seg_start + r;
-        groups = t.groups;
+        groups = t.runs * kTile;
         k = min(k, t.seg_len);
     }
     float kth;
@@ -453,27 +475,42 @@ __global__ void __launch_bounds__(128) segment_rerank_kernel(const float *__rest
 
 size_t up256(size_t x) { return (x + 255) & ~(size_t) 255; }
 
-// The sample of a pass over n rows for k neighbours: every stride-th tile, minima over `group` columns. The select
-// pass lets about stride x k columns through, the sample costs 1 / stride of it: 16 where at least 64 k rows remain,
-// less for smaller sets; groups as wide as leaves 8 k of them, so that few of the k smallest share one.
+// The sample of a pass over n rows for k neighbours, taken by `slices` CTAs per query tile: every stride-th row. The
+// select pass lets about stride x k columns through, the sample costs 1 / stride of it: 16 where at least 64 k rows remain,
+// less for smaller sets. 8 k minima, so that few of the k smallest share one: a thread's 32 columns over as many tiles as
+// that leaves; where few queries spread over many CTAs give thousands more, a thread folds its columns. At least
+// min(k, n) minima have a row: with one tile all of its rows have a minimum each, with more the first one fills 128.
 struct Sample {
-    uint32_t stride, group, groups;
+    uint32_t stride, slices, span, runs, fold, groups;
 };
-Sample sample_of(uint32_t n, uint32_t k) {
+Sample sample_of(uint32_t n, uint32_t k, uint32_t slices) {
     Sample s;
-    s.stride = n / (64u * k);
-    s.stride = s.stride < 1 ? 1 : (s.stride > 16 ? 16 : s.stride);
-    const uint32_t tiles = (n + kTile - 1) / kTile, taken = (tiles + s.stride - 1) / s.stride;
-    s.group = 32;
-    while (s.group > 1 && taken * kTile / s.group < 8u * k) s.group >>= 1;
-    s.groups = taken * (kTile / s.group);
+    s.stride = std::min(std::max(n / (64u * k), 1u), kMaxStride);
+    const uint32_t tiles = (n / s.stride + kTile - 1) / kTile;
+    s.slices = std::min(slices, tiles);
+    const uint32_t per = (tiles + s.slices - 1) / s.slices;
+    const uint32_t runs = std::min(per, (8u * k + kTile * s.slices - 1) / (kTile * s.slices));
+    s.span = (per + runs - 1) / runs;
+    s.runs = (per + s.span - 1) / s.span;
+    s.fold = 1;
+    while (s.fold < 8 && s.slices * s.runs * kTile / s.fold > 4096u) s.fold *= 2;
+    s.groups = s.slices * s.runs * kTile / s.fold;
     return s;
 }
+
+uint32_t sm_count() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 1;
+    return (uint32_t) sms;
+}
+
+// CTAs per query tile of a pass: a full wave where the tiles suffice
+uint32_t slices_of(uint32_t nq, uint32_t sms) { return std::max(1u, sms / ((nq + kTile - 1) / kTile)); }
 
 struct TruthPlan {
     uint32_t nb, qb, pitch;     // rows and queries per pass, padded row length
     bool pad;
-    Sample sample;
+    Sample sample, sample_last;   // of a full pass over queries, of the last one
     size_t norms, rows, q_rows, q_norm, q_rest, thr, count, cand, gmin, best, stats, total;
 };
 
@@ -484,7 +521,9 @@ TruthPlan truth_plan(const TcPasses &passes, const float *base, const float *que
     p.nb = std::min(n, std::max(k, passes.base_rows));   // the first pass has k results
     if (p.pad && (uint64_t) p.nb * p.pitch > passes.padded_values) p.nb = std::max(k, passes.padded_values / p.pitch);
     p.qb = Q < passes.queries ? Q : passes.queries;
-    p.sample = sample_of(p.nb < n ? p.nb : n, k);
+    const uint32_t last = Q % p.qb ? Q % p.qb : p.qb, sms = sm_count();
+    p.sample = sample_of(p.nb, k, slices_of(p.qb, sms));
+    p.sample_last = sample_of(p.nb, k, slices_of(last, sms));
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t o = at; at += up256(bytes); return o; };
     p.stats = take(sizeof(TruthStats));
@@ -494,7 +533,7 @@ TruthPlan truth_plan(const TcPasses &passes, const float *base, const float *que
     p.thr = take((size_t) p.qb * 4);
     p.count = take((size_t) p.qb * 4);
     p.cand = take((size_t) p.qb * kCap * 4);
-    p.gmin = take((size_t) p.qb * p.sample.groups * 4);
+    p.gmin = take(std::max((size_t) p.qb * p.sample.groups, (size_t) last * p.sample_last.groups) * 4);
     p.best = take((size_t) p.qb * k * 8);
     p.rows = take(p.pad ? (size_t) p.nb * p.pitch * 4 : 0);
     p.q_rows = take(p.pad ? (size_t) p.qb * p.pitch * 4 : 0);
@@ -543,10 +582,8 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
     uint32_t *count = reinterpret_cast<uint32_t *>(w + p.count), *cand = reinterpret_cast<uint32_t *>(w + p.cand);
     u64 *best = reinterpret_cast<u64 *>(w + p.best);
     *h_failed = 1;
-    int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaMemsetAsync(stats, 0, sizeof(TruthStats), stream);
+    const uint32_t sms = sm_count();
+    cudaError_t e = cudaMemsetAsync(stats, 0, sizeof(TruthStats), stream);
     if (e != cudaSuccess) return e;
 
     TruthArgs a{};
@@ -564,6 +601,7 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
         float *q_padded = p.pad ? at(p.q_rows) : nullptr;
         truth_rows_kernel<<<(nq + 7) / 8, 256, 0, stream>>>(qrows, nq, dim, q_norm, q_rest, p.pitch, q_padded, nullptr);
         CUtensorMap tm_q, tm_b;
+        SampleMaps tm_s{};
         if (!row_map(&tm_q, p.pad ? q_padded : qrows, nq, p.pitch)) return cudaSuccess;
         a.Q = nq;
         const uint32_t qtiles = (nq + kTile - 1) / kTile;
@@ -571,28 +609,24 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
             const uint32_t nr = n - ba < p.nb ? n - ba : p.nb;
             const float *brows = base + (size_t) ba * dim;
             float *b_padded = p.pad ? at(p.rows) : nullptr;
-            const uint32_t blocks = (nr + 7) / 8 < 8u * (uint32_t) sms ? (nr + 7) / 8 : 8u * (uint32_t) sms;
+            const uint32_t blocks = std::min((nr + 7) / 8, 8u * sms);
             truth_rows_kernel<<<blocks, 256, 0, stream>>>(brows, nr, dim, norms, nullptr, p.pitch, b_padded, stats);
             if (!row_map(&tm_b, p.pad ? b_padded : brows, nr, p.pitch)) return cudaSuccess;
             a.n = nr;
-            auto launch = [&](uint32_t taken) {   // the CTAs of a pass over `taken` tiles: a full wave where the tiles suffice
-                a.slices = (uint32_t) sms / qtiles;
-                if (a.slices < 1) a.slices = 1;
-                if (a.slices > taken) a.slices = taken;
-                truth_umma_kernel<<<qtiles * a.slices, kTruthThreads, smem, stream>>>(a, tm_q, tm_b);
-            };
-            const uint32_t tiles = (nr + kTile - 1) / kTile;
             if (ba == 0) {
+                const Sample &m = nq == p.qb ? p.sample : p.sample_last;
+                if (!make_strided_row_map(&tm_s.of[m.stride - 1], p.pad ? b_padded : brows, nr, p.pitch, m.stride, kTile)) return cudaSuccess;
                 a.sample = true;
-                a.stride = p.sample.stride; a.group = p.sample.group; a.groups = p.sample.groups;
-                launch((tiles + a.stride - 1) / a.stride);
-                truth_threshold_kernel<<<nq, 128, (size_t) a.groups * 4, stream>>>(gmin, a.groups, k, nullptr, q_norm, q_rest, dim, nullptr, stats, thr, count);
+                a.slices = m.slices;
+                a.stride = m.stride; a.span = m.span; a.runs = m.runs; a.fold = m.fold; a.groups = m.groups;
+                truth_umma_kernel<<<qtiles * m.slices, kTruthThreads, smem, stream>>>(a, tm_q, tm_b, tm_s);
+                truth_threshold_kernel<<<nq, 128, (size_t) m.groups * 4, stream>>>(gmin, m.groups, k, nullptr, q_norm, q_rest, dim, nullptr, stats, thr, count);
             } else {
                 truth_threshold_kernel<<<nq, 128, 0, stream>>>(nullptr, 0, k, best, q_norm, q_rest, dim, nullptr, stats, thr, count);
             }
             a.sample = false;
-            a.stride = 1;
-            launch(tiles);
+            a.slices = std::min(slices_of(nq, sms), (nr + kTile - 1) / kTile);
+            truth_umma_kernel<<<qtiles * a.slices, kTruthThreads, smem, stream>>>(a, tm_q, tm_b, tm_s);
             const bool last = ba + nr == n;
             truth_rerank_kernel<<<nq, 128, rr_smem, stream>>>(base, ba, qrows, dim, cand, count, k, best, ba > 0, metric,
                                                               last ? out_ids + (size_t) qa * k : nullptr, last && out_dists ? out_dists + (size_t) qa * k : nullptr, stats);
@@ -620,7 +654,7 @@ SegPlan seg_plan(const TcPasses &passes, const float *data, uint32_t rows, uint3
     size_t tiles = 0;
     for (uint32_t s = 0; s < S; s++)
         if (h_len[s] > 0 && h_len[s] <= max_len) {
-            const uint32_t g = sample_of(h_len[s], out_degree + 1).groups;
+            const uint32_t g = sample_of(h_len[s], out_degree + 1, 1).groups;
             if (g > p.groups) p.groups = g;
             tiles += (h_len[s] + kTile - 1) / kTile;
         }
@@ -672,8 +706,8 @@ cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_
     std::vector<SegmentTile> tiles;
     for (uint32_t s = 0; s < S; s++) {
         if (h_len[s] == 0 || h_len[s] > max_len) continue;
-        const Sample m = sample_of(h_len[s], out_degree + 1);
-        for (uint32_t first = 0; first < h_len[s]; first += kTile) tiles.push_back(SegmentTile{h_start[s], h_len[s], first, m.stride, m.group, m.groups});
+        const Sample m = sample_of(h_len[s], out_degree + 1, 1);
+        for (uint32_t first = 0; first < h_len[s]; first += kTile) tiles.push_back(SegmentTile{h_start[s], h_len[s], first, m.stride, m.span, m.runs});
     }
     *h_failed = 0;
     if (tiles.empty()) return cudaSuccess;
@@ -685,7 +719,14 @@ cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_
     uint32_t *count = reinterpret_cast<uint32_t *>(w + p.count), *cand = reinterpret_cast<uint32_t *>(w + p.cand);
     float *padded = p.pad ? at(p.rows) : nullptr;
     CUtensorMap tm;
+    SampleMaps tm_s{};
     if (!row_map(&tm, p.pad ? padded : data, rows, p.pitch)) return cudaSuccess;
+    uint32_t mapped = 0;   // a bit per stride
+    for (const SegmentTile &t : tiles) {
+        if (mapped & (1u << t.stride)) continue;
+        mapped |= 1u << t.stride;
+        if (!make_strided_row_map(&tm_s.of[t.stride - 1], p.pad ? padded : data, rows, p.pitch, t.stride, kTile)) return cudaSuccess;
+    }
     cudaError_t e = cudaMemsetAsync(stats, 0, sizeof(TruthStats), stream);
     // the table is pageable host memory: the copy has read it when the call returns
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_tiles, tiles.data(), tiles.size() * sizeof(SegmentTile), cudaMemcpyHostToDevice, stream);
@@ -695,6 +736,7 @@ cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_
     TruthArgs a{};
     a.dim = dim; a.cap = kSegCap; a.kblocks = (p.pitch + kBlock - 1) / kBlock; a.stages = ring_stages(a.kblocks);
     a.groups = p.groups;
+    a.fold = 1;
     a.norms = at(p.norms); a.thr = at(p.thr); a.gmin = at(p.gmin); a.count = count; a.cand = cand; a.stats = stats;
     const size_t smem = umma_smem(a.stages), rr_smem = (size_t) kSegCap * 8 + (size_t) p.pitch * 4;
     if ((e = cudaFuncSetAttribute(truth_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
@@ -702,11 +744,11 @@ cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_
         const uint32_t n = (uint32_t) (tiles.size() - first < passes.tiles ? tiles.size() - first : passes.tiles);
         a.segments = d_tiles + first;
         a.sample = true;
-        truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm);
+        truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm, tm_s);
         truth_threshold_kernel<<<n * kTile, 128, (size_t) p.groups * 4, stream>>>(a.gmin, p.groups, out_degree + 1, nullptr, a.norms, at(p.rest), dim, a.segments,
                                                                                   stats, at(p.thr), count);
         a.sample = false;
-        truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm);
+        truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm, tm_s);
         segment_rerank_kernel<<<n * kTile, 128, rr_smem, stream>>>(data, dim, a.segments, cand, count, out_degree, row_base, out, stats);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }

@@ -103,6 +103,13 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const void *tmap, uint32_
                  "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(smem_u32(bar))
                  : "memory");
 }
+// The same of a 3-D map
+__device__ __forceinline__ void tma_load_3d(void *dst, const void *tmap, uint32_t x, uint32_t y, uint32_t z, uint64_t *bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+                     smem_u32(dst)),
+                 "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+                 : "memory");
+}
 // Shared-memory descriptor of a K-major operand with 128-byte swizzle: rows of 128 bytes, 8-row groups
 // 1024 bytes apart (what a TMA box of 32 floats x rows with CU_TENSOR_MAP_SWIZZLE_128B writes)
 __device__ __forceinline__ uint64_t desc_sw128(uint32_t smem_addr) {
@@ -143,6 +150,19 @@ inline bool make_row_map(CUtensorMap *tm, const float *ptr, uint64_t rows, uint3
     const cuuint32_t box[2] = {32, box_rows};
     const cuuint32_t elem[2] = {1, 1};
     return fn(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(ptr), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// The same rows as blocks of `stride`: box (x, y, z) holds row y of the blocks z, z + 1, ... (every stride-th row).
+// Rows behind the last whole block are outside.
+inline bool make_strided_row_map(CUtensorMap *tm, const float *ptr, uint64_t rows, uint32_t dim, uint32_t stride, uint32_t box_rows) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[3] = {dim, stride, rows / stride};
+    const cuuint64_t strides[2] = {(cuuint64_t) dim * 4, (cuuint64_t) dim * 4 * stride};
+    const cuuint32_t box[3] = {32, 1, box_rows};
+    const cuuint32_t elem[3] = {1, 1, 1};
+    return fn(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float *>(ptr), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 

@@ -154,3 +154,45 @@ def test_several_launches_over_partitions_give_the_tile_kernels_graph(short_pass
         ids, _ = _tile_kernel(ctx, part, part, k + 1)
         for r, row in enumerate(ids.cpu().numpy()):
             assert list(got[int(lo) + r][:k]) == [i for i in row if i != r][:k]
+
+
+def _sorted_by_cluster(rng, n, dim, size, spread=0.1):
+    """`size` adjacent rows around each of n / size centres."""
+    centres = rng.normal(0, 10, ((n + size - 1) // size, dim))
+    return (np.repeat(centres, size, axis=0)[:n] + rng.normal(0, spread, (n, dim))).astype(np.float32)
+
+
+@pytest.mark.parametrize("size,k", [(1000, 100), (300, 32), (64, 10)])
+def test_files_sorted_by_cluster_keep_their_candidates_few(gpu_ctx, size, k):
+    """A query's neighbours lie side by side in the file: sample and groups that follow the file's order would let many
+    clusters through."""
+    rng = np.random.default_rng(size)
+    base = _sorted_by_cluster(rng, 60_000, 16, size)
+    queries = base[rng.choice(60_000, 40, replace=False)] + rng.normal(0, 0.05, (40, 16)).astype(np.float32)
+    base, queries = (torch.from_numpy(x).to(gpu_ctx.torch_device) for x in (base, queries.astype(np.float32)))
+    before = gpu_ctx.exact_knn_counts
+    ids, dists = api.bruteforce_knn(gpu_ctx, base, queries, k)
+    after = gpu_ctx.exact_knn_counts
+    assert after[0] - before[0] == 40 and after[1] == before[1]
+    want_ids, want = _tile_kernel(gpu_ctx, base, queries, k)
+    assert torch.equal(ids, want_ids) and torch.equal(dists, want)
+
+
+@pytest.mark.parametrize("degree", [4, 32])
+def test_tiny_partitions_and_partitions_sorted_by_cluster_stay_with_the_candidates(gpu_ctx, degree):
+    lens = np.array([2, 3, 5, 8, 9000, 33], np.uint32)
+    start = np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.uint32)
+    rng = np.random.default_rng(degree)
+    rows = torch.from_numpy(_sorted_by_cluster(rng, int(lens.sum()), 36, 400)).to(gpu_ctx.torch_device)
+    before = gpu_ctx.exact_knn_counts
+    got, _, _ = api.build_nnd(gpu_ctx, NNDescentParameter(degree), rows, start, lens, exact_max_rows=16384)
+    after = gpu_ctx.exact_knn_counts
+    assert after[2] - before[2] == int(lens.sum()) and after[3] == before[3]
+    got = got.cpu().numpy()
+    for lo, n in zip(start, lens):
+        k = min(degree, int(n) - 1)
+        part = rows[int(lo):int(lo) + int(n)].contiguous()
+        check = np.arange(int(n)) if n < 100 else rng.choice(int(n), 60, replace=False)
+        ids, _ = _tile_kernel(gpu_ctx, part, part[torch.from_numpy(check).to(part.device)].contiguous(), k + 1)
+        for r, row in zip(check, ids.cpu().numpy()):
+            assert list(got[int(lo) + r][:k]) == [i for i in row if i != r][:k]
