@@ -123,7 +123,7 @@ static int build_nnd_simt(glide_ctx *ctx, const float *d_reorder_data, uint32_t 
                           const uint32_t *h_segment_start, const uint32_t *h_segment_length, uint32_t S, uint32_t knn_degree,
                           uint32_t K, uint32_t max_iterations, float termination_threshold, uint32_t sample,
                           uint32_t exact_max_rows, uint64_t seed, int metric, uint32_t row_base, int32_t *d_knn,
-                          uint32_t *iterations_run, bool skip_exact);
+                          uint32_t *iterations_run, bool skip_exact, bool skip_tc);
 
 int glide_ctx_create(int device, glide_ctx **out) {
     if (!out) return GLIDE_ERR_BAD_ARG;
@@ -510,24 +510,25 @@ int glide_build_nnd_range(glide_ctx *ctx, const float *d_reorder_data, uint32_t 
                 const float tc_ms = ctx->last_ms;
                 rc0 = build_nnd_simt(ctx, d_reorder_data, rows, dim, h_segment_start, h_segment_length, S, knn_degree, K,
                                      max_iterations, termination_threshold, sample, exact_max_rows, seed, metric, row_base,
-                                     d_knn, iterations_run, /*skip_exact=*/true);
+                                     d_knn, iterations_run, /*skip_exact=*/true, /*skip_tc=*/true);
                 ctx->last_ms += tc_ms;
                 return rc0;
             }
             // no tensor map, a wait that ran out, or a candidate buffer that overflowed: the fp32
-            // kernels redo everything; the time of the attempt stays in the stage's time
+            // kernels redo everything (at once: candidates from the other tensor-core path would overflow on the same
+            // rows); the time of the attempt stays in the stage's time
             if (exact_max_rows > 16384) exact_max_rows = 16384;
             const float tc_ms = ctx->last_ms;
             rc0 = build_nnd_simt(ctx, d_reorder_data, rows, dim, h_segment_start, h_segment_length, S, knn_degree, K,
                                  max_iterations, termination_threshold, sample, exact_max_rows, seed, metric, row_base, d_knn,
-                                 iterations_run, false);
+                                 iterations_run, false, /*skip_tc=*/true);
             ctx->last_ms += tc_ms;
             ctx->tc_knn_fallbacks++;
             return rc0;
         }
     }
     return build_nnd_simt(ctx, d_reorder_data, rows, dim, h_segment_start, h_segment_length, S, knn_degree, K, max_iterations,
-                          termination_threshold, sample, exact_max_rows, seed, metric, row_base, d_knn, iterations_run, false);
+                          termination_threshold, sample, exact_max_rows, seed, metric, row_base, d_knn, iterations_run, false, false);
 }
 
 uint32_t glide_tc_knn_fallbacks(const glide_ctx *ctx) { return ctx ? ctx->tc_knn_fallbacks : 0; }
@@ -547,18 +548,18 @@ int glide_limit_exact_knn(glide_ctx *ctx, uint32_t base_rows, uint32_t queries, 
     return GLIDE_OK;
 }
 
-// The fp32 kernels of the kNN stage: the register-tile all-pairs kernel for partitions of at most
-// exact_max_rows rows (unless skip_exact: the tensor-core kernel has done them) and NN-descent for the rest.
+// The kNN stage but for knn_tc.cu: partitions of at most exact_max_rows rows (unless skip_exact: they are done) from tensor-core
+// candidates where that serves them (unless skip_tc) and from the fp32 register-tile kernel otherwise, NN-descent for the rest.
 static int build_nnd_simt(glide_ctx *ctx, const float *d_reorder_data, uint32_t rows, uint32_t dim,
                           const uint32_t *h_segment_start, const uint32_t *h_segment_length, uint32_t S, uint32_t knn_degree,
                           uint32_t K, uint32_t max_iterations, float termination_threshold, uint32_t sample,
                           uint32_t exact_max_rows, uint64_t seed, int metric, uint32_t row_base, int32_t *d_knn,
-                          uint32_t *iterations_run, bool skip_exact) {
+                          uint32_t *iterations_run, bool skip_exact, bool skip_tc) {
     const uint32_t tile_count = skip_exact ? 0 : segment_knn_tile_count(h_segment_length, S, exact_max_rows);
     bool need_nnd = false;
     for (uint32_t s = 0; s < S; s++) need_nnd = need_nnd || h_segment_length[s] > exact_max_rows;
     const size_t nnd_bytes = need_nnd ? nnd_workspace_bytes(rows, K, sample, S) : 0;
-    bool tc = tile_count != 0 && segment_tc_eligible(d_reorder_data, rows, dim, h_segment_length, S, exact_max_rows, knn_degree);
+    bool tc = tile_count != 0 && !skip_tc && segment_tc_eligible(d_reorder_data, rows, dim, h_segment_length, S, exact_max_rows, knn_degree);
     const size_t tc_bytes = tc ? segment_tc_scratch_bytes(ctx->tc_passes, d_reorder_data, rows, dim, h_segment_length, S, exact_max_rows, knn_degree) : 0;
     size_t work_bytes = std::max(nnd_bytes, tc_bytes);   // one after the other
     const size_t tables = 2 * align256((size_t) S * 4) + align256((size_t) tile_count * 12) + 256;
@@ -574,28 +575,29 @@ static int build_nnd_simt(glide_ctx *ctx, const float *d_reorder_data, uint32_t 
     uint32_t *d_start = b.take<uint32_t>(S), *d_len = b.take<uint32_t>(S);
     uint32_t *d_tiles = b.take<uint32_t>((size_t) tile_count * 3 + 1);
     void *work = b.take<char>(work_bytes);
-    std::vector<uint32_t> h_tiles((size_t) tile_count * 3 + 1);
+    std::vector<uint32_t> h_tiles((size_t) tile_count * 3);
+    uint32_t by_tiles = tile_count;
     if (tile_count) segment_knn_fill_tiles(h_segment_start, h_segment_length, S, exact_max_rows, h_tiles.data());
     // empty segments (C == 1 leaves the boundary segment empty, partition_kernel.cuh:58) need no launch
     Timed timer(ctx);
     GL_CUDA(ctx, cudaMemcpyAsync(d_start, h_segment_start, (size_t) S * 4, cudaMemcpyHostToDevice, ctx->stream));
     GL_CUDA(ctx, cudaMemcpyAsync(d_len, h_segment_length, (size_t) S * 4, cudaMemcpyHostToDevice, ctx->stream));
     if (iterations_run) *iterations_run = 0;
-    uint32_t by_tiles = tile_count;
     if (tc) {
-        uint32_t failed = 1;
+        bool all = true;
+        std::vector<uint32_t> left;
         GL_CUDA(ctx, launch_segment_tc(ctx->tc_passes, d_reorder_data, rows, dim, h_segment_start, h_segment_length, S, exact_max_rows, knn_degree, row_base, work, d_knn,
-                                       &failed, ctx->stream));
-        if (!failed) by_tiles = 0;
+                                       &all, &left, ctx->stream));
         for (uint32_t s = 0; s < S; s++)
-            if (h_segment_length[s] <= exact_max_rows) {
-                ctx->exact_knn[2] += h_segment_length[s];
-                if (failed) ctx->exact_knn[3] += h_segment_length[s];
-            }
+            if (h_segment_length[s] <= exact_max_rows) ctx->exact_knn[2] += h_segment_length[s];
+        if (!all) h_tiles.swap(left);   // some of the tiles, or none
+        by_tiles = all ? tile_count : (uint32_t) (h_tiles.size() / 3);
+        for (uint32_t t = 0; t < by_tiles; t++) ctx->exact_knn[3] += std::min(64u, h_tiles[3 * t + 1] - h_tiles[3 * t + 2]);
+        if (by_tiles) ctx->tc_knn_fallbacks++;
     }
     if (by_tiles) {
-        GL_CUDA(ctx, cudaMemcpyAsync(d_tiles, h_tiles.data(), (size_t) tile_count * 12, cudaMemcpyHostToDevice, ctx->stream));
-        GL_CUDA(ctx, launch_segment_knn(d_reorder_data, dim, d_tiles, tile_count, knn_degree, row_base, d_knn, ctx->stream));
+        GL_CUDA(ctx, cudaMemcpyAsync(d_tiles, h_tiles.data(), (size_t) by_tiles * 12, cudaMemcpyHostToDevice, ctx->stream));
+        GL_CUDA(ctx, launch_segment_knn(d_reorder_data, dim, d_tiles, by_tiles, knn_degree, row_base, d_knn, ctx->stream));
     }
     if (!need_nnd) return timer.finish();
     NndArgs a{};
@@ -617,8 +619,8 @@ int glide_bruteforce_knn(glide_ctx *ctx, const float *d_base, uint32_t n, const 
     GL_CUDA(ctx, cudaSetDevice(ctx->device));
     const uint32_t splits = bruteforce_default_splits(n, q);
     bool tc = q > 0 && truth_tc_eligible(n, q, dim, k);
-    const size_t need = bruteforce_scratch_bytes(q, k, splits) + 256;
-    int rc = ensure_ws(ctx, tc ? std::max(need, truth_tc_scratch_bytes(ctx->tc_passes, d_base, d_queries, n, q, dim, k)) : need);
+    const size_t need = bruteforce_scratch_bytes(q, k, splits) + 256, listed = align256((size_t) q * 4);
+    int rc = ensure_ws(ctx, tc ? std::max(listed + need, truth_tc_scratch_bytes(ctx->tc_passes, d_base, d_queries, n, q, dim, k)) : need);
     if (tc && rc == GLIDE_ERR_NO_MEMORY) {   // the tile kernel asks for less
         cudaGetLastError();
         tc = false;
@@ -627,11 +629,18 @@ int glide_bruteforce_knn(glide_ctx *ctx, const float *d_base, uint32_t n, const 
     if (rc) return rc;
     Timed timer(ctx);
     if (tc) {
-        uint32_t failed = 1;
-        GL_CUDA(ctx, launch_truth_tc(ctx->tc_passes, d_base, n, d_queries, q, dim, k, metric, ctx->ws, d_out_ids, d_out_dists, &failed, ctx->stream));
+        uint32_t left[2] = {1, 0};
+        GL_CUDA(ctx, launch_truth_tc(ctx->tc_passes, d_base, n, d_queries, q, dim, k, metric, ctx->ws, d_out_ids, d_out_dists, left, ctx->stream));
         ctx->exact_knn[0] += q;
-        if (!failed) return timer.finish();
-        ctx->exact_knn[1] += q;
+        ctx->exact_knn[1] += left[0] ? q : left[1];
+        if (!left[0]) {
+            if (left[1] == 0) return timer.finish();
+            // the queries it lists, in the scratch behind the list: as many slices of the base as fit there
+            const uint32_t few = left[1], fit = (uint32_t) ((uint64_t) q * splits / few);
+            GL_CUDA(ctx, launch_bruteforce(d_base, n, d_queries, few, dim, k, metric, std::min(bruteforce_default_splits(n, few), fit),
+                                           static_cast<char *>(ctx->ws) + listed, d_out_ids, d_out_dists, ctx->stream, static_cast<uint32_t *>(ctx->ws)));
+            return timer.finish();
+        }
     }
     GL_CUDA(ctx, launch_bruteforce(d_base, n, d_queries, q, dim, k, metric, splits, ctx->ws, d_out_ids, d_out_dists, ctx->stream));
     return timer.finish();

@@ -59,7 +59,7 @@ __device__ __forceinline__ void list_insert(float *ld, uint32_t *li, uint32_t k,
 __global__ void __launch_bounds__(256) bruteforce_tile_kernel(const float *__restrict__ base, uint32_t n,
                                                               const float *__restrict__ queries, uint32_t Q,
                                                               uint32_t dim, uint32_t k, uint32_t splits,
-                                                              Cand *__restrict__ partial) {
+                                                              Cand *__restrict__ partial, const uint32_t *__restrict__ list) {
     extern __shared__ __align__(16) uint32_t smem[];
     float *Qs = reinterpret_cast<float *>(smem);                  // [kKT][kQPad]
     float *Bs = Qs + kKT * kQPad;                                 // [kKT][kBPad]
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(256) bruteforce_tile_kernel(const float *__res
             for (uint32_t e = tid; e < kQT * kKT; e += 256) {
                 const uint32_t row = e / kKT, kk = e % kKT;
                 const uint32_t q = q0 + row, d = k0 + kk;
-                Qs[kk * kQPad + row] = (q < Q && d < dim) ? __ldg(queries + (uint64_t) q * dim + d) : 0.0f;
+                Qs[kk * kQPad + row] = (q < Q && d < dim) ? __ldg(queries + (uint64_t) (list ? __ldg(list + q) : q) * dim + d) : 0.0f;
             }
             for (uint32_t e = tid; e < kBT * kKT; e += 256) {
                 const uint32_t row = e / kKT, kk = e % kKT;
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(256) bruteforce_tile_kernel(const float *__res
 // One warp per query folds the per-split lists.
 __global__ void __launch_bounds__(128) bruteforce_merge_kernel(const Cand *__restrict__ partial, uint32_t Q, uint32_t k,
                                                                uint32_t splits, int metric, uint32_t *out_ids,
-                                                               float *out_dists) {
+                                                               float *out_dists, const uint32_t *__restrict__ list) {
     extern __shared__ __align__(16) uint32_t smem[];
     const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
     const uint32_t q = blockIdx.x * (blockDim.x >> 5) + warp;
@@ -167,9 +167,10 @@ __global__ void __launch_bounds__(128) bruteforce_merge_kernel(const Cand *__res
         const Cand cd = src[c];
         if (cd.id != kInvalid) list_insert(ld, li, k, cd.d, cd.id);
     }
+    const uint64_t row = list ? list[q] : q;
     for (uint32_t i = lane; i < k; i += 32) {
-        out_ids[(uint64_t) q * k + i] = li[i];
-        if (out_dists) out_dists[(uint64_t) q * k + i] = finish_metric(ld[i], metric);
+        out_ids[row * k + i] = li[i];
+        if (out_dists) out_dists[row * k + i] = finish_metric(ld[i], metric);
     }
 }
 
@@ -333,7 +334,7 @@ size_t bruteforce_scratch_bytes(uint32_t Q, uint32_t k, uint32_t splits) {
 
 cudaError_t launch_bruteforce(const float *base, uint32_t n, const float *queries, uint32_t Q, uint32_t dim,
                               uint32_t k, int metric, uint32_t splits, void *scratch, uint32_t *out_ids,
-                              float *out_dists, cudaStream_t stream) {
+                              float *out_dists, cudaStream_t stream, const uint32_t *list) {
     if (Q == 0) return cudaSuccess;
     if (k == 0 || k > kMaxK || k > n || splits == 0) return cudaErrorInvalidValue;
     const size_t smem_bytes = tile_smem_bytes(k);
@@ -342,12 +343,12 @@ cudaError_t launch_bruteforce(const float *base, uint32_t n, const float *querie
     if (e != cudaSuccess) return e;
     const dim3 grid((Q + kQT - 1) / kQT, splits);
     bruteforce_tile_kernel<<<grid, 256, smem_bytes, stream>>>(base, n, queries, Q, dim, k, splits,
-                                                             static_cast<Cand *>(scratch));
+                                                             static_cast<Cand *>(scratch), list);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const uint32_t warps = 4;
     bruteforce_merge_kernel<<<(Q + warps - 1) / warps, warps * 32, (size_t) warps * 2 * k * 4, stream>>>(
-        static_cast<const Cand *>(scratch), Q, k, splits, metric, out_ids, out_dists);
+        static_cast<const Cand *>(scratch), Q, k, splits, metric, out_ids, out_dists, list);
     return cudaGetLastError();
 }
 

@@ -15,8 +15,9 @@
 //   select     the pass over all tiles stores every column with a <= t + 2E.
 //   re-rank    their fp32 distances in the order of bruteforce_tile_kernel, sorted by (distance, id).
 //
-// A query with more candidates than its buffer holds (or fewer than k), a value that is no finite number, a tensor map
-// that cannot be made or a wait that runs out makes the caller fall back to bruteforce_tile_kernel.
+// A query with more candidates than its buffer holds (foreseen from the sample where it can be), or fewer than k, or with values
+// beyond the bounds, is left to bruteforce_tile_kernel, in the segment form with the 63 rows beside it to segment_knn_kernel; a
+// tensor map that cannot be made or a wait that runs out leaves everything to them.
 // Bound by the tensor pipe and, below it, by the trip of the row tiles from L2 (once per 128 queries).
 // bruteforce_tile_kernel against this: 1M x 128 rows, 1,000 queries, k = 10: 22.5 to 1.14 ms (0.22 of measured bf16
 // peak is what tf32 gives at best: 0.36 ms of it), k = 100: 39.1 to 2.29 ms; 100,000 x 960, 333 queries 6.5 to 0.55 ms;
@@ -46,16 +47,29 @@ constexpr uint32_t kCap = 3968;              // candidates per query; with up to
 constexpr uint32_t kSegCap = 2048;           // candidates per row of a segment call
 constexpr uint32_t kSegRows = 1u << 21;      // rows of the largest partition of a segment call
 
-struct TruthStats {
-    uint32_t max_norm, max_rest;             // bits of the largest |b|^2 and |b - tf32(b)|^2 (non-negative floats order as integers)
-    uint32_t failed;
-    uint32_t pad;
+// Largest |b|^2 and |b - tf32(b)|^2 of the base rows (of a partition), as bits: non-negative floats order as integers.
+struct TruthTops {
+    uint32_t norm, rest;
+};
+
+// Rows whose |b|^2 is no number below this are nobody's neighbour as long as the k-th smallest a is below kFarBound and
+// |q|^2 below kFarQuery: a >= |b| (|b| - 2 |q|) > 9e35 for them. Their norm is set to infinity, so that they meet no threshold,
+// and they count in no bound.
+constexpr float kFarNorm = 1e36f, kFarBound = 1e34f, kFarQuery = 1e32f;
+
+// What the call hands back: queries, or (segment form) halves of 64 rows of a tile, that have too many candidates, too few, or
+// values beyond the bounds. A query's `thr` is then -infinity: later kernels pass it by.
+struct TruthBad {
+    uint32_t *gave_up;                       // a wait ran out: everything
+    uint32_t *count, *items;
+    uint32_t *seen;                          // segment form: one flag per half, each is listed once
+    uint32_t first;                          // added to the queries of a pass
 };
 
 // A CTA's share of a partition's own kNN graph (segment form): rows [first, first + 128) of the partition are the
 // queries, all of its rows the base; `stride`, `span` and `runs` are the sample's, as in TruthArgs.
 struct SegmentTile {
-    uint32_t seg_start, seg_len, first, stride, span, runs;
+    uint32_t seg_start, seg_len, first, stride, span, runs, part, index;
 };
 
 struct TruthArgs {
@@ -71,20 +85,33 @@ struct TruthArgs {
     float *gmin;                             // Q x groups
     uint32_t *count;                         // per query
     uint32_t *cand;                          // Q x cap
-    TruthStats *stats;
+    uint32_t *gave_up;
 };
+
+__device__ __forceinline__ void report_bad(const TruthBad &bad, uint32_t item) {
+    if (bad.seen == nullptr || atomicExch(bad.seen + item, 1u) == 0u) bad.items[atomicAdd(bad.count, 1u)] = bad.first + item;
+}
 
 __device__ __forceinline__ float tf32_rest(float x) { return x - __uint_as_float(__float_as_uint(x) & 0xffffe000u); }
 
 // A warp per row: |x|^2, |x - tf32(x)|^2 (two floats per row if `rest` is given), the maxima, and the row padded to `pitch`.
+// Segment form: a CTA per tile, maxima per partition.
 __global__ void truth_rows_kernel(const float *__restrict__ data, uint32_t rows, uint32_t dim, float *norms, float *rest, uint32_t pitch,
-                                  float *padded, TruthStats *stats) {
+                                  float *padded, TruthTops *tops, const SegmentTile *__restrict__ segments) {
     __shared__ uint32_t top[2];
     if (threadIdx.x < 2) top[threadIdx.x] = 0;
     __syncthreads();
     const uint32_t lane = lane_id(), warps = blockDim.x >> 5;
     uint32_t best_n = 0, best_r = 0;
-    for (uint64_t r = (uint64_t) blockIdx.x * warps + (threadIdx.x >> 5); r < rows; r += (uint64_t) gridDim.x * warps) {
+    uint64_t first = (uint64_t) blockIdx.x * warps, end = rows, step = (uint64_t) gridDim.x * warps;
+    if (segments != nullptr) {
+        const SegmentTile t = segments[blockIdx.x];
+        first = t.seg_start + t.first;
+        end = t.seg_start + min(t.first + kTile, t.seg_len);
+        step = warps;
+        tops += t.part;
+    }
+    for (uint64_t r = first + (threadIdx.x >> 5); r < end; r += step) {
         const float *row = data + r * dim;
         float s = 0.0f, t = 0.0f;
         if (padded == nullptr) {
@@ -108,21 +135,24 @@ __global__ void truth_rows_kernel(const float *__restrict__ data, uint32_t rows,
             s += __shfl_xor_sync(kFullMask, s, off);
             t += __shfl_xor_sync(kFullMask, t, off);
         }
+        const bool far = !(s < kFarNorm);
         if (lane == 0) {
-            norms[r] = s;
-            if (rest) rest[r] = t;
+            norms[r] = far ? __int_as_float(0x7f800000) : s;
+            if (rest) rest[r] = far ? 0.0f : t;
         }
-        best_n = max(best_n, __float_as_uint(s));   // a NaN or an infinity is larger than any number and is caught with it
-        best_r = max(best_r, __float_as_uint(fabsf(t)));
+        if (!far) {
+            best_n = max(best_n, __float_as_uint(s));
+            best_r = max(best_r, __float_as_uint(t));
+        }
     }
     if (lane == 0) {
         atomicMax(&top[0], best_n);
         atomicMax(&top[1], best_r);
     }
     __syncthreads();
-    if (stats && threadIdx.x == 0) {
-        atomicMax(&stats->max_norm, top[0]);
-        atomicMax(&stats->max_rest, top[1]);
+    if (tops && threadIdx.x == 0) {
+        atomicMax(&tops->norm, top[0]);
+        atomicMax(&tops->rest, top[1]);
     }
 }
 
@@ -176,7 +206,9 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
     const uint32_t slice = seg ? 0u : blockIdx.x / qtiles, slices = seg ? 1u : a.slices;
     const uint32_t b_row = part_of.seg_start, stride = a.sample ? part_of.stride : 1u;
     const uint32_t n = part_of.seg_len / stride, all = (n + kTile - 1) / kTile;             // columns, tiles of them
-    const uint32_t tiles = slice < all ? (all - slice + slices - 1) / slices : 0u;          // of this CTA
+    // a query of the CTA, by thread: one that wants candidates?
+    bool wanted = tid < kTile && (seg ? part_of.first + tid < part_of.seg_len : q0 + tid < a.Q);
+    if (wanted && !a.sample) wanted = __ldg(a.thr + q0 + tid) != -__int_as_float(0x7f800000);
 
     if (tid == 0) {
         mbar_init(a_full, 1);
@@ -190,9 +222,10 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     fence_before();
-    __syncthreads();
+    const bool any_wanted = __syncthreads_or(wanted);
     fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tiles = any_wanted && slice < all ? (all - slice + slices - 1) / slices : 0u;   // of this CTA
 
     if (warp == kEpi + 1) {
         // ================= copies: one thread =================
@@ -243,8 +276,9 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
     } else {
         // ================= epilogue: thread (query, part) owns 32 columns of every tile =================
         const uint32_t quad = warp & 3u, part = warp >> 2, q = q0 + quad * 32u + lane;
-        const bool active = seg ? part_of.first + quad * 32u + lane < part_of.seg_len : q < a.Q;
+        bool active = seg ? part_of.first + quad * 32u + lane < part_of.seg_len : q < a.Q;
         const float thr = (active && !a.sample) ? __ldg(a.thr + q) : 0.0f;
+        active = active && thr != -__int_as_float(0x7f800000);
         float *cn = cn_w + warp * 32u;
         auto norm_of = [&](uint32_t t) {
             const uint32_t c = (slice + t * slices) * kTile + part * 32u + lane;
@@ -310,7 +344,7 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
         }
         if (a.sample)   // spans that this CTA has no tile for
             for (; run < part_of.runs; run++) store_minima(m, a.fold, minima ? minima + run * (kTile / a.fold) : nullptr);
-        if (*failed && lane == 0) atomicExch(&a.stats->failed, 1u);
+        if (*failed && lane == 0) atomicExch(a.gave_up, 1u);
     }
     fence_before();
     __syncthreads();
@@ -324,14 +358,17 @@ __device__ __forceinline__ uint32_t ordered(float x) {   // ascending floats as 
 __device__ __forceinline__ float from_ordered(uint32_t o) { return __uint_as_float((o & 0x80000000u) ? (o & 0x7fffffffu) : ~o); }
 
 // A CTA per query: the k-th smallest of its group minima (or, on later base passes, its k-th result so far) plus the error
-// bounds. Also clears the query's candidate counter.
+// bounds. Also clears the query's candidate counter. Where the sample says that far more rows than `cap` will meet the
+// threshold (`n` rows in all, `cols` of them sampled), the query is handed back before the pass over all tiles.
 __global__ void __launch_bounds__(128) truth_threshold_kernel(const float *__restrict__ gmin, uint32_t groups, uint32_t k, const u64 *__restrict__ best,
                                                               const float *__restrict__ q_norm, const float *__restrict__ q_rest, uint32_t dim,
-                                                              const SegmentTile *segments, TruthStats *stats, float *thr, uint32_t *count) {
+                                                              const SegmentTile *segments, const TruthTops *tops, uint32_t n, uint32_t cols, uint32_t cap,
+                                                              const TruthBad bad, float *thr, uint32_t *count) {
     extern __shared__ uint32_t keys[];
     __shared__ uint32_t below;
     const uint32_t q = blockIdx.x, tid = threadIdx.x;
-    uint32_t row = q, pitch = groups;   // the query's row in q_norm and q_rest, minima per query in gmin
+    uint32_t row = q, pitch = groups, item = q;   // the query's row in q_norm and q_rest, minima per query in gmin
+    if (best != nullptr && thr[q] == -__int_as_float(0x7f800000)) return;   // handed back by an earlier pass
     if (segments != nullptr) {
         const SegmentTile t = segments[q / kTile];
         const uint32_t r = t.first + q % kTile;
@@ -339,6 +376,10 @@ __global__ void __launch_bounds__(128) truth_threshold_kernel(const float *__res
         row = t.seg_start + r;
         groups = t.runs * kTile;
         k = min(k, t.seg_len);
+        n = t.seg_len;
+        cols = t.seg_len / t.stride;
+        tops += t.part;
+        item = 2u * t.index + (r - t.first) / (kTile / 2);
     }
     float kth;
     if (best == nullptr) {
@@ -360,17 +401,36 @@ __global__ void __launch_bounds__(128) truth_threshold_kernel(const float *__res
     } else {
         kth = __uint_as_float((uint32_t) (best[(uint64_t) q * k + k - 1] >> 32)) - q_norm[row];
     }
-    if (tid != 0) return;
     const float qn = sqrtf(q_norm[row]), ql = sqrtf(q_rest[row]);
-    const float bn = sqrtf(__uint_as_float(stats->max_norm)), bl = sqrtf(__uint_as_float(stats->max_rest));
+    const float bn = sqrtf(__uint_as_float(tops->norm)), bl = sqrtf(__uint_as_float(tops->rest));
     // |2 q.b - 2 tf32(q).tf32(b)| <= 2 (|q| |b - tf32(b)| + |q - tf32(q)| |b|); every sum (the two norms, the MMA's, the
     // fp32 distance) is within dim + 8 steps of 2^-23 of its terms' magnitudes, all below (|q| + |b|)^2
     const float sums = (float) (dim + 64u) * 4.0f * 1.1920929e-7f * (qn + bn) * (qn + bn);
     const float E = 1.001f * 2.0f * (qn * bl + ql * bn) + sums + 1e-30f;
     const float t = kth + 2.0f * E;
-    if (!(fabsf(t) < FLT_MAX) || !(bn < 1e18f) || !(qn < 1e18f)) atomicExch(&stats->failed, 1u);
-    thr[q] = t;
+    bool good = fabsf(t) < kFarBound && q_norm[row] < kFarQuery;
+    if (best == nullptr && n > cap) {
+        // of G groups that have a row, g have one at or below t: (1 - p)^(cols / G) = 1 - g / G for the share p of such rows
+        const uint32_t limit = ordered(t);
+        uint32_t g = 0, all = 0;
+        for (uint32_t i = tid; i < groups; i += 128) {
+            g += keys[i] <= limit ? 1u : 0u;
+            all += keys[i] < ordered(FLT_MAX) ? 1u : 0u;
+        }
+        if (tid == 0) below = 0;
+        __syncthreads();
+        g = __reduce_add_sync(kFullMask, g);
+        all = __reduce_add_sync(kFullMask, all);
+        if ((tid & 31u) == 0) atomicAdd(&below, (g << 16) | all);   // at most 4,096 groups
+        __syncthreads();
+        const float G = (float) (below & 0xffffu), share = fminf((float) (below >> 16), G - 0.5f) / G;
+        const float p = 1.0f - expf(logf(1.0f - share) * G / (float) cols);
+        if (p * (float) n > 1.25f * (float) cap) good = false;
+    }
+    if (tid != 0) return;
+    thr[q] = good ? t : -__int_as_float(0x7f800000);
     count[q] = 0;
+    if (!good) report_bad(bad, item);
 }
 
 // Ascending dimensions, one fused multiply-add each: the order of bruteforce_tile_kernel and segment_knn_kernel.
@@ -418,16 +478,23 @@ __device__ __forceinline__ void sort_keys(u64 *keys, uint32_t total) {
 // A CTA per query: exact distances of the candidates (and the earlier passes' results), sorted by (distance, id).
 __global__ void __launch_bounds__(128) truth_rerank_kernel(const float *__restrict__ base, uint32_t first_row, const float *__restrict__ queries, uint32_t dim,
                                                            const uint32_t *__restrict__ cand, const uint32_t *__restrict__ count, uint32_t k, u64 *best,
-                                                           bool earlier, int metric, uint32_t *out_ids, float *out_dists, TruthStats *stats) {
+                                                           bool earlier, int metric, uint32_t *out_ids, float *out_dists, float *thr, const TruthBad bad) {
     extern __shared__ __align__(16) uint32_t smem[];
     u64 *keys = reinterpret_cast<u64 *>(smem);                      // 4096
     float *query = reinterpret_cast<float *>(keys + 4096);          // dim
     const uint32_t q = blockIdx.x, tid = threadIdx.x;
     const uint32_t found = count[q], n = min(found, kCap);
     const uint32_t total = n + (earlier ? k : 0u);
-    if (tid == 0 && (found > kCap || total < k)) atomicExch(&stats->failed, 1u);
+    if (thr[q] == -__int_as_float(0x7f800000)) return;
     for (uint32_t d = tid; d < dim; d += 128) query[d] = queries[(uint64_t) q * dim + d];
     __syncthreads();
+    if (found > kCap || total < k) {
+        if (tid == 0) {
+            thr[q] = -__int_as_float(0x7f800000);
+            report_bad(bad, q);
+        }
+        return;
+    }
     for (uint32_t i = tid; i < n; i += 128) {
         const uint32_t id = first_row + cand[(uint64_t) q * kCap + i];
         keys[i] = ((u64) __float_as_uint(direct_distance(query, base + (uint64_t) id * dim, dim)) << 32) | id;
@@ -446,7 +513,7 @@ __global__ void __launch_bounds__(128) truth_rerank_kernel(const float *__restri
 // than out_degree others is padded with xorshift32(flat index) % partition size (nn_descent.cuh:1384-1391).
 __global__ void __launch_bounds__(128) segment_rerank_kernel(const float *__restrict__ data, uint32_t dim, const SegmentTile *__restrict__ segments,
                                                              const uint32_t *__restrict__ cand, const uint32_t *__restrict__ count, uint32_t out_degree,
-                                                             uint32_t row_base, int32_t *out, TruthStats *stats) {
+                                                             uint32_t row_base, int32_t *out, const float *__restrict__ thr, const TruthBad bad) {
     extern __shared__ __align__(16) uint32_t smem[];
     u64 *keys = reinterpret_cast<u64 *>(smem);                      // kSegCap
     float *query = reinterpret_cast<float *>(keys + kSegCap);       // dim
@@ -457,7 +524,11 @@ __global__ void __launch_bounds__(128) segment_rerank_kernel(const float *__rest
     const float *seg = data + (uint64_t) t.seg_start * dim;
     const uint32_t found = count[q], n = min(found, kSegCap);
     const uint32_t want = min(out_degree, t.seg_len - 1u);
-    if (tid == 0 && (found > kSegCap || n < want + 1u)) atomicExch(&stats->failed, 1u);
+    if (thr[q] == -__int_as_float(0x7f800000)) return;
+    if (found > kSegCap || n < want + 1u) {
+        if (tid == 0) report_bad(bad, 2u * t.index + (r - t.first) / (kTile / 2));
+        return;
+    }
     for (uint32_t d = tid; d < dim; d += 128) query[d] = seg[(uint64_t) r * dim + d];
     __syncthreads();
     for (uint32_t i = tid; i < n; i += 128) {
@@ -511,7 +582,7 @@ struct TruthPlan {
     uint32_t nb, qb, pitch;     // rows and queries per pass, padded row length
     bool pad;
     Sample sample, sample_last;   // of a full pass over queries, of the last one
-    size_t norms, rows, q_rows, q_norm, q_rest, thr, count, cand, gmin, best, stats, total;
+    size_t bad, items, tops, norms, rows, q_rows, q_norm, q_rest, thr, count, cand, gmin, best, total;
 };
 
 TruthPlan truth_plan(const TcPasses &passes, const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k) {
@@ -526,7 +597,9 @@ TruthPlan truth_plan(const TcPasses &passes, const float *base, const float *que
     p.sample_last = sample_of(p.nb, k, slices_of(last, sms));
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t o = at; at += up256(bytes); return o; };
-    p.stats = take(sizeof(TruthStats));
+    p.items = take((size_t) Q * 4);   // first: what it lists is answered from the rest of the scratch
+    p.bad = take(8 + sizeof(TruthTops));
+    p.tops = p.bad + 8;
     p.norms = take((size_t) p.nb * 4);
     p.q_norm = take((size_t) p.qb * 4);
     p.q_rest = take((size_t) p.qb * 4);
@@ -571,25 +644,28 @@ size_t truth_tc_scratch_bytes(const TcPasses &passes, const float *base, const f
     return truth_plan(passes, base, queries, n, Q, dim, k).total;
 }
 
-// *h_failed != 0: the caller computes the results by other means. Synchronises the stream.
+// What is left for the caller to answer by other means: h_left[0] != 0 everything, else h_left[1] queries, whose numbers lie at
+// the start of the scratch. Synchronises the stream.
 cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t n, const float *queries, uint32_t Q, uint32_t dim, uint32_t k, int metric,
-                            void *scratch, uint32_t *out_ids, float *out_dists, uint32_t *h_failed, cudaStream_t stream) {
+                            void *scratch, uint32_t *out_ids, float *out_dists, uint32_t (&h_left)[2], cudaStream_t stream) {
     const TruthPlan p = truth_plan(passes, base, queries, n, Q, dim, k);
     char *w = static_cast<char *>(scratch);
     auto at = [&](size_t o) { return reinterpret_cast<float *>(w + o); };
-    TruthStats *stats = reinterpret_cast<TruthStats *>(w + p.stats);
+    uint32_t *left = reinterpret_cast<uint32_t *>(w + p.bad);
+    TruthTops *tops = reinterpret_cast<TruthTops *>(w + p.tops);
+    TruthBad bad{left, left + 1, reinterpret_cast<uint32_t *>(w + p.items), nullptr, 0};
     float *norms = at(p.norms), *q_norm = at(p.q_norm), *q_rest = at(p.q_rest), *thr = at(p.thr), *gmin = at(p.gmin);
     uint32_t *count = reinterpret_cast<uint32_t *>(w + p.count), *cand = reinterpret_cast<uint32_t *>(w + p.cand);
     u64 *best = reinterpret_cast<u64 *>(w + p.best);
-    *h_failed = 1;
+    h_left[0] = 1;
     const uint32_t sms = sm_count();
-    cudaError_t e = cudaMemsetAsync(stats, 0, sizeof(TruthStats), stream);
+    cudaError_t e = cudaMemsetAsync(left, 0, 8 + sizeof(TruthTops), stream);
     if (e != cudaSuccess) return e;
 
     TruthArgs a{};
     a.dim = dim; a.cap = kCap; a.kblocks = (p.pitch + kBlock - 1) / kBlock;
     a.stages = ring_stages(a.kblocks);
-    a.norms = norms; a.thr = thr; a.gmin = gmin; a.count = count; a.cand = cand; a.stats = stats;
+    a.norms = norms; a.thr = thr; a.gmin = gmin; a.count = count; a.cand = cand; a.gave_up = bad.gave_up;
     const size_t smem = umma_smem(a.stages);
     if ((e = cudaFuncSetAttribute(truth_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
     const size_t rr_smem = 4096 * 8 + (size_t) p.pitch * 4;
@@ -599,7 +675,8 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
         const uint32_t nq = Q - qa < p.qb ? Q - qa : p.qb;
         const float *qrows = queries + (size_t) qa * dim;
         float *q_padded = p.pad ? at(p.q_rows) : nullptr;
-        truth_rows_kernel<<<(nq + 7) / 8, 256, 0, stream>>>(qrows, nq, dim, q_norm, q_rest, p.pitch, q_padded, nullptr);
+        truth_rows_kernel<<<(nq + 7) / 8, 256, 0, stream>>>(qrows, nq, dim, q_norm, q_rest, p.pitch, q_padded, nullptr, nullptr);
+        bad.first = qa;
         CUtensorMap tm_q, tm_b;
         SampleMaps tm_s{};
         if (!row_map(&tm_q, p.pad ? q_padded : qrows, nq, p.pitch)) return cudaSuccess;
@@ -610,7 +687,7 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
             const float *brows = base + (size_t) ba * dim;
             float *b_padded = p.pad ? at(p.rows) : nullptr;
             const uint32_t blocks = std::min((nr + 7) / 8, 8u * sms);
-            truth_rows_kernel<<<blocks, 256, 0, stream>>>(brows, nr, dim, norms, nullptr, p.pitch, b_padded, stats);
+            truth_rows_kernel<<<blocks, 256, 0, stream>>>(brows, nr, dim, norms, nullptr, p.pitch, b_padded, tops, nullptr);
             if (!row_map(&tm_b, p.pad ? b_padded : brows, nr, p.pitch)) return cudaSuccess;
             a.n = nr;
             if (ba == 0) {
@@ -620,20 +697,21 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
                 a.slices = m.slices;
                 a.stride = m.stride; a.span = m.span; a.runs = m.runs; a.fold = m.fold; a.groups = m.groups;
                 truth_umma_kernel<<<qtiles * m.slices, kTruthThreads, smem, stream>>>(a, tm_q, tm_b, tm_s);
-                truth_threshold_kernel<<<nq, 128, (size_t) m.groups * 4, stream>>>(gmin, m.groups, k, nullptr, q_norm, q_rest, dim, nullptr, stats, thr, count);
+                truth_threshold_kernel<<<nq, 128, (size_t) m.groups * 4, stream>>>(gmin, m.groups, k, nullptr, q_norm, q_rest, dim, nullptr, tops, nr, nr / m.stride, kCap,
+                                                                                       bad, thr, count);
             } else {
-                truth_threshold_kernel<<<nq, 128, 0, stream>>>(nullptr, 0, k, best, q_norm, q_rest, dim, nullptr, stats, thr, count);
+                truth_threshold_kernel<<<nq, 128, 0, stream>>>(nullptr, 0, k, best, q_norm, q_rest, dim, nullptr, tops, nr, 0, kCap, bad, thr, count);
             }
             a.sample = false;
             a.slices = std::min(slices_of(nq, sms), (nr + kTile - 1) / kTile);
             truth_umma_kernel<<<qtiles * a.slices, kTruthThreads, smem, stream>>>(a, tm_q, tm_b, tm_s);
             const bool last = ba + nr == n;
             truth_rerank_kernel<<<nq, 128, rr_smem, stream>>>(base, ba, qrows, dim, cand, count, k, best, ba > 0, metric,
-                                                              last ? out_ids + (size_t) qa * k : nullptr, last && out_dists ? out_dists + (size_t) qa * k : nullptr, stats);
+                                                              last ? out_ids + (size_t) qa * k : nullptr, last && out_dists ? out_dists + (size_t) qa * k : nullptr, thr, bad);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
     }
-    if ((e = cudaMemcpyAsync(h_failed, &stats->failed, 4, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
+    if ((e = cudaMemcpyAsync(h_left, left, 8, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
     return cudaStreamSynchronize(stream);
 }
 
@@ -643,7 +721,7 @@ namespace {
 struct SegPlan {
     bool pad;
     uint32_t pitch, groups;
-    size_t stats, tiles, norms, rest, thr, count, cand, gmin, rows, total;
+    size_t bad, items, seen, tops, tiles, norms, rest, thr, count, cand, gmin, rows, total;
 };
 
 SegPlan seg_plan(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree) {
@@ -651,9 +729,10 @@ SegPlan seg_plan(const TcPasses &passes, const float *data, uint32_t rows, uint3
     p.pad = (dim & 3u) != 0 || (reinterpret_cast<uintptr_t>(data) & 15u) != 0;
     p.pitch = (dim + 3u) & ~3u;
     p.groups = 1;
-    size_t tiles = 0;
+    size_t tiles = 0, parts = 0;
     for (uint32_t s = 0; s < S; s++)
         if (h_len[s] > 0 && h_len[s] <= max_len) {
+            parts++;
             const uint32_t g = sample_of(h_len[s], out_degree + 1, 1).groups;
             if (g > p.groups) p.groups = g;
             tiles += (h_len[s] + kTile - 1) / kTile;
@@ -661,7 +740,10 @@ SegPlan seg_plan(const TcPasses &passes, const float *data, uint32_t rows, uint3
     const size_t slots = (size_t) (tiles < passes.tiles ? tiles : passes.tiles) * kTile;
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t o = at; at += up256(bytes); return o; };
-    p.stats = take(sizeof(TruthStats));
+    p.bad = take(8 + 2 * tiles * 4 + parts * sizeof(TruthTops));
+    p.seen = p.bad + 8;
+    p.tops = p.seen + 2 * tiles * 4;
+    p.items = take(2 * tiles * 4);
     p.tiles = take(tiles * sizeof(SegmentTile));
     p.norms = take((size_t) rows * 4);
     p.rest = take((size_t) rows * 4);
@@ -698,23 +780,28 @@ size_t segment_tc_scratch_bytes(const TcPasses &passes, const float *data, uint3
     return seg_plan(passes, data, rows, dim, h_len, S, max_len, out_degree).total;
 }
 
-// Exact kNN rows of every partition of at most max_len rows: what segment_knn_kernel writes, bit for bit. *h_failed != 0: use
-// that kernel. Synchronises the stream.
+// Exact kNN rows of every partition of at most max_len rows: what segment_knn_kernel writes, bit for bit. What is left for that
+// kernel: *h_all everything, otherwise h_tiles, three words each (its tiles). Synchronises the stream.
 cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len,
-                              uint32_t S, uint32_t max_len, uint32_t out_degree, uint32_t row_base, void *scratch, int32_t *out, uint32_t *h_failed, cudaStream_t stream) {
+                              uint32_t S, uint32_t max_len, uint32_t out_degree, uint32_t row_base, void *scratch, int32_t *out, bool *h_all, std::vector<uint32_t> *h_tiles, cudaStream_t stream) {
     const SegPlan p = seg_plan(passes, data, rows, dim, h_len, S, max_len, out_degree);
     std::vector<SegmentTile> tiles;
+    uint32_t parts = 0;
     for (uint32_t s = 0; s < S; s++) {
         if (h_len[s] == 0 || h_len[s] > max_len) continue;
         const Sample m = sample_of(h_len[s], out_degree + 1, 1);
-        for (uint32_t first = 0; first < h_len[s]; first += kTile) tiles.push_back(SegmentTile{h_start[s], h_len[s], first, m.stride, m.span, m.runs});
+        for (uint32_t first = 0; first < h_len[s]; first += kTile) tiles.push_back(SegmentTile{h_start[s], h_len[s], first, m.stride, m.span, m.runs, parts, (uint32_t) tiles.size()});
+        parts++;
     }
-    *h_failed = 0;
+    h_tiles->clear();
+    *h_all = false;
     if (tiles.empty()) return cudaSuccess;
-    *h_failed = 1;
+    *h_all = true;
     char *w = static_cast<char *>(scratch);
     auto at = [&](size_t o) { return reinterpret_cast<float *>(w + o); };
-    TruthStats *stats = reinterpret_cast<TruthStats *>(w + p.stats);
+    uint32_t *left = reinterpret_cast<uint32_t *>(w + p.bad);
+    TruthTops *tops = reinterpret_cast<TruthTops *>(w + p.tops);
+    const TruthBad bad{left, left + 1, reinterpret_cast<uint32_t *>(w + p.items), reinterpret_cast<uint32_t *>(w + p.seen), 0};
     SegmentTile *d_tiles = reinterpret_cast<SegmentTile *>(w + p.tiles);
     uint32_t *count = reinterpret_cast<uint32_t *>(w + p.count), *cand = reinterpret_cast<uint32_t *>(w + p.cand);
     float *padded = p.pad ? at(p.rows) : nullptr;
@@ -727,17 +814,16 @@ cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_
         mapped |= 1u << t.stride;
         if (!make_strided_row_map(&tm_s.of[t.stride - 1], p.pad ? padded : data, rows, p.pitch, t.stride, kTile)) return cudaSuccess;
     }
-    cudaError_t e = cudaMemsetAsync(stats, 0, sizeof(TruthStats), stream);
+    cudaError_t e = cudaMemsetAsync(left, 0, 8 + 2 * tiles.size() * 4 + parts * sizeof(TruthTops), stream);
     // the table is pageable host memory: the copy has read it when the call returns
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_tiles, tiles.data(), tiles.size() * sizeof(SegmentTile), cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) return e;
-    const uint32_t blocks = (rows + 7) / 8 < 1184u ? (rows + 7) / 8 : 1184u;
-    truth_rows_kernel<<<blocks, 256, 0, stream>>>(data, rows, dim, at(p.norms), at(p.rest), p.pitch, padded, stats);
+    truth_rows_kernel<<<(uint32_t) tiles.size(), 256, 0, stream>>>(data, rows, dim, at(p.norms), at(p.rest), p.pitch, padded, tops, d_tiles);
     TruthArgs a{};
     a.dim = dim; a.cap = kSegCap; a.kblocks = (p.pitch + kBlock - 1) / kBlock; a.stages = ring_stages(a.kblocks);
     a.groups = p.groups;
     a.fold = 1;
-    a.norms = at(p.norms); a.thr = at(p.thr); a.gmin = at(p.gmin); a.count = count; a.cand = cand; a.stats = stats;
+    a.norms = at(p.norms); a.thr = at(p.thr); a.gmin = at(p.gmin); a.count = count; a.cand = cand; a.gave_up = bad.gave_up;
     const size_t smem = umma_smem(a.stages), rr_smem = (size_t) kSegCap * 8 + (size_t) p.pitch * 4;
     if ((e = cudaFuncSetAttribute(truth_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
     for (size_t first = 0; first < tiles.size(); first += passes.tiles) {
@@ -746,14 +832,25 @@ cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_
         a.sample = true;
         truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm, tm_s);
         truth_threshold_kernel<<<n * kTile, 128, (size_t) p.groups * 4, stream>>>(a.gmin, p.groups, out_degree + 1, nullptr, a.norms, at(p.rest), dim, a.segments,
-                                                                                  stats, at(p.thr), count);
+                                                                                  tops, 0, 0, kSegCap, bad, at(p.thr), count);
         a.sample = false;
         truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm, tm_s);
-        segment_rerank_kernel<<<n * kTile, 128, rr_smem, stream>>>(data, dim, a.segments, cand, count, out_degree, row_base, out, stats);
+        segment_rerank_kernel<<<n * kTile, 128, rr_smem, stream>>>(data, dim, a.segments, cand, count, out_degree, row_base, out, at(p.thr), bad);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    if ((e = cudaMemcpyAsync(h_failed, &stats->failed, 4, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
-    return cudaStreamSynchronize(stream);
+    uint32_t h_left[2] = {1, 0};
+    if ((e = cudaMemcpyAsync(h_left, left, 8, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
+    if ((e = cudaStreamSynchronize(stream)) != cudaSuccess || h_left[0]) return e;
+    *h_all = false;
+    if (h_left[1] == 0) return cudaSuccess;
+    std::vector<uint32_t> items(h_left[1]);
+    if ((e = cudaMemcpyAsync(items.data(), bad.items, items.size() * 4, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
+    if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
+    for (const uint32_t i : items) {
+        const SegmentTile &t = tiles[i / 2];
+        h_tiles->insert(h_tiles->end(), {t.seg_start, t.seg_len, t.first + (i % 2) * (kTile / 2)});
+    }
+    return cudaSuccess;
 }
 
 }  // namespace glide

@@ -215,9 +215,9 @@ int glide_comm_all_reduce_u64(glide_ctx *ctx, uint64_t *d_buf, uint64_t count, i
 /* Waits for everything enqueued on the context's stream (kernels, copies, collectives). */
 int glide_ctx_synchronize(glide_ctx *ctx);
 
-/* How many kNN stages of this context the tensor-core kernel gave back to the fp32 kernels (no
- * tensor map, a bounded wait that ran out, or more candidates at a row's threshold than its buffers
- * hold): 0 in normal operation; the results are correct either way. */
+/* How many kNN stages of this context the tensor-core kernels gave back to the fp32 kernels, whole or (where
+ * candidates come from truth_tc.cu) for some of their rows: no tensor map, a bounded wait that ran out, or more
+ * candidates at a row's threshold than its buffers hold. 0 in normal operation; the results are correct either way. */
 uint32_t glide_tc_knn_fallbacks(const glide_ctx *ctx);
 /* What the context's calls of exact kNN got from tensor-core candidates (truth_tc.cu) so far: [0] queries
  * of glide_bruteforce_knn that were given to them, [1] of those, queries answered by the fp32 tile kernel

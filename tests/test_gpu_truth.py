@@ -196,3 +196,77 @@ def test_tiny_partitions_and_partitions_sorted_by_cluster_stay_with_the_candidat
         ids, _ = _tile_kernel(gpu_ctx, part, part[torch.from_numpy(check).to(part.device)].contiguous(), k + 1)
         for r, row in zip(check, ids.cpu().numpy()):
             assert list(got[int(lo) + r][:k]) == [i for i in row if i != r][:k]
+
+
+def test_only_the_queries_that_overflow_or_hold_no_numbers_are_redone(gpu_ctx):
+    """5,000 equal rows are too many candidates for the queries beside them; rows that hold an infinity, no number or squares
+    beyond fp32 cost the other queries nothing."""
+    rng = np.random.default_rng(8)
+    n, dim, q, k = 20_000, 20, 120, 10
+    base, queries = rng.random((n, dim), np.float32), rng.random((q, dim), np.float32)
+    base[7000:12000] = base[7000] + np.float32(3)
+    base[3, 2], base[4000, 0], base[19_999, 5], base[150] = np.nan, np.inf, -np.inf, np.float32(2e19)
+    queries[[5, 64, 119]] = base[7000]
+    queries[10, 3], queries[11, 0] = np.nan, np.inf
+    base, queries = (torch.from_numpy(x).to(gpu_ctx.torch_device) for x in (base, queries))
+    before = gpu_ctx.exact_knn_counts
+    ids, dists = api.bruteforce_knn(gpu_ctx, base, queries, k)
+    after = gpu_ctx.exact_knn_counts
+    assert (after[0] - before[0], after[1] - before[1]) == (q, 5)
+    want_ids, want = _tile_kernel(gpu_ctx, base, queries, k)
+    assert torch.equal(ids, want_ids)
+    assert torch.equal(dists.view(torch.int32), want.view(torch.int32))
+
+
+def test_a_query_handed_back_in_one_pass_stays_so_in_the_next(short_passes):
+    rng = np.random.default_rng(9)
+    base, queries = rng.random((15_000, 24), np.float32), rng.random((200, 24), np.float32)
+    base[:5000], base[9000:9003] = base[0] + np.float32(3), base[0]
+    queries[[0, 130]] = base[0]
+    ctx = short_passes(base_rows=6000, queries=128)
+    base, queries = (torch.from_numpy(x).to(ctx.torch_device) for x in (base, queries))
+    before = ctx.exact_knn_counts
+    ids, dists = api.bruteforce_knn(ctx, base, queries, 10)
+    after = ctx.exact_knn_counts
+    assert (after[0] - before[0], after[1] - before[1]) == (200, 2)
+    want_ids, want = _tile_kernel(ctx, base, queries, 10)
+    assert torch.equal(ids, want_ids) and torch.equal(dists, want)
+
+
+def test_bad_rows_of_one_partition_leave_the_others_on_the_tensor_cores(gpu_ctx):
+    dim, degree = 36, 32
+    lens = np.array([900, 900, 900, 4000], np.uint32)     # alone, 900 rows take segment_knn_kernel
+    start = np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.uint32)
+    rows = np.random.default_rng(4).random((int(lens.sum()), dim), np.float32)
+    rows[900 + 130, 3] = np.nan
+    rows[1800 + 64, 0], rows[1800 + 100, 1] = np.inf, -np.inf      # both in one half tile
+    rows[2700 + 1000:2700 + 3500] = rows[0] + np.float32(2)        # halves 15 to 54 of the last partition
+    rows = torch.from_numpy(rows).to(gpu_ctx.torch_device)
+    before, stages = gpu_ctx.exact_knn_counts, gpu_ctx.tc_knn_fallbacks
+    got, _, _ = api.build_nnd(gpu_ctx, NNDescentParameter(degree), rows, start, lens, exact_max_rows=16384)
+    after = gpu_ctx.exact_knn_counts
+    assert (after[2] - before[2], after[3] - before[3]) == (int(lens.sum()), 64 + 64 + 40 * 64)
+    assert gpu_ctx.tc_knn_fallbacks == stages + 1
+    got = got.cpu().numpy()
+    for lo in (0, 900, 1800):
+        alone, _, _ = api.build_nnd(gpu_ctx, NNDescentParameter(degree), rows[lo:lo + 900].contiguous(), np.array([0], np.uint32),
+                                    np.array([900], np.uint32), exact_max_rows=16384)
+        real = torch.isfinite(rows[lo:lo + 900]).all(dim=1).cpu().numpy()   # (the others' rows are padding, by the row's own number)
+        assert real.sum() >= 898 and np.array_equal(got[lo:lo + 900][real], alone.cpu().numpy()[real])
+    part = rows[2700:].contiguous()
+    check = np.concatenate([np.arange(900, 1100), np.arange(3400, 3600)])
+    ids, _ = _tile_kernel(gpu_ctx, part, part[torch.from_numpy(check).to(part.device)].contiguous(), degree + 1)
+    for r, row in zip(check, ids.cpu().numpy()):
+        assert list(got[2700 + r]) == [i for i in row if i != r][:degree]
+
+
+def test_rows_that_overflow_one_tensor_core_path_are_not_given_to_the_other(gpu_ctx):
+    rows = np.random.default_rng(4).random((5000, 64), np.float32)
+    rows[1000:4500] = rows[0]
+    rows = torch.from_numpy(rows).to(gpu_ctx.torch_device)
+    before, stages = gpu_ctx.exact_knn_counts, gpu_ctx.tc_knn_fallbacks
+    got, _, _ = api.build_nnd(gpu_ctx, NNDescentParameter(32), rows, np.array([0], np.uint32), np.array([5000], np.uint32))
+    assert gpu_ctx.tc_knn_fallbacks == stages + 1 and gpu_ctx.exact_knn_counts == before
+    ids, _ = _tile_kernel(gpu_ctx, rows, rows[900:1100].contiguous(), 33)
+    for r, row in zip(range(900, 1100), ids.cpu().numpy()):
+        assert list(got[r].cpu().numpy()) == [i for i in row if i != r][:32]
