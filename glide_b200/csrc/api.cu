@@ -559,8 +559,8 @@ static int build_nnd_simt(glide_ctx *ctx, const float *d_reorder_data, uint32_t 
     bool need_nnd = false;
     for (uint32_t s = 0; s < S; s++) need_nnd = need_nnd || h_segment_length[s] > exact_max_rows;
     const size_t nnd_bytes = need_nnd ? nnd_workspace_bytes(rows, K, sample, S) : 0;
-    bool tc = tile_count != 0 && !skip_tc && segment_tc_eligible(d_reorder_data, rows, dim, h_segment_length, S, exact_max_rows, knn_degree);
-    const size_t tc_bytes = tc ? segment_tc_scratch_bytes(ctx->tc_passes, d_reorder_data, rows, dim, h_segment_length, S, exact_max_rows, knn_degree) : 0;
+    bool tc = tile_count != 0 && !skip_tc && segment_tc_eligible(d_reorder_data, dim, h_segment_length, S, exact_max_rows, knn_degree);
+    const size_t tc_bytes = tc ? segment_tc_scratch_bytes(ctx->tc_passes, d_reorder_data, rows, dim, h_segment_start, h_segment_length, S, exact_max_rows, knn_degree) : 0;
     size_t work_bytes = std::max(nnd_bytes, tc_bytes);   // one after the other
     const size_t tables = 2 * align256((size_t) S * 4) + align256((size_t) tile_count * 12) + 256;
     int rc = ensure_ws(ctx, work_bytes + tables);

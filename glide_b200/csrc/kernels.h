@@ -182,8 +182,8 @@ cudaError_t preload_truth_kernels();
 struct TcPasses {
     uint32_t base_rows = 1u << 21;      // base rows of a bruteforce call
     uint32_t queries = 8192;            // its queries
-    uint32_t padded_values = 1u << 28;  // values in the padded copy of rows that TMA cannot read (1 GB)
-    uint32_t tiles = 296;               // CTAs of 128 rows of a launch over partitions
+    uint32_t padded_values = 1u << 26;  // values in the padded copy of rows that TMA cannot read (256 MB)
+    uint32_t tiles = 148;               // CTAs of 128 rows of a launch over partitions (about 200 KB of shared memory each: one per SM)
 };
 // The same results from the tensor cores' candidates (truth_tc.cu). h_left[0] != 0: use launch_bruteforce; otherwise for
 // h_left[1] queries, whose numbers are the first words of the scratch.
@@ -204,8 +204,9 @@ void segment_knn_fill_tiles(const uint32_t *h_seg_start, const uint32_t *h_seg_l
 // row_base: index of data's row 0 within the whole reordered set (enters the padding hash of short partitions)
 // The same rows from the tensor cores' candidates (truth_tc.cu). *h_all: use launch_segment_knn; otherwise for the tiles
 // listed in h_tiles.
-bool segment_tc_eligible(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree);
-size_t segment_tc_scratch_bytes(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree);
+bool segment_tc_eligible(const float *data, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree);
+size_t segment_tc_scratch_bytes(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len, uint32_t S,
+                                uint32_t max_len, uint32_t out_degree);
 cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len,
                               uint32_t S, uint32_t max_len, uint32_t out_degree, uint32_t row_base, void *scratch, int32_t *out, bool *h_all,
                               std::vector<uint32_t> *h_tiles, cudaStream_t stream);

@@ -74,6 +74,7 @@ struct SegmentTile {
 
 struct TruthArgs {
     uint32_t n, Q, dim, kblocks, stages, cap;
+    uint32_t map_from;                       // the tensor maps' first row
     const SegmentTile *segments;             // segment form: one per CTA; per-query arrays are indexed by CTA * 128 + row
     uint32_t slices;                         // CTA (query tile, slice) takes tiles slice, slice + slices, ...
     // sample pass: column c stands for row c * stride; a thread keeps the minima of its columns over `span` of its tiles,
@@ -95,9 +96,9 @@ __device__ __forceinline__ void report_bad(const TruthBad &bad, uint32_t item) {
 __device__ __forceinline__ float tf32_rest(float x) { return x - __uint_as_float(__float_as_uint(x) & 0xffffe000u); }
 
 // A warp per row: |x|^2, |x - tf32(x)|^2 (two floats per row if `rest` is given), the maxima, and the row padded to `pitch`.
-// Segment form: a CTA per tile, maxima per partition.
+// Segment form: a CTA per tile, maxima per partition, the padded copy from row `padded_from` on.
 __global__ void truth_rows_kernel(const float *__restrict__ data, uint32_t rows, uint32_t dim, float *norms, float *rest, uint32_t pitch,
-                                  float *padded, TruthTops *tops, const SegmentTile *__restrict__ segments) {
+                                  float *padded, uint32_t padded_from, TruthTops *tops, const SegmentTile *__restrict__ segments) {
     __shared__ uint32_t top[2];
     if (threadIdx.x < 2) top[threadIdx.x] = 0;
     __syncthreads();
@@ -125,7 +126,7 @@ __global__ void truth_rows_kernel(const float *__restrict__ data, uint32_t rows,
         } else {
             for (uint32_t k = lane; k < pitch; k += 32) {
                 const float v = k < dim ? __ldg(row + k) : 0.0f, l = tf32_rest(v);
-                padded[r * pitch + k] = v;
+                padded[(r - padded_from) * pitch + k] = v;
                 s += v * v;
                 t += l * l;
             }
@@ -202,9 +203,9 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
     const SegmentTile part_of = seg ? a.segments[blockIdx.x] : SegmentTile{0, a.n, 0, a.stride, a.span, a.runs};
     const uint32_t qtiles = seg ? 1u : (a.Q + kTile - 1) / kTile;
     const uint32_t q0 = seg ? blockIdx.x * kTile : (blockIdx.x % qtiles) * kTile;      // index of the first query's results
-    const uint32_t q_row = seg ? part_of.seg_start + part_of.first : q0;                // its row in the query map
+    const uint32_t q_row = seg ? part_of.seg_start + part_of.first - a.map_from : q0;   // its row in the query map
     const uint32_t slice = seg ? 0u : blockIdx.x / qtiles, slices = seg ? 1u : a.slices;
-    const uint32_t b_row = part_of.seg_start, stride = a.sample ? part_of.stride : 1u;
+    const uint32_t b_row = part_of.seg_start, m_row = b_row - a.map_from, stride = a.sample ? part_of.stride : 1u;
     const uint32_t n = part_of.seg_len / stride, all = (n + kTile - 1) / kTile;             // columns, tiles of them
     // a query of the CTA, by thread: one that wants candidates?
     bool wanted = tid < kTile && (seg ? part_of.first + tid < part_of.seg_len : q0 + tid < a.Q);
@@ -242,8 +243,8 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
                     if (use > 0 && !mbar_wait(freed + s, (use - 1) & 1u, failed)) { ok = false; break; }
                     uint8_t *dst = ring + s * stage_bytes;
                     mbar_expect_tx(full + s, stage_bytes);
-                    if (a.sample) tma_load_3d(dst, &tm_s.of[stride - 1u], kb * kBlock, b_row % stride, b_row / stride + c0, full + s);
-                    else tma_load_2d(dst, &tm_b, kb * kBlock, b_row + c0, full + s);
+                    if (a.sample) tma_load_3d(dst, &tm_s.of[stride - 1u], kb * kBlock, m_row % stride, m_row / stride + c0, full + s);
+                    else tma_load_2d(dst, &tm_b, kb * kBlock, m_row + c0, full + s);
                     if (!resident) tma_load_2d(dst + kBlockBytes, &tm_q, kb * kBlock, q_row, full + s);
                     if (++s == stages) { s = 0; use++; }
                 }
@@ -675,7 +676,7 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
         const uint32_t nq = Q - qa < p.qb ? Q - qa : p.qb;
         const float *qrows = queries + (size_t) qa * dim;
         float *q_padded = p.pad ? at(p.q_rows) : nullptr;
-        truth_rows_kernel<<<(nq + 7) / 8, 256, 0, stream>>>(qrows, nq, dim, q_norm, q_rest, p.pitch, q_padded, nullptr, nullptr);
+        truth_rows_kernel<<<(nq + 7) / 8, 256, 0, stream>>>(qrows, nq, dim, q_norm, q_rest, p.pitch, q_padded, 0, nullptr, nullptr);
         bad.first = qa;
         CUtensorMap tm_q, tm_b;
         SampleMaps tm_s{};
@@ -687,7 +688,7 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
             const float *brows = base + (size_t) ba * dim;
             float *b_padded = p.pad ? at(p.rows) : nullptr;
             const uint32_t blocks = std::min((nr + 7) / 8, 8u * sms);
-            truth_rows_kernel<<<blocks, 256, 0, stream>>>(brows, nr, dim, norms, nullptr, p.pitch, b_padded, tops, nullptr);
+            truth_rows_kernel<<<blocks, 256, 0, stream>>>(brows, nr, dim, norms, nullptr, p.pitch, b_padded, 0, tops, nullptr);
             if (!row_map(&tm_b, p.pad ? b_padded : brows, nr, p.pitch)) return cudaSuccess;
             a.n = nr;
             if (ba == 0) {
@@ -718,13 +719,34 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
 // ---- every row's nearest rows of its own partition ----------------------------------------------
 namespace {
 
+// Rows that TMA cannot read are copied, padded, a run of whole partitions at a time.
+struct SegChunk {
+    uint32_t row, rows, tile, tiles;   // its rows; its tiles in the call's table
+};
+
+std::vector<SegChunk> seg_chunks(const TcPasses &passes, bool pad, uint32_t pitch, uint32_t rows, const uint32_t *h_start, const uint32_t *h_len, uint32_t S,
+                                 uint32_t max_len) {
+    std::vector<SegChunk> chunks;
+    uint32_t tile = 0;
+    for (uint32_t s = 0; s < S; s++) {
+        if (h_len[s] == 0 || h_len[s] > max_len) continue;
+        const uint32_t tiles = (h_len[s] + kTile - 1) / kTile, end = h_start[s] + h_len[s];
+        if (chunks.empty() || (pad && (uint64_t) (end - chunks.back().row) * pitch > passes.padded_values)) chunks.push_back({pad ? h_start[s] : 0u, 0, tile, 0});
+        chunks.back().rows = pad ? end - chunks.back().row : rows;
+        chunks.back().tiles += tiles;
+        tile += tiles;
+    }
+    return chunks;
+}
+
 struct SegPlan {
     bool pad;
     uint32_t pitch, groups;
+    std::vector<SegChunk> chunks;
     size_t bad, items, seen, tops, tiles, norms, rest, thr, count, cand, gmin, rows, total;
 };
 
-SegPlan seg_plan(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree) {
+SegPlan seg_plan(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree) {
     SegPlan p;
     p.pad = (dim & 3u) != 0 || (reinterpret_cast<uintptr_t>(data) & 15u) != 0;
     p.pitch = (dim + 3u) & ~3u;
@@ -751,21 +773,24 @@ SegPlan seg_plan(const TcPasses &passes, const float *data, uint32_t rows, uint3
     p.count = take(slots * 4);
     p.cand = take(slots * kSegCap * 4);
     p.gmin = take(slots * p.groups * 4);
-    p.rows = take(p.pad ? (size_t) rows * p.pitch * 4 : 0);
+    p.chunks = seg_chunks(passes, p.pad, p.pitch, rows, h_start, h_len, S, max_len);
+    uint32_t padded = 0;
+    for (const SegChunk &c : p.chunks) padded = std::max(padded, c.rows);
+    p.rows = take(p.pad ? (size_t) padded * p.pitch * 4 : 0);
     p.total = at;
     return p;
 }
 
 }  // namespace
 
-// The padded copy of rows that TMA cannot read is bounded, and so are a partition's minima.
-bool segment_tc_eligible(const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree) {
+// The padded copy of a partition that TMA cannot read is bounded, and so are its minima.
+bool segment_tc_eligible(const float *data, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree) {
     const bool pad = (dim & 3u) != 0 || (reinterpret_cast<uintptr_t>(data) & 15u) != 0;
-    if (dim < 16 || dim > 4096 || out_degree < 1 || out_degree > 64 || (pad && (uint64_t) rows * dim > (1ull << 30)) || encode_tiled_fn() == nullptr) return false;
+    if (dim < 16 || dim > 4096 || out_degree < 1 || out_degree > 64 || encode_tiled_fn() == nullptr) return false;
     uint64_t taken = 0, pairs = 0;
     for (uint32_t s = 0; s < S; s++) {
         if (h_len[s] > max_len) continue;
-        if (h_len[s] > kSegRows) return false;
+        if (h_len[s] > kSegRows || (pad && (uint64_t) h_len[s] * dim > (1ull << 30))) return false;
         taken += h_len[s];
         pairs += (uint64_t) h_len[s] * h_len[s];
     }
@@ -775,16 +800,16 @@ bool segment_tc_eligible(const float *data, uint32_t rows, uint32_t dim, const u
     return pairs * dim >= taken << 15;
 }
 
-size_t segment_tc_scratch_bytes(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len,
-                                uint32_t out_degree) {
-    return seg_plan(passes, data, rows, dim, h_len, S, max_len, out_degree).total;
+size_t segment_tc_scratch_bytes(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len, uint32_t S,
+                                uint32_t max_len, uint32_t out_degree) {
+    return seg_plan(passes, data, rows, dim, h_start, h_len, S, max_len, out_degree).total;
 }
 
 // Exact kNN rows of every partition of at most max_len rows: what segment_knn_kernel writes, bit for bit. What is left for that
 // kernel: *h_all everything, otherwise h_tiles, three words each (its tiles). Synchronises the stream.
 cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len,
                               uint32_t S, uint32_t max_len, uint32_t out_degree, uint32_t row_base, void *scratch, int32_t *out, bool *h_all, std::vector<uint32_t> *h_tiles, cudaStream_t stream) {
-    const SegPlan p = seg_plan(passes, data, rows, dim, h_len, S, max_len, out_degree);
+    const SegPlan p = seg_plan(passes, data, rows, dim, h_start, h_len, S, max_len, out_degree);
     std::vector<SegmentTile> tiles;
     uint32_t parts = 0;
     for (uint32_t s = 0; s < S; s++) {
@@ -805,20 +830,10 @@ cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_
     SegmentTile *d_tiles = reinterpret_cast<SegmentTile *>(w + p.tiles);
     uint32_t *count = reinterpret_cast<uint32_t *>(w + p.count), *cand = reinterpret_cast<uint32_t *>(w + p.cand);
     float *padded = p.pad ? at(p.rows) : nullptr;
-    CUtensorMap tm;
-    SampleMaps tm_s{};
-    if (!row_map(&tm, p.pad ? padded : data, rows, p.pitch)) return cudaSuccess;
-    uint32_t mapped = 0;   // a bit per stride
-    for (const SegmentTile &t : tiles) {
-        if (mapped & (1u << t.stride)) continue;
-        mapped |= 1u << t.stride;
-        if (!make_strided_row_map(&tm_s.of[t.stride - 1], p.pad ? padded : data, rows, p.pitch, t.stride, kTile)) return cudaSuccess;
-    }
     cudaError_t e = cudaMemsetAsync(left, 0, 8 + 2 * tiles.size() * 4 + parts * sizeof(TruthTops), stream);
     // the table is pageable host memory: the copy has read it when the call returns
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_tiles, tiles.data(), tiles.size() * sizeof(SegmentTile), cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) return e;
-    truth_rows_kernel<<<(uint32_t) tiles.size(), 256, 0, stream>>>(data, rows, dim, at(p.norms), at(p.rest), p.pitch, padded, tops, d_tiles);
     TruthArgs a{};
     a.dim = dim; a.cap = kSegCap; a.kblocks = (p.pitch + kBlock - 1) / kBlock; a.stages = ring_stages(a.kblocks);
     a.groups = p.groups;
@@ -826,17 +841,32 @@ cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_
     a.norms = at(p.norms); a.thr = at(p.thr); a.gmin = at(p.gmin); a.count = count; a.cand = cand; a.gave_up = bad.gave_up;
     const size_t smem = umma_smem(a.stages), rr_smem = (size_t) kSegCap * 8 + (size_t) p.pitch * 4;
     if ((e = cudaFuncSetAttribute(truth_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
-    for (size_t first = 0; first < tiles.size(); first += passes.tiles) {
-        const uint32_t n = (uint32_t) (tiles.size() - first < passes.tiles ? tiles.size() - first : passes.tiles);
-        a.segments = d_tiles + first;
-        a.sample = true;
-        truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm, tm_s);
-        truth_threshold_kernel<<<n * kTile, 128, (size_t) p.groups * 4, stream>>>(a.gmin, p.groups, out_degree + 1, nullptr, a.norms, at(p.rest), dim, a.segments,
-                                                                                  tops, 0, 0, kSegCap, bad, at(p.thr), count);
-        a.sample = false;
-        truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm, tm_s);
-        segment_rerank_kernel<<<n * kTile, 128, rr_smem, stream>>>(data, dim, a.segments, cand, count, out_degree, row_base, out, at(p.thr), bad);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    for (const SegChunk &c : p.chunks) {
+        truth_rows_kernel<<<c.tiles, 256, 0, stream>>>(data, rows, dim, at(p.norms), at(p.rest), p.pitch, padded, c.row, tops, d_tiles + c.tile);
+        const float *mapped_rows = p.pad ? padded : data;
+        CUtensorMap tm;
+        SampleMaps tm_s{};
+        if (!row_map(&tm, mapped_rows, c.rows, p.pitch)) return cudaSuccess;
+        uint32_t mapped = 0;   // a bit per stride
+        for (uint32_t i = c.tile; i < c.tile + c.tiles; i++) {
+            const uint32_t stride = tiles[i].stride;
+            if (mapped & (1u << stride)) continue;
+            mapped |= 1u << stride;
+            if (!make_strided_row_map(&tm_s.of[stride - 1], mapped_rows, c.rows, p.pitch, stride, kTile)) return cudaSuccess;
+        }
+        a.map_from = c.row;
+        for (uint32_t first = 0; first < c.tiles; first += passes.tiles) {
+            const uint32_t n = std::min(c.tiles - first, passes.tiles);
+            a.segments = d_tiles + c.tile + first;
+            a.sample = true;
+            truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm, tm_s);
+            truth_threshold_kernel<<<n * kTile, 128, (size_t) p.groups * 4, stream>>>(a.gmin, p.groups, out_degree + 1, nullptr, a.norms, at(p.rest), dim,
+                                                                                      a.segments, tops, 0, 0, kSegCap, bad, at(p.thr), count);
+            a.sample = false;
+            truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm, tm_s);
+            segment_rerank_kernel<<<n * kTile, 128, rr_smem, stream>>>(data, dim, a.segments, cand, count, out_degree, row_base, out, at(p.thr), bad);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        }
     }
     uint32_t h_left[2] = {1, 0};
     if ((e = cudaMemcpyAsync(h_left, left, 8, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;

@@ -270,3 +270,27 @@ def test_rows_that_overflow_one_tensor_core_path_are_not_given_to_the_other(gpu_
     ids, _ = _tile_kernel(gpu_ctx, rows, rows[900:1100].contiguous(), 33)
     for r, row in zip(range(900, 1100), ids.cpu().numpy()):
         assert list(got[r].cpu().numpy()) == [i for i in row if i != r][:32]
+
+
+@pytest.mark.parametrize("lens", [[1500, 1600, 1, 1700, 0, 1800, 900], [1500, 4200, 1600, 1700]])
+def test_padded_partitions_are_copied_a_run_at_a_time(lens):
+    """Rows of 35 values need a padded copy: the context's scratch holds that of a run of partitions, not of all rows, and the
+    graph is the one that a single run gives. A partition beyond the exact limit lies between them once."""
+    lens = np.array(lens, np.uint32)
+    start = np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.uint32)
+    n, small = int(lens.sum()), lens <= 2000
+    ctx = api.Context(0)
+    rows = torch.from_numpy(np.random.default_rng(4).random((n, 35), np.float32)).to(ctx.torch_device)
+    graphs, held = [], []
+    for values in (36 * 2000, 0):
+        ctx.limit_exact_knn(padded_values=values)
+        got, _, _ = api.build_nnd(ctx, NNDescentParameter(16), rows, start, lens, exact_max_rows=2000, seed=3)
+        graphs.append(got.cpu().numpy())
+        held.append(int(ctx.lib.glide_ctx_workspace_bytes(ctx.handle)))
+    counts = ctx.exact_knn_counts
+    ctx.close()
+    assert counts[2] == 2 * int(lens[small].sum()) and counts[3] == 0
+    for lo, l in zip(start[small], lens[small]):
+        assert np.array_equal(graphs[0][lo:lo + l], graphs[1][lo:lo + l])
+    if small.all():       # (otherwise descent's scratch is the larger)
+        assert held[1] - held[0] >= 4 * 36 * (n - 2000)
