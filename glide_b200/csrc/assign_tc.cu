@@ -334,9 +334,9 @@ __global__ void __launch_bounds__(kTmaThreads) assign_umma_tma_kernel(const Assi
     float *rowmin = cn_s + 4 * kUmmaRows;                                 // 2 halves x 128 rows x 2
     uint32_t *cand = reinterpret_cast<uint32_t *>(rowmin + 4 * kUmmaRows);  // 128 x kCand
     uint32_t *cnt = cand + kUmmaRows * kCand;                 // 128 counters; later bit 31: far second
-    uint64_t *bars = reinterpret_cast<uint64_t *>(cnt + kUmmaRows);       // a_full, b_full[2], mma_done[2], tmem_free[2]
-    uint64_t *a_full = bars, *b_full = bars + 1, *mma_done = bars + 3, *tmem_free = bars + 5;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 7);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(cnt + kUmmaRows);       // a_full, b_full[2], mma_done[2], tmem_free[2], drained
+    uint64_t *a_full = bars, *b_full = bars + 1, *mma_done = bars + 3, *tmem_free = bars + 5, *drained = bars + 7;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 8);
     volatile uint32_t *failed = tmem_slot + 1;
     const float *norms = a.tc_norms;
 
@@ -346,6 +346,7 @@ __global__ void __launch_bounds__(kTmaThreads) assign_umma_tma_kernel(const Assi
 
     if (tid == 0) {
         mbar_init(a_full, 1);
+        mbar_init(drained, 1);
         for (int s = 0; s < 2; s++) { mbar_init(b_full + s, 1); mbar_init(mma_done + s, 1); mbar_init(tmem_free + s, kEpilogueWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         *failed = 0;
@@ -361,12 +362,14 @@ __global__ void __launch_bounds__(kTmaThreads) assign_umma_tma_kernel(const Assi
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
 
+    uint32_t copies = 0;   // centroid tiles asked for, by the producer
     if (warp == kEpilogueWarps) {
         // ================= producer: TMA copies and MMA issue, one thread =================
         if (lane == 0) {
             // a centroid tile travels with the 128 norms of its rows (a plain bulk copy; the norms
             // array is padded to a whole tile)
             auto load_tile = [&](uint8_t *dst, const CUtensorMap *tm, uint32_t row0, uint64_t *bar, float *norm_dst) {
+                if (norm_dst) copies++;
                 mbar_expect_tx(bar, tile_bytes + (norm_dst ? kUmmaRows * 4u : 0u));
                 for (uint32_t kb = 0; kb < kblocks; kb++) tma_load_2d(dst + kb * sub_bytes, tm, kb * 32u, row0, bar);
                 if (norm_dst)
@@ -475,6 +478,14 @@ __global__ void __launch_bounds__(kTmaThreads) assign_umma_tma_kernel(const Assi
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (*failed) {   // otherwise the epilogue has seen the last MMA, and that all copies
+        if (warp == kEpilogueWarps && lane == 0) {
+            mbar_drain(a_full, 0);
+            drain_copies(b_full, 2, copies);
+            drain_mmas(drained);
+        }
+        __syncthreads();
+    }
     if (warp == kEpilogueWarps) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
         return;
@@ -488,7 +499,7 @@ cudaError_t launch_umma_tma(const AssignArgs &a, cudaStream_t stream) {
     if ((reinterpret_cast<uintptr_t>(a.data) & 15u) || (reinterpret_cast<uintptr_t>(a.centroids) & 15u)) return cudaErrorNotSupported;
     CUtensorMap tm_points, tm_centroids;
     if (!make_row_map(&tm_points, a.data, a.n, a.dim, kUmmaRows) || !make_row_map(&tm_centroids, a.centroids, a.C, a.dim, kUmmaRows)) return cudaErrorNotSupported;
-    const size_t smem_bytes = 1024 + (size_t) 3 * kUmmaRows * a.dim * 4 + 8 * kUmmaRows * 4 + kUmmaRows * kCand * 4 + kUmmaRows * 4 + 7 * 8 + 16;
+    const size_t smem_bytes = 1024 + (size_t) 3 * kUmmaRows * a.dim * 4 + 8 * kUmmaRows * 4 + kUmmaRows * kCand * 4 + kUmmaRows * 4 + 8 * 8 + 16;
     cudaError_t e = cudaFuncSetAttribute(assign_umma_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem_bytes);
     if (e != cudaSuccess) return e;
     assign_umma_tma_kernel<<<(a.n + kUmmaRows - 1) / kUmmaRows, kTmaThreads, smem_bytes, stream>>>(a, tm_points, tm_centroids);

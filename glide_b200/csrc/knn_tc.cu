@@ -144,9 +144,10 @@ __global__ void __launch_bounds__(kThreads) knn_umma_kernel(const KnnTcArgs a, c
     uint8_t *Bs = base;                                       // kStages tiles of the partition; the CTA's own rows live in tensor memory
     float *cn_w = reinterpret_cast<float *>(Bs + kStages * tile_bytes); // a warp's column norms of the current tile
     float *thr_s = cn_w + kEpiWarps * kCols;                            // 128 row thresholds
-    uint64_t *bars = reinterpret_cast<uint64_t *>(thr_s + kRows);       // a_full, b_full[3], stage_free[3], mma_done[2], tmem_free[2]
+    uint64_t *bars = reinterpret_cast<uint64_t *>(thr_s + kRows);       // a_full, b_full[3], stage_free[3], mma_done[2], tmem_free[2], drained
     uint64_t *a_full = bars, *b_full = bars + 1, *stage_free = b_full + kStages, *mma_done = stage_free + kStages, *tmem_free = mma_done + 2;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_free + 2);
+    uint64_t *drained = tmem_free + 2;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drained + 1);
     volatile uint32_t *failed = tmem_slot + 1;
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -156,6 +157,7 @@ __global__ void __launch_bounds__(kThreads) knn_umma_kernel(const KnnTcArgs a, c
 
     if (tid == 0) {
         mbar_init(a_full, 4 * kblocks);   // the warps that write the CTA's rows into tensor memory
+        mbar_init(drained, 1);
         for (uint32_t s = 0; s < kStages; s++) { mbar_init(b_full + s, 1); mbar_init(stage_free + s, 1); }
         for (int c = 0; c < 2; c++) { mbar_init(mma_done + c, 1); mbar_init(tmem_free + c, kEpiWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -171,12 +173,14 @@ __global__ void __launch_bounds__(kThreads) knn_umma_kernel(const KnnTcArgs a, c
     fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
+    uint32_t copies = 0;   // tiles asked for, by the thread that copies
     if (warp == kEpiWarps + 1) {
         // ================= copy warp: operand tiles by TMA, one thread =================
         // Stage s takes tile t + 2 as soon as the MMAs of tile t have read it; the MMA thread does not
         // wait for that, so the MMAs of tile t + 1 are already queued behind those of tile t.
         if (lane == 0) {
             auto load_tile = [&](uint8_t *dst, uint32_t row0, uint64_t *bar) {
+                copies++;
                 mbar_expect_tx(bar, tile_bytes);
                 for (uint32_t kb = 0; kb < kblocks; kb++) tma_load_2d(dst + kb * sub_bytes, &tm_rows, kb * 32u, row0, bar);
             };
@@ -366,6 +370,11 @@ __global__ void __launch_bounds__(kThreads) knn_umma_kernel(const KnnTcArgs a, c
     }
     fence_before();
     __syncthreads();
+    if (*failed) {   // otherwise the epilogue has seen the last MMA, and that all copies
+        if (warp == kEpiWarps + 1 && lane == 0) drain_copies(b_full, kStages, copies);
+        if (warp == kEpiWarps && lane == 0) drain_mmas(drained);
+        __syncthreads();
+    }
     if (warp == kEpiWarps) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
 }
 
@@ -456,7 +465,7 @@ cudaError_t run(const float *data, uint64_t rows_total, uint32_t dim, const std:
     cudaError_t e = cudaMemsetAsync(fail_flag, 0, 4, stream);
     if (e != cudaSuccess) return e;
     row_norms_kernel<<<(unsigned) ((rows_total * 32 + 255) / 256), 256, 0, stream>>>(data, rows_total, dim, norms);
-    const size_t smem_main = 1024 + (size_t) 3 * kRows * dim * 4 + (kEpiWarps * kCols + kRows) * 4 + (1 + 2 * kStages + 4) * 8 + 16;
+    const size_t smem_main = 1024 + (size_t) 3 * kRows * dim * 4 + (kEpiWarps * kCols + kRows) * 4 + (1 + 2 * kStages + 5) * 8 + 16;
     if ((e = cudaFuncSetAttribute(knn_umma_kernel<NL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem_main)) != cudaSuccess) return e;
     const uint32_t rr_warps = 8;
     const size_t smem_rr = (size_t) rr_warps * (dim_pad4(dim) + 2 * Sizes<NL>::keep) * 4;

@@ -75,6 +75,7 @@ struct SegmentTile {
 struct TruthArgs {
     uint32_t n, Q, dim, kblocks, stages, cap;
     uint32_t map_from;                       // the tensor maps' first row
+    uint32_t polls;                          // of a wait
     const SegmentTile *segments;             // segment form: one per CTA; per-query arrays are indexed by CTA * 128 + row
     uint32_t slices;                         // CTA (query tile, slice) takes tiles slice, slice + slices, ...
     // sample pass: column c stands for row c * stride; a thread keeps the minima of its columns over `span` of its tiles,
@@ -194,8 +195,8 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
     uint8_t *As = base, *ring = base + (resident ? kblocks * kBlockBytes : 0u);
     float *cn_w = reinterpret_cast<float *>(ring + stages * stage_bytes);     // a warp's column norms
     uint64_t *bars = reinterpret_cast<uint64_t *>(cn_w + kEpi * 32);
-    uint64_t *a_full = bars, *full = bars + 1, *freed = full + stages, *mma_done = freed + stages, *tmem_free = mma_done + 2;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_free + 2);
+    uint64_t *a_full = bars, *full = bars + 1, *freed = full + stages, *mma_done = freed + stages, *tmem_free = mma_done + 2, *drained = tmem_free + 2;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drained + 1);
     volatile uint32_t *failed = tmem_slot + 1;
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -213,6 +214,7 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
 
     if (tid == 0) {
         mbar_init(a_full, 1);
+        mbar_init(drained, 1);
         for (uint32_t s = 0; s < stages; s++) { mbar_init(full + s, 1); mbar_init(freed + s, 1); }
         for (int c = 0; c < 2; c++) { mbar_init(mma_done + c, 1); mbar_init(tmem_free + c, kEpi); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -228,6 +230,7 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tiles = any_wanted && slice < all ? (all - slice + slices - 1) / slices : 0u;   // of this CTA
 
+    uint32_t copies = 0;   // ring stages asked for, by the thread that copies
     if (warp == kEpi + 1) {
         // ================= copies: one thread =================
         if (lane == 0 && tiles > 0) {
@@ -240,12 +243,13 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
             for (uint32_t t = 0; t < tiles && ok; t++) {
                 const uint32_t c0 = (slice + t * slices) * kTile;
                 for (uint32_t kb = 0; kb < kblocks; kb++) {
-                    if (use > 0 && !mbar_wait(freed + s, (use - 1) & 1u, failed)) { ok = false; break; }
+                    if (use > 0 && !mbar_wait(freed + s, (use - 1) & 1u, failed, a.polls)) { ok = false; break; }
                     uint8_t *dst = ring + s * stage_bytes;
                     mbar_expect_tx(full + s, stage_bytes);
                     if (a.sample) tma_load_3d(dst, &tm_s.of[stride - 1u], kb * kBlock, m_row % stride, m_row / stride + c0, full + s);
                     else tma_load_2d(dst, &tm_b, kb * kBlock, m_row + c0, full + s);
                     if (!resident) tma_load_2d(dst + kBlockBytes, &tm_q, kb * kBlock, q_row, full + s);
+                    copies++;
                     if (++s == stages) { s = 0; use++; }
                 }
             }
@@ -255,13 +259,13 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
         if (lane == 0 && tiles > 0) {
             const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((kTile >> 3) << 17) | ((kTile >> 4) << 24);
             const uint32_t a_addr = smem_u32(As), r_addr = smem_u32(ring);
-            bool ok = !resident || mbar_wait(a_full, 0, failed);
+            bool ok = !resident || mbar_wait(a_full, 0, failed, a.polls);
             uint32_t s = 0, use = 0;
             for (uint32_t t = 0; t < tiles && ok; t++) {
                 const uint32_t acc = t & 1u;
-                if (t >= 2) ok = mbar_wait(tmem_free + acc, ((t >> 1) - 1) & 1u, failed);
+                if (t >= 2) ok = mbar_wait(tmem_free + acc, ((t >> 1) - 1) & 1u, failed, a.polls);
                 for (uint32_t kb = 0; kb < kblocks && ok; kb++) {
-                    ok = mbar_wait(full + s, use & 1u, failed);
+                    ok = mbar_wait(full + s, use & 1u, failed, a.polls);
                     if (!ok) break;
                     fence_after();
                     const uint32_t b = r_addr + s * stage_bytes, q = resident ? a_addr + kb * kBlockBytes : b + kBlockBytes;
@@ -297,7 +301,7 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
             ahead = norm_of(t + 1);
             __syncwarp();
             const uint32_t acc = t & 1u, c0 = (slice + t * slices) * kTile + part * 32u;
-            bool ok = !*failed && mbar_wait(mma_done + acc, (t >> 1) & 1u, failed);
+            bool ok = !*failed && mbar_wait(mma_done + acc, (t >> 1) & 1u, failed, a.polls);
             ok = __all_sync(kFullMask, ok);
             if (!ok) break;
             fence_after();
@@ -349,6 +353,14 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
     }
     fence_before();
     __syncthreads();
+    if (*failed) {   // otherwise the epilogue has seen the last MMA, and that all copies
+        if (warp == kEpi + 1 && lane == 0 && tiles > 0) {
+            if (resident) mbar_drain(a_full, 0);
+            drain_copies(full, stages, copies);
+        }
+        if (warp == kEpi && lane == 0) drain_mmas(drained);
+        __syncthreads();
+    }
     if (warp == kEpi) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(2 * kTile) : "memory");
 }
 
@@ -616,7 +628,7 @@ TruthPlan truth_plan(const TcPasses &passes, const float *base, const float *que
 }
 
 uint32_t ring_stages(uint32_t kblocks) { return kblocks <= kResidentBlocks ? 12u - kblocks : 6u; }    // 192 KB of operand blocks
-size_t umma_smem(uint32_t stages) { return 1024 + 12u * (size_t) kBlockBytes + kEpi * 32 * 4 + (1 + 2 * stages + 4) * 8 + 16; }
+size_t umma_smem(uint32_t stages) { return 1024 + 12u * (size_t) kBlockBytes + kEpi * 32 * 4 + (1 + 2 * stages + 5) * 8 + 16; }
 
 // row-major rows of `pitch` floats as TMA boxes of 32 values x 128 rows (make_row_map takes the row length as the pitch)
 bool row_map(CUtensorMap *tm, const float *ptr, uint32_t rows, uint32_t pitch) { return make_row_map(tm, ptr, rows, pitch, kTile); }
@@ -664,7 +676,7 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
     if (e != cudaSuccess) return e;
 
     TruthArgs a{};
-    a.dim = dim; a.cap = kCap; a.kblocks = (p.pitch + kBlock - 1) / kBlock;
+    a.dim = dim; a.cap = kCap; a.polls = passes.polls; a.kblocks = (p.pitch + kBlock - 1) / kBlock;
     a.stages = ring_stages(a.kblocks);
     a.norms = norms; a.thr = thr; a.gmin = gmin; a.count = count; a.cand = cand; a.gave_up = bad.gave_up;
     const size_t smem = umma_smem(a.stages);
@@ -835,7 +847,7 @@ cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_tiles, tiles.data(), tiles.size() * sizeof(SegmentTile), cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) return e;
     TruthArgs a{};
-    a.dim = dim; a.cap = kSegCap; a.kblocks = (p.pitch + kBlock - 1) / kBlock; a.stages = ring_stages(a.kblocks);
+    a.dim = dim; a.cap = kSegCap; a.polls = passes.polls; a.kblocks = (p.pitch + kBlock - 1) / kBlock; a.stages = ring_stages(a.kblocks);
     a.groups = p.groups;
     a.fold = 1;
     a.norms = at(p.norms); a.thr = at(p.thr); a.gmin = at(p.gmin); a.count = count; a.cand = cand; a.gave_up = bad.gave_up;

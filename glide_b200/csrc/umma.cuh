@@ -76,24 +76,35 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
 }
 // Bounded wait: at most kSpinLimit polls; gives up early when another thread of the CTA has already
 // failed. A wait that runs out raises *failed, after which nobody waits any more.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *failed) {
-    const uint32_t addr = smem_u32(bar);
-    for (uint32_t spin = 0; spin < kSpinLimit; spin++) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t"
-            ".reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t"
-            "}\n"
-            : "=r"(done)
-            : "r"(addr), "r"(parity)
-            : "memory");
-        if (done) return true;
+__device__ __forceinline__ bool mbar_done(uint64_t *bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(done)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *failed, uint32_t polls = kSpinLimit) {
+    for (uint32_t spin = 0; spin < polls; spin++) {
+        if (mbar_done(bar, parity)) return true;
         if ((spin & 1023u) == 1023u && *failed) return false;
     }
     *failed = 1;
     return false;
+}
+// A CTA that has given up must not return while its copies still write shared memory or its MMAs read it and write
+// tensor memory. These waits, bounded too, go on whatever *failed says; the threads that issued the work call them.
+__device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity) {
+    for (uint32_t spin = 0; spin < kSpinLimit && !mbar_done(bar, parity); spin++) {}
+}
+// `issued` copies in turn into `stages` stages, each of which completes a phase of its stage's barrier
+__device__ __forceinline__ void drain_copies(uint64_t *full, uint32_t stages, uint32_t issued) {
+    for (uint32_t s = 0; s < stages && s < issued; s++) mbar_drain(full + s, ((issued - 1u - s) / stages) & 1u);
 }
 // One box of a 2-D tensor map into shared memory; x (the innermost coordinate) times the element size
 // must be a multiple of 16 bytes. No multicast.
@@ -120,6 +131,11 @@ __device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t threads
 }
 __device__ __forceinline__ void commit_to(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// everything that the calling thread has issued so far; `bar` (one arrival) serves this alone
+__device__ __forceinline__ void drain_mmas(uint64_t *bar) {
+    commit_to(bar);
+    mbar_drain(bar, 0);
 }
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }

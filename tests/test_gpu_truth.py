@@ -294,3 +294,20 @@ def test_padded_partitions_are_copied_a_run_at_a_time(lens):
         assert np.array_equal(graphs[0][lo:lo + l], graphs[1][lo:lo + l])
     if small.all():       # (otherwise descent's scratch is the larger)
         assert held[1] - held[0] >= 4 * 36 * (n - 2000)
+
+
+@pytest.mark.parametrize("dim", [64, 300])      # query blocks that stay in shared memory, blocks that ride along
+def test_waits_that_run_out_leave_everything_to_the_tile_kernels(short_passes, dim):
+    """One poll per wait: a CTA gives up, drains what it has in flight and returns; the results are the tile kernel's, and the
+    context goes on."""
+    rng = np.random.default_rng(dim)
+    ctx = short_passes(polls=1)
+    base, queries = (torch.from_numpy(rng.random((m, dim), np.float32)).to(ctx.torch_device) for m in (3000, 150))
+    before = ctx.exact_knn_counts
+    ids, dists = api.bruteforce_knn(ctx, base, queries, 10)
+    after = ctx.exact_knn_counts
+    assert (after[0] - before[0], after[1] - before[1]) == (150, 150)
+    ctx.limit_exact_knn()
+    want_ids, want = api.bruteforce_knn(ctx, base, queries, 10)
+    assert ctx.exact_knn_counts[1] == after[1]
+    assert torch.equal(ids, want_ids) and torch.equal(dists, want)
