@@ -561,41 +561,68 @@ static int build_nnd_simt(glide_ctx *ctx, const float *d_reorder_data, uint32_t 
     for (uint32_t s = 0; s < S; s++) need_nnd = need_nnd || h_segment_length[s] > exact_max_rows;
     const size_t nnd_bytes = need_nnd ? nnd_workspace_bytes(rows, K, sample, S) : 0;
     bool tc = tile_count != 0 && !skip_tc && segment_tc_eligible(d_reorder_data, dim, h_segment_length, S, exact_max_rows, knn_degree);
-    const size_t tc_bytes = tc ? segment_tc_scratch_bytes(ctx->tc_passes, d_reorder_data, rows, dim, h_segment_start, h_segment_length, S, exact_max_rows, knn_degree) : 0;
-    size_t work_bytes = std::max(nnd_bytes, tc_bytes);   // one after the other
+    auto tc_bytes = [&](bool centred) {
+        return segment_tc_scratch_bytes(ctx->tc_passes, d_reorder_data, rows, dim, h_segment_start, h_segment_length, S, exact_max_rows, knn_degree, centred);
+    };
     const size_t tables = 2 * align256((size_t) S * 4) + align256((size_t) tile_count * 12) + 256;
-    int rc = ensure_ws(ctx, work_bytes + tables);
+    uint32_t *d_start = nullptr, *d_len = nullptr, *d_tiles = nullptr;
+    void *work = nullptr;
+    // Room for the tables and `bytes` of work, all laid out anew.
+    auto lay_out = [&](size_t bytes) -> int {
+        const int rc = ensure_ws(ctx, bytes + tables);
+        if (rc) return rc;
+        Bump b(ctx->ws);
+        d_start = b.take<uint32_t>(S);
+        d_len = b.take<uint32_t>(S);
+        d_tiles = b.take<uint32_t>((size_t) tile_count * 3 + 1);
+        work = b.take<char>(bytes);
+        return GLIDE_OK;
+    };
+    int rc = lay_out(std::max(nnd_bytes, tc ? tc_bytes(false) : 0));   // one after the other
     if (tc && rc == GLIDE_ERR_NO_MEMORY) {   // the tile kernel needs none
         cudaGetLastError();
         tc = false;
-        work_bytes = nnd_bytes;
-        rc = ensure_ws(ctx, work_bytes + tables);
+        rc = lay_out(nnd_bytes);
     }
     if (rc) return rc;
-    Bump b(ctx->ws);
-    uint32_t *d_start = b.take<uint32_t>(S), *d_len = b.take<uint32_t>(S);
-    uint32_t *d_tiles = b.take<uint32_t>((size_t) tile_count * 3 + 1);
-    void *work = b.take<char>(work_bytes);
     std::vector<uint32_t> h_tiles((size_t) tile_count * 3);
     uint32_t by_tiles = tile_count;
     if (tile_count) segment_knn_fill_tiles(h_segment_start, h_segment_length, S, exact_max_rows, h_tiles.data());
     // empty segments (C == 1 leaves the boundary segment empty, partition_kernel.cuh:58) need no launch
     Timed timer(ctx);
-    GL_CUDA(ctx, cudaMemcpyAsync(d_start, h_segment_start, (size_t) S * 4, cudaMemcpyHostToDevice, ctx->stream));
-    GL_CUDA(ctx, cudaMemcpyAsync(d_len, h_segment_length, (size_t) S * 4, cudaMemcpyHostToDevice, ctx->stream));
     if (iterations_run) *iterations_run = 0;
     if (tc) {
-        bool all = true;
-        std::vector<uint32_t> left;
-        GL_CUDA(ctx, launch_segment_tc(ctx->tc_passes, d_reorder_data, rows, dim, h_segment_start, h_segment_length, S, exact_max_rows, knn_degree, row_base, work, d_knn,
-                                       &all, &left, ctx->stream));
-        for (uint32_t s = 0; s < S; s++)
-            if (h_segment_length[s] <= exact_max_rows) ctx->exact_knn[2] += h_segment_length[s];
-        if (!all) h_tiles.swap(left);   // some of the tiles, or none
-        by_tiles = all ? tile_count : (uint32_t) (h_tiles.size() / 3);
+        TcLeft left;
+        std::vector<uint32_t> left_tiles;
+        auto attempt = [&](bool centred) {
+            return launch_segment_tc(ctx->tc_passes, d_reorder_data, rows, dim, h_segment_start, h_segment_length, S, exact_max_rows, knn_degree, row_base,
+                                     centred, work, d_knn, &left, &left_tiles, ctx->stream);
+        };
+        uint64_t given = 0, largest = 0;
+        for (uint32_t s = 0; s < S; s++) {
+            if (h_segment_length[s] > exact_max_rows) continue;
+            given += h_segment_length[s];
+            largest = std::max<uint64_t>(largest, h_segment_length[s]);
+        }
+        GL_CUDA(ctx, attempt(false));
+        if (!left.everything && left.hopeful > given / 2 && largest * dim <= (1u << 28)) {   // a copy of a partition of 1 GB at most
+            rc = lay_out(std::max(nnd_bytes, tc_bytes(true)));
+            if (rc == GLIDE_OK) {
+                GL_CUDA(ctx, attempt(true));
+            } else if (rc == GLIDE_ERR_NO_MEMORY) {   // the fp32 kernel redoes what the first attempt left
+                cudaGetLastError();
+                rc = lay_out(nnd_bytes);
+            }
+            if (rc) return rc;
+        }
+        ctx->exact_knn[2] += given;
+        if (!left.everything) h_tiles.swap(left_tiles);   // some of the tiles, or none
+        by_tiles = left.everything ? tile_count : (uint32_t) (h_tiles.size() / 3);
         for (uint32_t t = 0; t < by_tiles; t++) ctx->exact_knn[3] += std::min(64u, h_tiles[3 * t + 1] - h_tiles[3 * t + 2]);
         if (by_tiles) ctx->tc_knn_fallbacks++;
     }
+    GL_CUDA(ctx, cudaMemcpyAsync(d_start, h_segment_start, (size_t) S * 4, cudaMemcpyHostToDevice, ctx->stream));
+    GL_CUDA(ctx, cudaMemcpyAsync(d_len, h_segment_length, (size_t) S * 4, cudaMemcpyHostToDevice, ctx->stream));
     if (by_tiles) {
         GL_CUDA(ctx, cudaMemcpyAsync(d_tiles, h_tiles.data(), (size_t) by_tiles * 12, cudaMemcpyHostToDevice, ctx->stream));
         GL_CUDA(ctx, launch_segment_knn(d_reorder_data, dim, d_tiles, by_tiles, knn_degree, row_base, d_knn, ctx->stream));
@@ -621,7 +648,7 @@ int glide_bruteforce_knn(glide_ctx *ctx, const float *d_base, uint32_t n, const 
     const uint32_t splits = bruteforce_default_splits(n, q);
     bool tc = q > 0 && truth_tc_eligible(n, q, dim, k);
     const size_t need = bruteforce_scratch_bytes(q, k, splits) + 256, listed = align256((size_t) q * 4);
-    int rc = ensure_ws(ctx, tc ? std::max(listed + need, truth_tc_scratch_bytes(ctx->tc_passes, d_base, d_queries, n, q, dim, k)) : need);
+    int rc = ensure_ws(ctx, tc ? std::max(listed + need, truth_tc_scratch_bytes(ctx->tc_passes, d_base, d_queries, n, q, dim, k, false)) : need);
     if (tc && rc == GLIDE_ERR_NO_MEMORY) {   // the tile kernel asks for less
         cudaGetLastError();
         tc = false;
@@ -630,14 +657,25 @@ int glide_bruteforce_knn(glide_ctx *ctx, const float *d_base, uint32_t n, const 
     if (rc) return rc;
     Timed timer(ctx);
     if (tc) {
-        uint32_t left[2] = {1, 0};
-        GL_CUDA(ctx, launch_truth_tc(ctx->tc_passes, d_base, n, d_queries, q, dim, k, metric, ctx->ws, d_out_ids, d_out_dists, left, ctx->stream));
+        TcLeft left;
+        GL_CUDA(ctx, launch_truth_tc(ctx->tc_passes, d_base, n, d_queries, q, dim, k, metric, false, ctx->ws, d_out_ids, d_out_dists, &left, ctx->stream));
+        if (!left.everything && left.items > q / 2 && left.hopeful > left.items / 2) {
+            rc = ensure_ws(ctx, std::max(listed + need, truth_tc_scratch_bytes(ctx->tc_passes, d_base, d_queries, n, q, dim, k, true)));
+            if (rc == GLIDE_OK) {
+                GL_CUDA(ctx, launch_truth_tc(ctx->tc_passes, d_base, n, d_queries, q, dim, k, metric, true, ctx->ws, d_out_ids, d_out_dists, &left, ctx->stream));
+            } else if (rc == GLIDE_ERR_NO_MEMORY) {   // the list went with the old scratch
+                cudaGetLastError();
+                left.everything = 1;
+                rc = ensure_ws(ctx, need);
+            }
+            if (rc) return rc;
+        }
         ctx->exact_knn[0] += q;
-        ctx->exact_knn[1] += left[0] ? q : left[1];
-        if (!left[0]) {
-            if (left[1] == 0) return timer.finish();
+        ctx->exact_knn[1] += left.everything ? q : left.items;
+        if (!left.everything) {
+            if (left.items == 0) return timer.finish();
             // the queries it lists, in the scratch behind the list: as many slices of the base as fit there
-            const uint32_t few = left[1], fit = (uint32_t) ((uint64_t) q * splits / few);
+            const uint32_t few = left.items, fit = (uint32_t) ((uint64_t) q * splits / few);
             GL_CUDA(ctx, launch_bruteforce(d_base, n, d_queries, few, dim, k, metric, std::min(bruteforce_default_splits(n, few), fit),
                                            static_cast<char *>(ctx->ws) + listed, d_out_ids, d_out_dists, ctx->stream, static_cast<uint32_t *>(ctx->ws)));
             return timer.finish();

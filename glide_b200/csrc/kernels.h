@@ -186,12 +186,19 @@ struct TcPasses {
     uint32_t polls = 1u << 22;          // of a wait inside these kernels before it gives up
     uint32_t tiles = 148;               // CTAs of 128 rows of a launch over partitions (about 200 KB of shared memory each: one per SM)
 };
-// The same results from the tensor cores' candidates (truth_tc.cu). h_left[0] != 0: use launch_bruteforce; otherwise for
-// h_left[1] queries, whose numbers are the first words of the scratch.
+// The same results from the tensor cores' candidates (truth_tc.cu); items of TcLeft: queries, whose numbers are the first words
+// of the scratch.
+//
+// What exact kNN from tensor-core candidates leaves to the fp32 kernels. `hopeful`: of its queries, those that had too many
+// candidates for the norms' sake only (rows far from the origin, close to one another): where most are, a second attempt, `centred`
+// on rows in the middle, serves them. It costs a copy of the rows and is not worth starting with.
+struct TcLeft {
+    uint32_t everything, items, hopeful;
+};
 bool truth_tc_eligible(uint32_t n, uint32_t Q, uint32_t dim, uint32_t k);
-size_t truth_tc_scratch_bytes(const TcPasses &passes, const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k);
+size_t truth_tc_scratch_bytes(const TcPasses &passes, const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k, bool centred);
 cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t n, const float *queries, uint32_t Q, uint32_t dim, uint32_t k, int metric,
-                            void *scratch, uint32_t *out_ids, float *out_dists, uint32_t (&h_left)[2], cudaStream_t stream);
+                            bool centred, void *scratch, uint32_t *out_ids, float *out_dists, TcLeft *h_left, cudaStream_t stream);
 // `list`: the queries to answer are list[0..Q), their results go to their own rows; nullptr: queries 0..Q-1
 cudaError_t launch_bruteforce(const float *base, uint32_t n, const float *queries, uint32_t Q, uint32_t dim,
                               uint32_t k, int metric, uint32_t splits, void *scratch, uint32_t *out_ids,
@@ -203,14 +210,13 @@ uint32_t segment_knn_tile_count(const uint32_t *h_seg_len, uint32_t S, uint32_t 
 void segment_knn_fill_tiles(const uint32_t *h_seg_start, const uint32_t *h_seg_len, uint32_t S, uint32_t max_len,
                             uint32_t *h_tiles);
 // row_base: index of data's row 0 within the whole reordered set (enters the padding hash of short partitions)
-// The same rows from the tensor cores' candidates (truth_tc.cu). *h_all: use launch_segment_knn; otherwise for the tiles
-// listed in h_tiles.
+// The same rows from the tensor cores' candidates (truth_tc.cu); items of TcLeft: tiles of 64 rows, three words each in h_tiles.
 bool segment_tc_eligible(const float *data, uint32_t dim, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree);
 size_t segment_tc_scratch_bytes(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len, uint32_t S,
-                                uint32_t max_len, uint32_t out_degree);
+                                uint32_t max_len, uint32_t out_degree, bool centred);
 cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len,
-                              uint32_t S, uint32_t max_len, uint32_t out_degree, uint32_t row_base, void *scratch, int32_t *out, bool *h_all,
-                              std::vector<uint32_t> *h_tiles, cudaStream_t stream);
+                              uint32_t S, uint32_t max_len, uint32_t out_degree, uint32_t row_base, bool centred, void *scratch, int32_t *out,
+                              TcLeft *h_left, std::vector<uint32_t> *h_tiles, cudaStream_t stream);
 cudaError_t launch_segment_knn(const float *data, uint32_t dim, const uint32_t *d_tiles, uint32_t tile_count,
                                uint32_t out_degree, uint32_t row_base, int32_t *out, cudaStream_t stream);
 

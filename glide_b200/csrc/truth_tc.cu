@@ -62,6 +62,7 @@ constexpr float kFarNorm = 1e36f, kFarBound = 1e34f, kFarQuery = 1e32f;
 struct TruthBad {
     uint32_t *gave_up;                       // a wait ran out: everything
     uint32_t *count, *items;
+    uint32_t *hopeful;                       // queries handed back that the error bound alone, not the rows, gave too many candidates
     uint32_t *seen;                          // segment form: one flag per half, each is listed once
     uint32_t first;                          // added to the queries of a pass
 };
@@ -96,10 +97,36 @@ __device__ __forceinline__ void report_bad(const TruthBad &bad, uint32_t item) {
 
 __device__ __forceinline__ float tf32_rest(float x) { return x - __uint_as_float(__float_as_uint(x) & 0xffffe000u); }
 
+// The point that rows are taken about in a second attempt (TcLeft): the mean of up to 64 rows, evenly spaced, of a call's base or
+// (segment form, in the CTAs of its first tile) of a partition.
+__global__ void __launch_bounds__(128) truth_centre_kernel(const float *__restrict__ data, uint32_t rows, uint32_t dim, const SegmentTile *__restrict__ segments,
+                                                           float *centre) {
+    if (segments != nullptr) {
+        const SegmentTile t = segments[blockIdx.y];
+        if (t.first != 0) return;
+        data += (uint64_t) t.seg_start * dim;
+        rows = t.seg_len;
+        centre += (uint64_t) t.part * dim;
+    }
+    const uint32_t d = blockIdx.x * 128u + threadIdx.x, count = min(rows, 64u);
+    if (d >= dim) return;
+    float sum = 0.0f, used = 0.0f;
+    for (uint32_t i = 0; i < count; i++) {
+        const float v = __ldg(data + (uint64_t) i * rows / count * dim + d);
+        if (fabsf(v) < 1e18f) {
+            sum += v;
+            used += 1.0f;
+        }
+    }
+    centre[d] = used > 0.0f ? sum / used : 0.0f;
+}
+
 // A warp per row: |x|^2, |x - tf32(x)|^2 (two floats per row if `rest` is given), the maxima, and the row padded to `pitch`.
-// Segment form: a CTA per tile, maxima per partition, the padded copy from row `padded_from` on.
+// Segment form: a CTA per tile, maxima per partition, the padded copy from row `padded_from` on. With a centre (one per partition)
+// x is the row less that; what the subtraction rounds off is far within the bound on the sums.
 __global__ void truth_rows_kernel(const float *__restrict__ data, uint32_t rows, uint32_t dim, float *norms, float *rest, uint32_t pitch,
-                                  float *padded, uint32_t padded_from, TruthTops *tops, const SegmentTile *__restrict__ segments) {
+                                  float *padded, uint32_t padded_from, TruthTops *tops, const SegmentTile *__restrict__ segments,
+                                  const float *__restrict__ centre) {
     __shared__ uint32_t top[2];
     if (threadIdx.x < 2) top[threadIdx.x] = 0;
     __syncthreads();
@@ -112,6 +139,7 @@ __global__ void truth_rows_kernel(const float *__restrict__ data, uint32_t rows,
         end = t.seg_start + min(t.first + kTile, t.seg_len);
         step = warps;
         tops += t.part;
+        if (centre != nullptr) centre += (uint64_t) t.part * dim;
     }
     for (uint64_t r = first + (threadIdx.x >> 5); r < end; r += step) {
         const float *row = data + r * dim;
@@ -126,7 +154,7 @@ __global__ void truth_rows_kernel(const float *__restrict__ data, uint32_t rows,
             }
         } else {
             for (uint32_t k = lane; k < pitch; k += 32) {
-                const float v = k < dim ? __ldg(row + k) : 0.0f, l = tf32_rest(v);
+                const float v = k < dim ? __ldg(row + k) - (centre != nullptr ? __ldg(centre + k) : 0.0f) : 0.0f, l = tf32_rest(v);
                 padded[(r - padded_from) * pitch + k] = v;
                 s += v * v;
                 t += l * l;
@@ -438,7 +466,21 @@ __global__ void __launch_bounds__(128) truth_threshold_kernel(const float *__res
         __syncthreads();
         const float G = (float) (below & 0xffffu), share = fminf((float) (below >> 16), G - 0.5f) / G;
         const float p = 1.0f - expf(logf(1.0f - share) * G / (float) cols);
-        if (p * (float) n > 1.25f * (float) cap) good = false;
+        if (p * (float) n > 1.25f * (float) cap) {
+            // were the bound nothing, the k-th smallest itself would be the threshold
+            const uint32_t least = ordered(kth);
+            g = 0;
+            for (uint32_t i = tid; i < groups; i += 128) g += keys[i] <= least ? 1u : 0u;
+            __syncthreads();
+            if (tid == 0) below = 0;
+            __syncthreads();
+            g = __reduce_add_sync(kFullMask, g);
+            if ((tid & 31u) == 0) atomicAdd(&below, g);
+            __syncthreads();
+            const float p0 = 1.0f - expf(logf(1.0f - fminf((float) below, G - 0.5f) / G) * G / (float) cols);
+            if (tid == 0 && good && p0 * (float) n < 0.5f * (float) cap) atomicAdd(bad.hopeful, 1u);
+            good = false;
+        }
     }
     if (tid != 0) return;
     thr[q] = good ? t : -__int_as_float(0x7f800000);
@@ -595,12 +637,12 @@ struct TruthPlan {
     uint32_t nb, qb, pitch;     // rows and queries per pass, padded row length
     bool pad;
     Sample sample, sample_last;   // of a full pass over queries, of the last one
-    size_t bad, items, tops, norms, rows, q_rows, q_norm, q_rest, thr, count, cand, gmin, best, total;
+    size_t bad, items, tops, centre, norms, rows, q_rows, q_norm, q_rest, thr, count, cand, gmin, best, total;
 };
 
-TruthPlan truth_plan(const TcPasses &passes, const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k) {
+TruthPlan truth_plan(const TcPasses &passes, const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k, bool centred) {
     TruthPlan p;
-    p.pad = (dim & 3u) != 0 || ((reinterpret_cast<uintptr_t>(base) | reinterpret_cast<uintptr_t>(queries)) & 15u) != 0;
+    p.pad = centred || (dim & 3u) != 0 || ((reinterpret_cast<uintptr_t>(base) | reinterpret_cast<uintptr_t>(queries)) & 15u) != 0;
     p.pitch = (dim + 3u) & ~3u;
     p.nb = std::min(n, std::max(k, passes.base_rows));   // the first pass has k results
     if (p.pad && (uint64_t) p.nb * p.pitch > passes.padded_values) p.nb = std::max(k, passes.padded_values / p.pitch);
@@ -611,8 +653,9 @@ TruthPlan truth_plan(const TcPasses &passes, const float *base, const float *que
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t o = at; at += up256(bytes); return o; };
     p.items = take((size_t) Q * 4);   // first: what it lists is answered from the rest of the scratch
-    p.bad = take(8 + sizeof(TruthTops));
-    p.tops = p.bad + 8;
+    p.bad = take(sizeof(TcLeft) + sizeof(TruthTops));
+    p.tops = p.bad + sizeof(TcLeft);
+    p.centre = take(centred ? (size_t) dim * 4 : 0);
     p.norms = take((size_t) p.nb * 4);
     p.q_norm = take((size_t) p.qb * 4);
     p.q_rest = take((size_t) p.qb * 4);
@@ -653,27 +696,28 @@ bool truth_tc_eligible(uint32_t n, uint32_t Q, uint32_t dim, uint32_t k) {
     return dim >= 16 && dim <= 4096 && k >= 1 && k <= 128 && n >= 1 && (uint64_t) n * Q * dim >= (1ull << 20) && encode_tiled_fn() != nullptr;
 }
 
-size_t truth_tc_scratch_bytes(const TcPasses &passes, const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k) {
-    return truth_plan(passes, base, queries, n, Q, dim, k).total;
+size_t truth_tc_scratch_bytes(const TcPasses &passes, const float *base, const float *queries, uint32_t n, uint32_t Q, uint32_t dim, uint32_t k, bool centred) {
+    return truth_plan(passes, base, queries, n, Q, dim, k, centred).total;
 }
 
-// What is left for the caller to answer by other means: h_left[0] != 0 everything, else h_left[1] queries, whose numbers lie at
-// the start of the scratch. Synchronises the stream.
+// What is left for the caller to answer by other means: see TcLeft. Synchronises the stream.
 cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t n, const float *queries, uint32_t Q, uint32_t dim, uint32_t k, int metric,
-                            void *scratch, uint32_t *out_ids, float *out_dists, uint32_t (&h_left)[2], cudaStream_t stream) {
-    const TruthPlan p = truth_plan(passes, base, queries, n, Q, dim, k);
+                            bool centred, void *scratch, uint32_t *out_ids, float *out_dists, TcLeft *h_left, cudaStream_t stream) {
+    const TruthPlan p = truth_plan(passes, base, queries, n, Q, dim, k, centred);
     char *w = static_cast<char *>(scratch);
     auto at = [&](size_t o) { return reinterpret_cast<float *>(w + o); };
-    uint32_t *left = reinterpret_cast<uint32_t *>(w + p.bad);
+    TcLeft *left = reinterpret_cast<TcLeft *>(w + p.bad);
     TruthTops *tops = reinterpret_cast<TruthTops *>(w + p.tops);
-    TruthBad bad{left, left + 1, reinterpret_cast<uint32_t *>(w + p.items), nullptr, 0};
+    TruthBad bad{&left->everything, &left->items, reinterpret_cast<uint32_t *>(w + p.items), &left->hopeful, nullptr, 0};
+    float *centre = centred ? at(p.centre) : nullptr;
     float *norms = at(p.norms), *q_norm = at(p.q_norm), *q_rest = at(p.q_rest), *thr = at(p.thr), *gmin = at(p.gmin);
     uint32_t *count = reinterpret_cast<uint32_t *>(w + p.count), *cand = reinterpret_cast<uint32_t *>(w + p.cand);
     u64 *best = reinterpret_cast<u64 *>(w + p.best);
-    h_left[0] = 1;
+    *h_left = TcLeft{1, 0, 0};
     const uint32_t sms = sm_count();
-    cudaError_t e = cudaMemsetAsync(left, 0, 8 + sizeof(TruthTops), stream);
+    cudaError_t e = cudaMemsetAsync(left, 0, sizeof(TcLeft) + sizeof(TruthTops), stream);
     if (e != cudaSuccess) return e;
+    if (centred) truth_centre_kernel<<<(dim + 127) / 128, 128, 0, stream>>>(base, n, dim, nullptr, centre);
 
     TruthArgs a{};
     a.dim = dim; a.cap = kCap; a.polls = passes.polls; a.kblocks = (p.pitch + kBlock - 1) / kBlock;
@@ -688,7 +732,7 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
         const uint32_t nq = Q - qa < p.qb ? Q - qa : p.qb;
         const float *qrows = queries + (size_t) qa * dim;
         float *q_padded = p.pad ? at(p.q_rows) : nullptr;
-        truth_rows_kernel<<<(nq + 7) / 8, 256, 0, stream>>>(qrows, nq, dim, q_norm, q_rest, p.pitch, q_padded, 0, nullptr, nullptr);
+        truth_rows_kernel<<<(nq + 7) / 8, 256, 0, stream>>>(qrows, nq, dim, q_norm, q_rest, p.pitch, q_padded, 0, nullptr, nullptr, centre);
         bad.first = qa;
         CUtensorMap tm_q, tm_b;
         SampleMaps tm_s{};
@@ -700,7 +744,7 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
             const float *brows = base + (size_t) ba * dim;
             float *b_padded = p.pad ? at(p.rows) : nullptr;
             const uint32_t blocks = std::min((nr + 7) / 8, 8u * sms);
-            truth_rows_kernel<<<blocks, 256, 0, stream>>>(brows, nr, dim, norms, nullptr, p.pitch, b_padded, 0, tops, nullptr);
+            truth_rows_kernel<<<blocks, 256, 0, stream>>>(brows, nr, dim, norms, nullptr, p.pitch, b_padded, 0, tops, nullptr, centre);
             if (!row_map(&tm_b, p.pad ? b_padded : brows, nr, p.pitch)) return cudaSuccess;
             a.n = nr;
             if (ba == 0) {
@@ -724,7 +768,7 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
     }
-    if ((e = cudaMemcpyAsync(h_left, left, 8, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
+    if ((e = cudaMemcpyAsync(h_left, left, sizeof(TcLeft), cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
     return cudaStreamSynchronize(stream);
 }
 
@@ -755,12 +799,13 @@ struct SegPlan {
     bool pad;
     uint32_t pitch, groups;
     std::vector<SegChunk> chunks;
-    size_t bad, items, seen, tops, tiles, norms, rest, thr, count, cand, gmin, rows, total;
+    size_t bad, items, seen, tops, centre, tiles, norms, rest, thr, count, cand, gmin, rows, total;
 };
 
-SegPlan seg_plan(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree) {
+SegPlan seg_plan(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len, uint32_t S, uint32_t max_len, uint32_t out_degree,
+                 bool centred) {
     SegPlan p;
-    p.pad = (dim & 3u) != 0 || (reinterpret_cast<uintptr_t>(data) & 15u) != 0;
+    p.pad = centred || (dim & 3u) != 0 || (reinterpret_cast<uintptr_t>(data) & 15u) != 0;
     p.pitch = (dim + 3u) & ~3u;
     p.groups = 1;
     size_t tiles = 0, parts = 0;
@@ -774,10 +819,11 @@ SegPlan seg_plan(const TcPasses &passes, const float *data, uint32_t rows, uint3
     const size_t slots = (size_t) (tiles < passes.tiles ? tiles : passes.tiles) * kTile;
     size_t at = 0;
     auto take = [&](size_t bytes) { const size_t o = at; at += up256(bytes); return o; };
-    p.bad = take(8 + 2 * tiles * 4 + parts * sizeof(TruthTops));
-    p.seen = p.bad + 8;
+    p.bad = take(sizeof(TcLeft) + 2 * tiles * 4 + parts * sizeof(TruthTops));
+    p.seen = p.bad + sizeof(TcLeft);
     p.tops = p.seen + 2 * tiles * 4;
     p.items = take(2 * tiles * 4);
+    p.centre = take(centred ? parts * dim * 4 : 0);
     p.tiles = take(tiles * sizeof(SegmentTile));
     p.norms = take((size_t) rows * 4);
     p.rest = take((size_t) rows * 4);
@@ -813,15 +859,16 @@ bool segment_tc_eligible(const float *data, uint32_t dim, const uint32_t *h_len,
 }
 
 size_t segment_tc_scratch_bytes(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len, uint32_t S,
-                                uint32_t max_len, uint32_t out_degree) {
-    return seg_plan(passes, data, rows, dim, h_start, h_len, S, max_len, out_degree).total;
+                                uint32_t max_len, uint32_t out_degree, bool centred) {
+    return seg_plan(passes, data, rows, dim, h_start, h_len, S, max_len, out_degree, centred).total;
 }
 
 // Exact kNN rows of every partition of at most max_len rows: what segment_knn_kernel writes, bit for bit. What is left for that
 // kernel: *h_all everything, otherwise h_tiles, three words each (its tiles). Synchronises the stream.
 cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_t rows, uint32_t dim, const uint32_t *h_start, const uint32_t *h_len,
-                              uint32_t S, uint32_t max_len, uint32_t out_degree, uint32_t row_base, void *scratch, int32_t *out, bool *h_all, std::vector<uint32_t> *h_tiles, cudaStream_t stream) {
-    const SegPlan p = seg_plan(passes, data, rows, dim, h_start, h_len, S, max_len, out_degree);
+                              uint32_t S, uint32_t max_len, uint32_t out_degree, uint32_t row_base, bool centred, void *scratch, int32_t *out, TcLeft *h_left,
+                              std::vector<uint32_t> *h_tiles, cudaStream_t stream) {
+    const SegPlan p = seg_plan(passes, data, rows, dim, h_start, h_len, S, max_len, out_degree, centred);
     std::vector<SegmentTile> tiles;
     uint32_t parts = 0;
     for (uint32_t s = 0; s < S; s++) {
@@ -831,18 +878,19 @@ cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_
         parts++;
     }
     h_tiles->clear();
-    *h_all = false;
+    *h_left = TcLeft{0, 0, 0};
     if (tiles.empty()) return cudaSuccess;
-    *h_all = true;
+    h_left->everything = 1;
     char *w = static_cast<char *>(scratch);
     auto at = [&](size_t o) { return reinterpret_cast<float *>(w + o); };
-    uint32_t *left = reinterpret_cast<uint32_t *>(w + p.bad);
+    TcLeft *left = reinterpret_cast<TcLeft *>(w + p.bad);
     TruthTops *tops = reinterpret_cast<TruthTops *>(w + p.tops);
-    const TruthBad bad{left, left + 1, reinterpret_cast<uint32_t *>(w + p.items), reinterpret_cast<uint32_t *>(w + p.seen), 0};
+    const TruthBad bad{&left->everything, &left->items, reinterpret_cast<uint32_t *>(w + p.items), &left->hopeful, reinterpret_cast<uint32_t *>(w + p.seen), 0};
+    float *centre = centred ? at(p.centre) : nullptr;
     SegmentTile *d_tiles = reinterpret_cast<SegmentTile *>(w + p.tiles);
     uint32_t *count = reinterpret_cast<uint32_t *>(w + p.count), *cand = reinterpret_cast<uint32_t *>(w + p.cand);
     float *padded = p.pad ? at(p.rows) : nullptr;
-    cudaError_t e = cudaMemsetAsync(left, 0, 8 + 2 * tiles.size() * 4 + parts * sizeof(TruthTops), stream);
+    cudaError_t e = cudaMemsetAsync(left, 0, sizeof(TcLeft) + 2 * tiles.size() * 4 + parts * sizeof(TruthTops), stream);
     // the table is pageable host memory: the copy has read it when the call returns
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_tiles, tiles.data(), tiles.size() * sizeof(SegmentTile), cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) return e;
@@ -854,7 +902,10 @@ cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_
     const size_t smem = umma_smem(a.stages), rr_smem = (size_t) kSegCap * 8 + (size_t) p.pitch * 4;
     if ((e = cudaFuncSetAttribute(truth_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
     for (const SegChunk &c : p.chunks) {
-        truth_rows_kernel<<<c.tiles, 256, 0, stream>>>(data, rows, dim, at(p.norms), at(p.rest), p.pitch, padded, c.row, tops, d_tiles + c.tile);
+        // (a grid's second dimension ends at 65,535)
+        for (uint32_t t = 0; centred && t < c.tiles; t += 32768)
+            truth_centre_kernel<<<dim3((dim + 127) / 128, std::min(c.tiles - t, 32768u)), 128, 0, stream>>>(data, 0, dim, d_tiles + c.tile + t, centre);
+        truth_rows_kernel<<<c.tiles, 256, 0, stream>>>(data, rows, dim, at(p.norms), at(p.rest), p.pitch, padded, c.row, tops, d_tiles + c.tile, centre);
         const float *mapped_rows = p.pad ? padded : data;
         CUtensorMap tm;
         SampleMaps tm_s{};
@@ -880,12 +931,12 @@ cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
     }
-    uint32_t h_left[2] = {1, 0};
-    if ((e = cudaMemcpyAsync(h_left, left, 8, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
-    if ((e = cudaStreamSynchronize(stream)) != cudaSuccess || h_left[0]) return e;
-    *h_all = false;
-    if (h_left[1] == 0) return cudaSuccess;
-    std::vector<uint32_t> items(h_left[1]);
+    TcLeft got{1, 0, 0};
+    if ((e = cudaMemcpyAsync(&got, left, sizeof got, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
+    if ((e = cudaStreamSynchronize(stream)) != cudaSuccess || got.everything) return e;
+    *h_left = got;
+    if (got.items == 0) return cudaSuccess;
+    std::vector<uint32_t> items(got.items);
     if ((e = cudaMemcpyAsync(items.data(), bad.items, items.size() * 4, cudaMemcpyDeviceToHost, stream)) != cudaSuccess) return e;
     if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
     for (const uint32_t i : items) {

@@ -311,3 +311,39 @@ def test_waits_that_run_out_leave_everything_to_the_tile_kernels(short_passes, d
     want_ids, want = api.bruteforce_knn(ctx, base, queries, 10)
     assert ctx.exact_knn_counts[1] == after[1]
     assert torch.equal(ids, want_ids) and torch.equal(dists, want)
+
+
+@pytest.mark.parametrize("dim", [40, 35])
+@pytest.mark.parametrize("offset", [1000, -30_000])
+def test_rows_far_from_the_origin_are_taken_about_their_middle(gpu_ctx, dim, offset):
+    """Norms far above the distances make every row a candidate; about a point amid the rows the bound is small again."""
+    rng = np.random.default_rng(dim)
+    base, queries = (torch.from_numpy(rng.random((m, dim), np.float32) + np.float32(offset)).to(gpu_ctx.torch_device) for m in (20_000, 100))
+    base[77, 3] = float("nan")
+    before = gpu_ctx.exact_knn_counts
+    ids, dists = api.bruteforce_knn(gpu_ctx, base, queries, 10)
+    after = gpu_ctx.exact_knn_counts
+    assert (after[0] - before[0], after[1] - before[1]) == (100, 0)
+    want_ids, want = _tile_kernel(gpu_ctx, base, queries, 10)
+    assert torch.equal(ids, want_ids) and torch.equal(dists, want)
+
+
+def test_partitions_far_from_the_origin_are_taken_about_their_middles(gpu_ctx):
+    lens = np.array([5000, 300, 6000], np.uint32)
+    start = np.concatenate([[0], np.cumsum(lens)[:-1]]).astype(np.uint32)
+    rng = np.random.default_rng(2)
+    rows = rng.random((int(lens.sum()), 36), np.float32)
+    for lo, n, offset in zip(start, lens, (1000, -400, 3000)):
+        rows[lo:lo + n] += np.float32(offset)
+    rows = torch.from_numpy(rows).to(gpu_ctx.torch_device)
+    before, stages = gpu_ctx.exact_knn_counts, gpu_ctx.tc_knn_fallbacks
+    got, _, _ = api.build_nnd(gpu_ctx, NNDescentParameter(32), rows, start, lens, exact_max_rows=16384)
+    after = gpu_ctx.exact_knn_counts
+    assert (after[2] - before[2], after[3] - before[3]) == (int(lens.sum()), 0) and gpu_ctx.tc_knn_fallbacks == stages
+    got = got.cpu().numpy()
+    for lo, n in zip(start, lens):
+        part = rows[int(lo):int(lo) + int(n)].contiguous()
+        check = rng.choice(int(n), 60, replace=False)
+        ids, _ = _tile_kernel(gpu_ctx, part, part[torch.from_numpy(check).to(part.device)].contiguous(), 33)
+        for r, row in zip(check, ids.cpu().numpy()):
+            assert list(got[int(lo) + r]) == [i for i in row if i != r][:32]
