@@ -110,10 +110,11 @@ class Context:
         self.lib.glide_exact_knn_counts(self.handle, out)
         return tuple(int(x) for x in out)
 
-    def limit_exact_knn(self, base_rows: int = 0, queries: int = 0, padded_values: int = 0, tiles: int = 0, polls: int = 0):
-        """Bounds the scratch of exact kNN from tensor-core candidates by the size of its passes, and the polls of a wait
-        inside its kernels (0: the default)."""
-        self.check(self.lib.glide_limit_exact_knn(self.handle, base_rows, queries, padded_values, tiles, polls))
+    def limit_exact_knn(self, base_rows: int = 0, queries: int = 0, padded_values: int = 0, tiles: int = 0,
+                        give_up: bool = False):
+        """Bounds the scratch of exact kNN from tensor-core candidates by the size of its passes (0: the default). give_up:
+        its kernels behave as if a wait had run out (a test of that path)."""
+        self.check(self.lib.glide_limit_exact_knn(self.handle, base_rows, queries, padded_values, tiles, 1 if give_up else 0))
 
     def empty(self, shape, dtype) -> torch.Tensor:
         return torch.empty(shape, dtype=dtype, device=self.torch_device)

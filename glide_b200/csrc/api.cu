@@ -538,13 +538,13 @@ void glide_exact_knn_counts(const glide_ctx *ctx, uint64_t out[4]) {
     for (int i = 0; i < 4; i++) out[i] = ctx->exact_knn[i];
 }
 
-int glide_limit_exact_knn(glide_ctx *ctx, uint32_t base_rows, uint32_t queries, uint32_t padded_values, uint32_t tiles, uint32_t polls) {
+int glide_limit_exact_knn(glide_ctx *ctx, uint32_t base_rows, uint32_t queries, uint32_t padded_values, uint32_t tiles, int give_up) {
     if (!ctx) return GLIDE_ERR_BAD_ARG;
     const TcPasses usual;
     ctx->tc_passes.base_rows = base_rows ? base_rows : usual.base_rows;
     ctx->tc_passes.queries = queries ? std::min(queries, usual.queries) : usual.queries;
     ctx->tc_passes.padded_values = padded_values ? padded_values : usual.padded_values;
-    ctx->tc_passes.polls = polls ? std::min(polls, usual.polls) : usual.polls;
+    ctx->tc_passes.give_up = give_up != 0;
     ctx->tc_passes.tiles = tiles ? std::min(tiles, usual.tiles) : usual.tiles;
     return GLIDE_OK;
 }

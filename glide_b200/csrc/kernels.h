@@ -183,7 +183,7 @@ struct TcPasses {
     uint32_t base_rows = 1u << 21;      // base rows of a bruteforce call
     uint32_t queries = 8192;            // its queries
     uint32_t padded_values = 1u << 26;  // values in the padded copy of rows that TMA cannot read (256 MB)
-    uint32_t polls = 1u << 22;          // of a wait inside these kernels before it gives up
+    bool give_up = false;               // the kernels behave as if a wait had run out
     uint32_t tiles = 148;               // CTAs of 128 rows of a launch over partitions (about 200 KB of shared memory each: one per SM)
 };
 // The same results from the tensor cores' candidates (truth_tc.cu); items of TcLeft: queries, whose numbers are the first words

@@ -76,13 +76,12 @@ struct SegmentTile {
 struct TruthArgs {
     uint32_t n, Q, dim, kblocks, stages, cap;
     uint32_t map_from;                       // the tensor maps' first row
-    uint32_t polls;                          // of a wait
+    bool give_up;                            // as if a wait had run out
     const SegmentTile *segments;             // segment form: one per CTA; per-query arrays are indexed by CTA * 128 + row
     uint32_t slices;                         // CTA (query tile, slice) takes tiles slice, slice + slices, ...
     // sample pass: column c stands for row c * stride; a thread keeps the minima of its columns over `span` of its tiles,
     // takes the minimum of every `fold` of them and stores those, for each of `runs` such spans; `groups` minima per query
     uint32_t stride, span, runs, fold, groups;
-    bool sample;
     const float *norms;
     const float *thr;                        // per query (select pass)
     float *gmin;                             // Q x groups
@@ -121,30 +120,32 @@ __global__ void __launch_bounds__(128) truth_centre_kernel(const float *__restri
     centre[d] = used > 0.0f ? sum / used : 0.0f;
 }
 
-// A warp per row: |x|^2, |x - tf32(x)|^2 (two floats per row if `rest` is given), the maxima, and the row padded to `pitch`.
-// Segment form: a CTA per tile, maxima per partition, the padded copy from row `padded_from` on. With a centre (one per partition)
-// x is the row less that; what the subtraction rounds off is far within the bound on the sums.
-__global__ void truth_rows_kernel(const float *__restrict__ data, uint32_t rows, uint32_t dim, float *norms, float *rest, uint32_t pitch,
-                                  float *padded, uint32_t padded_from, TruthTops *tops, const SegmentTile *__restrict__ segments,
-                                  const float *__restrict__ centre) {
+// A warp per row: |x|^2, |x - tf32(x)|^2 (two floats per row if `rest` is given) and the maxima. Segment form: a CTA per tile,
+// maxima per partition. Not kRowsInPlace: the rows padded to `pitch` are written too, from row `padded_from` on; kRowsCentred: x is
+// the row less a centre (one per partition); what the subtraction rounds off is far within the bound on the sums.
+enum RowsForm : int { kRowsInPlace = 0, kRowsPadded = 1, kRowsCentred = 2 };
+template<int FORM>
+__global__ void __launch_bounds__(256, 8) truth_rows_kernel(const float *__restrict__ data, uint32_t rows, uint32_t dim, float *norms, float *rest,
+                                                            uint32_t pitch, float *padded, uint32_t padded_from, TruthTops *tops,
+                                                            const SegmentTile *__restrict__ segments, const float *__restrict__ centre) {
     __shared__ uint32_t top[2];
     if (threadIdx.x < 2) top[threadIdx.x] = 0;
     __syncthreads();
     const uint32_t lane = lane_id(), warps = blockDim.x >> 5;
     uint32_t best_n = 0, best_r = 0;
-    uint64_t first = (uint64_t) blockIdx.x * warps, end = rows, step = (uint64_t) gridDim.x * warps;
+    uint32_t r = blockIdx.x * warps + (threadIdx.x >> 5), end = rows, step = gridDim.x * warps;
     if (segments != nullptr) {
         const SegmentTile t = segments[blockIdx.x];
-        first = t.seg_start + t.first;
+        r = t.seg_start + t.first + (threadIdx.x >> 5);
         end = t.seg_start + min(t.first + kTile, t.seg_len);
         step = warps;
         tops += t.part;
-        if (centre != nullptr) centre += (uint64_t) t.part * dim;
+        if constexpr (FORM == kRowsCentred) centre += (uint64_t) t.part * dim;
     }
-    for (uint64_t r = first + (threadIdx.x >> 5); r < end; r += step) {
-        const float *row = data + r * dim;
+    for (; r < end; r += step) {
+        const float *row = data + (uint64_t) r * dim;
         float s = 0.0f, t = 0.0f;
-        if (padded == nullptr) {
+        if constexpr (FORM == kRowsInPlace) {
             const float4 *row4 = reinterpret_cast<const float4 *>(row);   // dim % 4 == 0 and aligned, or a padded copy would be wanted
             for (uint32_t k = lane; k < (dim >> 2); k += 32) {
                 const float4 v = __ldg(row4 + k);
@@ -153,9 +154,12 @@ __global__ void truth_rows_kernel(const float *__restrict__ data, uint32_t rows,
                 t += l.x * l.x + l.y * l.y + l.z * l.z + l.w * l.w;
             }
         } else {
+            float *copy = padded + (uint64_t) (r - padded_from) * pitch;
             for (uint32_t k = lane; k < pitch; k += 32) {
-                const float v = k < dim ? __ldg(row + k) - (centre != nullptr ? __ldg(centre + k) : 0.0f) : 0.0f, l = tf32_rest(v);
-                padded[(r - padded_from) * pitch + k] = v;
+                float v = k < dim ? __ldg(row + k) : 0.0f;
+                if constexpr (FORM == kRowsCentred) v -= k < dim ? __ldg(centre + k) : 0.0f;
+                const float l = tf32_rest(v);
+                copy[k] = v;
                 s += v * v;
                 t += l * l;
             }
@@ -170,10 +174,8 @@ __global__ void truth_rows_kernel(const float *__restrict__ data, uint32_t rows,
             norms[r] = far ? __int_as_float(0x7f800000) : s;
             if (rest) rest[r] = far ? 0.0f : t;
         }
-        if (!far) {
-            best_n = max(best_n, __float_as_uint(s));
-            best_r = max(best_r, __float_as_uint(t));
-        }
+        best_n = max(best_n, far ? 0u : __float_as_uint(s));
+        best_r = max(best_r, far ? 0u : __float_as_uint(t));
     }
     if (lane == 0) {
         atomicMax(&top[0], best_n);
@@ -184,6 +186,11 @@ __global__ void truth_rows_kernel(const float *__restrict__ data, uint32_t rows,
         atomicMax(&tops->norm, top[0]);
         atomicMax(&tops->rest, top[1]);
     }
+}
+
+void (*rows_kernel(bool pad, bool centred))(const float *, uint32_t, uint32_t, float *, float *, uint32_t, float *, uint32_t, TruthTops *, const SegmentTile *,
+                                            const float *) {
+    return centred ? truth_rows_kernel<kRowsCentred> : (pad ? truth_rows_kernel<kRowsPadded> : truth_rows_kernel<kRowsInPlace>);
 }
 
 // 32 / fold minima, 16-byte aligned; m is FLT_MAX again afterwards.
@@ -208,13 +215,17 @@ __device__ __forceinline__ void store_minima(float (&m)[32], uint32_t fold, floa
     for (int j = 0; j < 32; j++) m[j] = FLT_MAX;
 }
 
+// Maps of the base rows: a call of one stride has one, partitions have strides of their own.
 constexpr uint32_t kMaxStride = 16;
 struct SampleMaps {
     CUtensorMap of[kMaxStride];              // by stride - 1
 };
+__device__ __forceinline__ const CUtensorMap *map_of(const CUtensorMap &m, uint32_t) { return &m; }
+__device__ __forceinline__ const CUtensorMap *map_of(const SampleMaps &m, uint32_t stride) { return m.of + (stride - 1u); }
 
-__global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthArgs a, const __grid_constant__ CUtensorMap tm_q,
-                                                                   const __grid_constant__ CUtensorMap tm_b, const __grid_constant__ SampleMaps tm_s) {
+// SAMPLE: the sample pass, a kernel of its own for the registers of its minima (in one kernel the select pass took 4 % longer).
+template<bool SAMPLE, typename Maps>
+__global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthArgs a, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ Maps tm_b) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t) 1023);
     const uint32_t kblocks = a.kblocks, stages = a.stages;
@@ -234,11 +245,11 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
     const uint32_t q0 = seg ? blockIdx.x * kTile : (blockIdx.x % qtiles) * kTile;      // index of the first query's results
     const uint32_t q_row = seg ? part_of.seg_start + part_of.first - a.map_from : q0;   // its row in the query map
     const uint32_t slice = seg ? 0u : blockIdx.x / qtiles, slices = seg ? 1u : a.slices;
-    const uint32_t b_row = part_of.seg_start, m_row = b_row - a.map_from, stride = a.sample ? part_of.stride : 1u;
+    const uint32_t b_row = part_of.seg_start, m_row = b_row - a.map_from, stride = SAMPLE ? part_of.stride : 1u;
     const uint32_t n = part_of.seg_len / stride, all = (n + kTile - 1) / kTile;             // columns, tiles of them
     // a query of the CTA, by thread: one that wants candidates?
     bool wanted = tid < kTile && (seg ? part_of.first + tid < part_of.seg_len : q0 + tid < a.Q);
-    if (wanted && !a.sample) wanted = __ldg(a.thr + q0 + tid) != -__int_as_float(0x7f800000);
+    if (wanted && !SAMPLE) wanted = __ldg(a.thr + q0 + tid) != -__int_as_float(0x7f800000);
 
     if (tid == 0) {
         mbar_init(a_full, 1);
@@ -246,7 +257,7 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
         for (uint32_t s = 0; s < stages; s++) { mbar_init(full + s, 1); mbar_init(freed + s, 1); }
         for (int c = 0; c < 2; c++) { mbar_init(mma_done + c, 1); mbar_init(tmem_free + c, kEpi); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        *failed = 0;
+        *failed = a.give_up ? 1u : 0u;
     }
     if (warp == kEpi) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(2 * kTile) : "memory");
@@ -271,11 +282,11 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
             for (uint32_t t = 0; t < tiles && ok; t++) {
                 const uint32_t c0 = (slice + t * slices) * kTile;
                 for (uint32_t kb = 0; kb < kblocks; kb++) {
-                    if (use > 0 && !mbar_wait(freed + s, (use - 1) & 1u, failed, a.polls)) { ok = false; break; }
+                    if (use > 0 && !mbar_wait(freed + s, (use - 1) & 1u, failed)) { ok = false; break; }
                     uint8_t *dst = ring + s * stage_bytes;
                     mbar_expect_tx(full + s, stage_bytes);
-                    if (a.sample) tma_load_3d(dst, &tm_s.of[stride - 1u], kb * kBlock, m_row % stride, m_row / stride + c0, full + s);
-                    else tma_load_2d(dst, &tm_b, kb * kBlock, m_row + c0, full + s);
+                    if constexpr (SAMPLE) tma_load_3d(dst, map_of(tm_b, stride), kb * kBlock, m_row % stride, m_row / stride + c0, full + s);
+                    else tma_load_2d(dst, map_of(tm_b, 1u), kb * kBlock, m_row + c0, full + s);
                     if (!resident) tma_load_2d(dst + kBlockBytes, &tm_q, kb * kBlock, q_row, full + s);
                     copies++;
                     if (++s == stages) { s = 0; use++; }
@@ -287,13 +298,13 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
         if (lane == 0 && tiles > 0) {
             const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((kTile >> 3) << 17) | ((kTile >> 4) << 24);
             const uint32_t a_addr = smem_u32(As), r_addr = smem_u32(ring);
-            bool ok = !resident || mbar_wait(a_full, 0, failed, a.polls);
+            bool ok = !resident || mbar_wait(a_full, 0, failed);
             uint32_t s = 0, use = 0;
             for (uint32_t t = 0; t < tiles && ok; t++) {
                 const uint32_t acc = t & 1u;
-                if (t >= 2) ok = mbar_wait(tmem_free + acc, ((t >> 1) - 1) & 1u, failed, a.polls);
+                if (t >= 2) ok = mbar_wait(tmem_free + acc, ((t >> 1) - 1) & 1u, failed);
                 for (uint32_t kb = 0; kb < kblocks && ok; kb++) {
-                    ok = mbar_wait(full + s, use & 1u, failed, a.polls);
+                    ok = mbar_wait(full + s, use & 1u, failed);
                     if (!ok) break;
                     fence_after();
                     const uint32_t b = r_addr + s * stage_bytes, q = resident ? a_addr + kb * kBlockBytes : b + kBlockBytes;
@@ -310,7 +321,7 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
         // ================= epilogue: thread (query, part) owns 32 columns of every tile =================
         const uint32_t quad = warp & 3u, part = warp >> 2, q = q0 + quad * 32u + lane;
         bool active = seg ? part_of.first + quad * 32u + lane < part_of.seg_len : q < a.Q;
-        const float thr = (active && !a.sample) ? __ldg(a.thr + q) : 0.0f;
+        const float thr = (active && !SAMPLE) ? __ldg(a.thr + q) : 0.0f;
         active = active && thr != -__int_as_float(0x7f800000);
         float *cn = cn_w + warp * 32u;
         auto norm_of = [&](uint32_t t) {
@@ -329,7 +340,7 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
             ahead = norm_of(t + 1);
             __syncwarp();
             const uint32_t acc = t & 1u, c0 = (slice + t * slices) * kTile + part * 32u;
-            bool ok = !*failed && mbar_wait(mma_done + acc, (t >> 1) & 1u, failed, a.polls);
+            bool ok = !*failed && mbar_wait(mma_done + acc, (t >> 1) & 1u, failed);
             ok = __all_sync(kFullMask, ok);
             if (!ok) break;
             fence_after();
@@ -352,7 +363,7 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
                 for (int j = 0; j < 32; j++)
                     if (c0 + j >= n) e[j] = FLT_MAX;
             }
-            if (a.sample) {
+            if (SAMPLE) {
 #pragma unroll
                 for (int j = 0; j < 32; j++) m[j] = fminf(m[j], e[j]);
                 if (--left == 0 || t + 1 == tiles) {
@@ -375,7 +386,7 @@ __global__ void __launch_bounds__(kTruthThreads) truth_umma_kernel(const TruthAr
                 }
             }
         }
-        if (a.sample)   // spans that this CTA has no tile for
+        if (SAMPLE)   // spans that this CTA has no tile for
             for (; run < part_of.runs; run++) store_minima(m, a.fold, minima ? minima + run * (kTile / a.fold) : nullptr);
         if (*failed && lane == 0) atomicExch(a.gave_up, 1u);
     }
@@ -405,9 +416,25 @@ __global__ void __launch_bounds__(128) truth_threshold_kernel(const float *__res
                                                               const float *__restrict__ q_norm, const float *__restrict__ q_rest, uint32_t dim,
                                                               const SegmentTile *segments, const TruthTops *tops, uint32_t n, uint32_t cols, uint32_t cap,
                                                               const TruthBad bad, float *thr, uint32_t *count) {
-    extern __shared__ uint32_t keys[];
-    __shared__ uint32_t below;
+    extern __shared__ uint32_t keys[];   // a thread reads those that it has written itself
+    __shared__ uint32_t part[2][4];
     const uint32_t q = blockIdx.x, tid = threadIdx.x;
+    __shared__ uint32_t range[4][3];     // by warp: smallest and largest key of the groups that have a row, their number
+    // the CTA's sum; calls take turns with the two sets of words, so that one barrier each is enough
+    uint32_t turn = 0;
+    auto cta_sum = [&](uint32_t x) {
+        x = __reduce_add_sync(kFullMask, x);
+        if ((tid & 31u) == 0) part[turn][tid >> 5] = x;
+        __syncthreads();
+        x = part[turn][0] + part[turn][1] + part[turn][2] + part[turn][3];
+        turn ^= 1u;
+        return x;
+    };
+    auto keys_to = [&](uint32_t limit) {
+        uint32_t c = 0;
+        for (uint32_t i = tid; i < groups; i += 128) c += keys[i] <= limit ? 1u : 0u;
+        return c;
+    };
     uint32_t row = q, pitch = groups, item = q;   // the query's row in q_norm and q_rest, minima per query in gmin
     if (best != nullptr && thr[q] == -__int_as_float(0x7f800000)) return;   // handed back by an earlier pass
     if (segments != nullptr) {
@@ -423,22 +450,35 @@ __global__ void __launch_bounds__(128) truth_threshold_kernel(const float *__res
         item = 2u * t.index + (r - t.first) / (kTile / 2);
     }
     float kth;
+    uint32_t with_row = 0;
     if (best == nullptr) {
-        for (uint32_t i = tid; i < groups; i += 128) keys[i] = ordered(gmin[(uint64_t) q * pitch + i]);
-        uint32_t lo = 0, hi = 0xffffffffu;   // smallest key with at least k keys at or below it
-        while (lo < hi) {
-            const uint32_t mid = lo + ((hi - lo) >> 1);
-            if (tid == 0) below = 0;
-            __syncthreads();
-            uint32_t c = 0;
-            for (uint32_t i = tid; i < groups; i += 128) c += keys[i] <= mid ? 1u : 0u;
-            c = __reduce_add_sync(kFullMask, c);
-            if ((tid & 31u) == 0) atomicAdd(&below, c);
-            __syncthreads();
-            if (below >= k) hi = mid; else lo = mid + 1;
-            __syncthreads();
+        uint32_t lo = 0xffffffffu, hi = 0, has_row = 0;
+        for (uint32_t i = tid; i < groups; i += 128) {
+            const uint32_t key = ordered(gmin[(uint64_t) q * pitch + i]);
+            keys[i] = key;
+            if (key < ordered(FLT_MAX)) {
+                lo = min(lo, key);
+                hi = max(hi, key);
+                has_row++;
+            }
         }
-        kth = from_ordered(lo);
+        lo = __reduce_min_sync(kFullMask, lo);
+        hi = __reduce_max_sync(kFullMask, hi);
+        has_row = __reduce_add_sync(kFullMask, has_row);
+        if ((tid & 31u) == 0) {
+            range[tid >> 5][0] = lo;
+            range[tid >> 5][1] = hi;
+            range[tid >> 5][2] = has_row;
+        }
+        __syncthreads();
+        lo = min(min(range[0][0], range[1][0]), min(range[2][0], range[3][0]));
+        hi = max(max(range[0][1], range[1][1]), max(range[2][1], range[3][1]));
+        with_row = range[0][2] + range[1][2] + range[2][2] + range[3][2];
+        while (lo < hi) {   // the smallest key with at least k keys at or below it
+            const uint32_t mid = lo + ((hi - lo) >> 1);
+            if (cta_sum(keys_to(mid)) >= k) hi = mid; else lo = mid + 1;
+        }
+        kth = with_row >= k ? from_ordered(lo) : FLT_MAX;   // (beyond every bound: the query is handed back)
     } else {
         kth = __uint_as_float((uint32_t) (best[(uint64_t) q * k + k - 1] >> 32)) - q_norm[row];
     }
@@ -452,33 +492,15 @@ __global__ void __launch_bounds__(128) truth_threshold_kernel(const float *__res
     bool good = fabsf(t) < kFarBound && q_norm[row] < kFarQuery;
     if (best == nullptr && n > cap) {
         // of G groups that have a row, g have one at or below t: (1 - p)^(cols / G) = 1 - g / G for the share p of such rows
-        const uint32_t limit = ordered(t);
-        uint32_t g = 0, all = 0;
-        for (uint32_t i = tid; i < groups; i += 128) {
-            g += keys[i] <= limit ? 1u : 0u;
-            all += keys[i] < ordered(FLT_MAX) ? 1u : 0u;
-        }
-        if (tid == 0) below = 0;
-        __syncthreads();
-        g = __reduce_add_sync(kFullMask, g);
-        all = __reduce_add_sync(kFullMask, all);
-        if ((tid & 31u) == 0) atomicAdd(&below, (g << 16) | all);   // at most 4,096 groups
-        __syncthreads();
-        const float G = (float) (below & 0xffffu), share = fminf((float) (below >> 16), G - 0.5f) / G;
-        const float p = 1.0f - expf(logf(1.0f - share) * G / (float) cols);
-        if (p * (float) n > 1.25f * (float) cap) {
+        const float G = (float) with_row;
+        auto expected = [&](float limit) {
+            const float share = fminf((float) cta_sum(keys_to(ordered(limit))), G - 0.5f) / G;
+            return (1.0f - expf(logf(1.0f - share) * G / (float) cols)) * (float) n;
+        };
+        if (expected(t) > 1.25f * (float) cap) {
             // were the bound nothing, the k-th smallest itself would be the threshold
-            const uint32_t least = ordered(kth);
-            g = 0;
-            for (uint32_t i = tid; i < groups; i += 128) g += keys[i] <= least ? 1u : 0u;
-            __syncthreads();
-            if (tid == 0) below = 0;
-            __syncthreads();
-            g = __reduce_add_sync(kFullMask, g);
-            if ((tid & 31u) == 0) atomicAdd(&below, g);
-            __syncthreads();
-            const float p0 = 1.0f - expf(logf(1.0f - fminf((float) below, G - 0.5f) / G) * G / (float) cols);
-            if (tid == 0 && good && p0 * (float) n < 0.5f * (float) cap) atomicAdd(bad.hopeful, 1u);
+            const bool hopeful = expected(kth) < 0.5f * (float) cap;
+            if (tid == 0 && good && hopeful) atomicAdd(bad.hopeful, 1u);
             good = false;
         }
     }
@@ -603,9 +625,10 @@ size_t up256(size_t x) { return (x + 255) & ~(size_t) 255; }
 
 // The sample of a pass over n rows for k neighbours, taken by `slices` CTAs per query tile: every stride-th row. The
 // select pass lets about stride x k columns through, the sample costs 1 / stride of it: 16 where at least 64 k rows remain,
-// less for smaller sets. 8 k minima, so that few of the k smallest share one: a thread's 32 columns over as many tiles as
-// that leaves; where few queries spread over many CTAs give thousands more, a thread folds its columns. At least
-// min(k, n) minima have a row: with one tile all of its rows have a minimum each, with more the first one fills 128.
+// less for smaller sets. 8 k minima or more, so that few of the k smallest share one: a thread's 32 columns over as many tiles as
+// that leaves; where few queries spread over many CTAs give 64 k and more, a thread folds its columns (every minimum costs the
+// threshold kernel time; a fold of eight still keeps four neighbours in the file apart). At least min(k, n) minima have a row:
+// with one tile all of its rows have a minimum each, with more the first one fills 128, or 32 k and more are left.
 struct Sample {
     uint32_t stride, slices, span, runs, fold, groups;
 };
@@ -619,7 +642,7 @@ Sample sample_of(uint32_t n, uint32_t k, uint32_t slices) {
     s.span = (per + runs - 1) / runs;
     s.runs = (per + s.span - 1) / s.span;
     s.fold = 1;
-    while (s.fold < 8 && s.slices * s.runs * kTile / s.fold > 4096u) s.fold *= 2;
+    while (s.fold < 8 && s.slices * s.runs * kTile / s.fold >= 64u * k) s.fold *= 2;
     s.groups = s.slices * s.runs * kTile / s.fold;
     return s;
 }
@@ -681,7 +704,10 @@ bool row_map(CUtensorMap *tm, const float *ptr, uint32_t rows, uint32_t pitch) {
 // A kernel is loaded when its attributes are first asked for; most builds whose rows knn_tc.cu does not take come here.
 cudaError_t preload_truth_kernels() {
     cudaFuncAttributes f;
-    const void *kernels[] = {reinterpret_cast<const void *>(truth_rows_kernel), reinterpret_cast<const void *>(truth_umma_kernel),
+    const void *kernels[] = {reinterpret_cast<const void *>(truth_rows_kernel<kRowsInPlace>), reinterpret_cast<const void *>(truth_rows_kernel<kRowsPadded>),
+                             reinterpret_cast<const void *>(truth_umma_kernel<false, CUtensorMap>),
+                             reinterpret_cast<const void *>(truth_umma_kernel<true, CUtensorMap>),
+                             reinterpret_cast<const void *>(truth_umma_kernel<true, SampleMaps>),
                              reinterpret_cast<const void *>(truth_threshold_kernel), reinterpret_cast<const void *>(truth_rerank_kernel),
                              reinterpret_cast<const void *>(segment_rerank_kernel)};
     for (const void *k : kernels) {
@@ -720,11 +746,12 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
     if (centred) truth_centre_kernel<<<(dim + 127) / 128, 128, 0, stream>>>(base, n, dim, nullptr, centre);
 
     TruthArgs a{};
-    a.dim = dim; a.cap = kCap; a.polls = passes.polls; a.kblocks = (p.pitch + kBlock - 1) / kBlock;
+    a.dim = dim; a.cap = kCap; a.give_up = passes.give_up; a.kblocks = (p.pitch + kBlock - 1) / kBlock;
     a.stages = ring_stages(a.kblocks);
     a.norms = norms; a.thr = thr; a.gmin = gmin; a.count = count; a.cand = cand; a.gave_up = bad.gave_up;
     const size_t smem = umma_smem(a.stages);
-    if ((e = cudaFuncSetAttribute(truth_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(truth_umma_kernel<true, CUtensorMap>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(truth_umma_kernel<false, CUtensorMap>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
     const size_t rr_smem = 4096 * 8 + (size_t) p.pitch * 4;
     if (rr_smem > 48 * 1024 && (e = cudaFuncSetAttribute(truth_rerank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) rr_smem)) != cudaSuccess) return e;
 
@@ -732,10 +759,10 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
         const uint32_t nq = Q - qa < p.qb ? Q - qa : p.qb;
         const float *qrows = queries + (size_t) qa * dim;
         float *q_padded = p.pad ? at(p.q_rows) : nullptr;
-        truth_rows_kernel<<<(nq + 7) / 8, 256, 0, stream>>>(qrows, nq, dim, q_norm, q_rest, p.pitch, q_padded, 0, nullptr, nullptr, centre);
+        rows_kernel(p.pad, centred)<<<(nq + 7) / 8, 256, 0, stream>>>(qrows, nq, dim, q_norm, q_rest, p.pitch, q_padded, 0, nullptr, nullptr, centre);
         bad.first = qa;
         CUtensorMap tm_q, tm_b;
-        SampleMaps tm_s{};
+        CUtensorMap tm_s;   // every stride-th row
         if (!row_map(&tm_q, p.pad ? q_padded : qrows, nq, p.pitch)) return cudaSuccess;
         a.Q = nq;
         const uint32_t qtiles = (nq + kTile - 1) / kTile;
@@ -744,24 +771,22 @@ cudaError_t launch_truth_tc(const TcPasses &passes, const float *base, uint32_t 
             const float *brows = base + (size_t) ba * dim;
             float *b_padded = p.pad ? at(p.rows) : nullptr;
             const uint32_t blocks = std::min((nr + 7) / 8, 8u * sms);
-            truth_rows_kernel<<<blocks, 256, 0, stream>>>(brows, nr, dim, norms, nullptr, p.pitch, b_padded, 0, tops, nullptr, centre);
+            rows_kernel(p.pad, centred)<<<blocks, 256, 0, stream>>>(brows, nr, dim, norms, nullptr, p.pitch, b_padded, 0, tops, nullptr, centre);
             if (!row_map(&tm_b, p.pad ? b_padded : brows, nr, p.pitch)) return cudaSuccess;
             a.n = nr;
             if (ba == 0) {
                 const Sample &m = nq == p.qb ? p.sample : p.sample_last;
-                if (!make_strided_row_map(&tm_s.of[m.stride - 1], p.pad ? b_padded : brows, nr, p.pitch, m.stride, kTile)) return cudaSuccess;
-                a.sample = true;
+                if (!make_strided_row_map(&tm_s, p.pad ? b_padded : brows, nr, p.pitch, m.stride, kTile)) return cudaSuccess;
                 a.slices = m.slices;
                 a.stride = m.stride; a.span = m.span; a.runs = m.runs; a.fold = m.fold; a.groups = m.groups;
-                truth_umma_kernel<<<qtiles * m.slices, kTruthThreads, smem, stream>>>(a, tm_q, tm_b, tm_s);
+                truth_umma_kernel<true, CUtensorMap><<<qtiles * m.slices, kTruthThreads, smem, stream>>>(a, tm_q, tm_s);
                 truth_threshold_kernel<<<nq, 128, (size_t) m.groups * 4, stream>>>(gmin, m.groups, k, nullptr, q_norm, q_rest, dim, nullptr, tops, nr, nr / m.stride, kCap,
                                                                                        bad, thr, count);
             } else {
                 truth_threshold_kernel<<<nq, 128, 0, stream>>>(nullptr, 0, k, best, q_norm, q_rest, dim, nullptr, tops, nr, 0, kCap, bad, thr, count);
             }
-            a.sample = false;
             a.slices = std::min(slices_of(nq, sms), (nr + kTile - 1) / kTile);
-            truth_umma_kernel<<<qtiles * a.slices, kTruthThreads, smem, stream>>>(a, tm_q, tm_b, tm_s);
+            truth_umma_kernel<false, CUtensorMap><<<qtiles * a.slices, kTruthThreads, smem, stream>>>(a, tm_q, tm_b);
             const bool last = ba + nr == n;
             truth_rerank_kernel<<<nq, 128, rr_smem, stream>>>(base, ba, qrows, dim, cand, count, k, best, ba > 0, metric,
                                                               last ? out_ids + (size_t) qa * k : nullptr, last && out_dists ? out_dists + (size_t) qa * k : nullptr, thr, bad);
@@ -895,17 +920,18 @@ cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_tiles, tiles.data(), tiles.size() * sizeof(SegmentTile), cudaMemcpyHostToDevice, stream);
     if (e != cudaSuccess) return e;
     TruthArgs a{};
-    a.dim = dim; a.cap = kSegCap; a.polls = passes.polls; a.kblocks = (p.pitch + kBlock - 1) / kBlock; a.stages = ring_stages(a.kblocks);
+    a.dim = dim; a.cap = kSegCap; a.give_up = passes.give_up; a.kblocks = (p.pitch + kBlock - 1) / kBlock; a.stages = ring_stages(a.kblocks);
     a.groups = p.groups;
     a.fold = 1;
     a.norms = at(p.norms); a.thr = at(p.thr); a.gmin = at(p.gmin); a.count = count; a.cand = cand; a.gave_up = bad.gave_up;
     const size_t smem = umma_smem(a.stages), rr_smem = (size_t) kSegCap * 8 + (size_t) p.pitch * 4;
-    if ((e = cudaFuncSetAttribute(truth_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(truth_umma_kernel<true, SampleMaps>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(truth_umma_kernel<false, CUtensorMap>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem)) != cudaSuccess) return e;
     for (const SegChunk &c : p.chunks) {
         // (a grid's second dimension ends at 65,535)
         for (uint32_t t = 0; centred && t < c.tiles; t += 32768)
             truth_centre_kernel<<<dim3((dim + 127) / 128, std::min(c.tiles - t, 32768u)), 128, 0, stream>>>(data, 0, dim, d_tiles + c.tile + t, centre);
-        truth_rows_kernel<<<c.tiles, 256, 0, stream>>>(data, rows, dim, at(p.norms), at(p.rest), p.pitch, padded, c.row, tops, d_tiles + c.tile, centre);
+        rows_kernel(p.pad, centred)<<<c.tiles, 256, 0, stream>>>(data, rows, dim, at(p.norms), at(p.rest), p.pitch, padded, c.row, tops, d_tiles + c.tile, centre);
         const float *mapped_rows = p.pad ? padded : data;
         CUtensorMap tm;
         SampleMaps tm_s{};
@@ -921,12 +947,10 @@ cudaError_t launch_segment_tc(const TcPasses &passes, const float *data, uint32_
         for (uint32_t first = 0; first < c.tiles; first += passes.tiles) {
             const uint32_t n = std::min(c.tiles - first, passes.tiles);
             a.segments = d_tiles + c.tile + first;
-            a.sample = true;
-            truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm, tm_s);
+            truth_umma_kernel<true, SampleMaps><<<n, kTruthThreads, smem, stream>>>(a, tm, tm_s);
             truth_threshold_kernel<<<n * kTile, 128, (size_t) p.groups * 4, stream>>>(a.gmin, p.groups, out_degree + 1, nullptr, a.norms, at(p.rest), dim,
                                                                                       a.segments, tops, 0, 0, kSegCap, bad, at(p.thr), count);
-            a.sample = false;
-            truth_umma_kernel<<<n, kTruthThreads, smem, stream>>>(a, tm, tm, tm_s);
+            truth_umma_kernel<false, CUtensorMap><<<n, kTruthThreads, smem, stream>>>(a, tm, tm);
             segment_rerank_kernel<<<n * kTile, 128, rr_smem, stream>>>(data, dim, a.segments, cand, count, out_degree, row_base, out, at(p.thr), bad);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }

@@ -89,8 +89,8 @@ __device__ __forceinline__ bool mbar_done(uint64_t *bar, uint32_t parity) {
         : "memory");
     return done != 0;
 }
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *failed, uint32_t polls = kSpinLimit) {
-    for (uint32_t spin = 0; spin < polls; spin++) {
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *failed) {
+    for (uint32_t spin = 0; spin < kSpinLimit; spin++) {
         if (mbar_done(bar, parity)) return true;
         if ((spin & 1023u) == 1023u && *failed) return false;
     }

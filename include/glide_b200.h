@@ -225,9 +225,10 @@ uint32_t glide_tc_knn_fallbacks(const glide_ctx *ctx);
 void glide_exact_knn_counts(const glide_ctx *ctx, uint64_t out[4]);
 /* Bounds the scratch that such calls take, by the size of their passes: base rows and queries of a
  * glide_bruteforce_knn call, values in the padded copy of rows whose length or address TMA cannot read, and
- * 128-row tiles of a kNN stage's launches. `polls` bounds the waits inside their kernels; a call in which one runs
- * out is answered by the fp32 kernels. 0 leaves a bound at its default. Results do not depend on them. */
-int glide_limit_exact_knn(glide_ctx *ctx, uint32_t base_rows, uint32_t queries, uint32_t padded_values, uint32_t tiles, uint32_t polls);
+ * 128-row tiles of a kNN stage's launches; 0 leaves a bound at its default. With give_up the kernels behave as if
+ * one of their bounded waits had run out, and the fp32 kernels answer (a test of that path). Results do not depend
+ * on any of it. */
+int glide_limit_exact_knn(glide_ctx *ctx, uint32_t base_rows, uint32_t queries, uint32_t padded_values, uint32_t tiles, int give_up);
 
 /* ---- matrix files ----------------------------------------------------------------------- */
 /* load_matrix_data, load.cuh:10-30 (u32 rows, u32 dim, then the rows; the reference reads row by

@@ -298,10 +298,10 @@ def test_padded_partitions_are_copied_a_run_at_a_time(lens):
 
 @pytest.mark.parametrize("dim", [64, 300])      # query blocks that stay in shared memory, blocks that ride along
 def test_waits_that_run_out_leave_everything_to_the_tile_kernels(short_passes, dim):
-    """One poll per wait: a CTA gives up, drains what it has in flight and returns; the results are the tile kernel's, and the
-    context goes on."""
+    """As if a wait had run out: a CTA gives up, drains what it has in flight and returns; the results are the tile kernel's, and
+    the context goes on."""
     rng = np.random.default_rng(dim)
-    ctx = short_passes(polls=1)
+    ctx = short_passes(give_up=True)
     base, queries = (torch.from_numpy(rng.random((m, dim), np.float32)).to(ctx.torch_device) for m in (3000, 150))
     before = ctx.exact_knn_counts
     ids, dists = api.bruteforce_knn(ctx, base, queries, 10)
