@@ -7,22 +7,25 @@
 //              in shared memory where they fit (up to 256 values a row), otherwise they ride along with the
 //              rows'. tcgen05.mma kind::tf32 accumulates the 128 x 128 dot products in tensor memory (two
 //              buffers), sixteen epilogue warps turn them into a = |b|^2 - 2 q.b (thread (query, part): 32 columns).
-//   threshold  a pass over every stride-th row keeps minima over groups of rows that lie tiles apart (rows that are
-//              neighbours in the file are often neighbours in space; a group has few of a query's k nearest rows even
-//              where the file is sorted by cluster); the k-th smallest of them, t, is an upper bound of the k-th smallest a. The true k nearest then have a <= t + 2E, where E
-//              bounds |a + |q|^2 - d| for the fp32 distance d (tf32 rounding by Cauchy's inequality from the
-//              norms of what it drops, which is nothing for integers below 2048; sums by their length).
+//   threshold  a pass over every stride-th row keeps minima over groups of rows that lie tiles apart (neighbours in the file
+//              are often neighbours in space; a group has few of a query's k nearest rows even where the file is sorted by
+//              cluster); the k-th smallest of them, t, is an upper bound of the k-th smallest a. The true k nearest then have
+//              a <= t + 2E, where E bounds |a + |q|^2 - d| for the fp32 distance d: tf32 rounding by Cauchy's inequality from
+//              the norms of what it drops, which is nothing for integers below 2048; sums by their length, four steps of 2^-23
+//              a term (how the tensor core accumulates is not specified: an assumption, and a generous one).
 //   select     the pass over all tiles stores every column with a <= t + 2E.
 //   re-rank    their fp32 distances in the order of bruteforce_tile_kernel, sorted by (distance, id).
 //
 // A query with more candidates than its buffer holds (foreseen from the sample where it can be), or fewer than k, or with values
 // beyond the bounds, is left to bruteforce_tile_kernel, in the segment form with the 63 rows beside it to segment_knn_kernel; a
-// tensor map that cannot be made or a wait that runs out leaves everything to them.
-// Bound by the tensor pipe and, below it, by the trip of the row tiles from L2 (once per 128 queries).
-// bruteforce_tile_kernel against this: 1M x 128 rows, 1,000 queries, k = 10: 22.5 to 1.14 ms (0.22 of measured bf16
-// peak is what tf32 gives at best: 0.36 ms of it), k = 100: 39.1 to 2.29 ms; 100,000 x 960, 333 queries 6.5 to 0.55 ms;
-// 1M x 64, 10 queries 1.79 to 0.28 ms; 4,000 x 32, 10 queries 122 to 71 us. Where the norms are far above the distances
-// (values around 1,000, spread 1) nearly every row is a candidate and the attempt is lost: 0.39 to 0.81 ms at 50,000 x 64.
+// tensor map that cannot be made or a wait that runs out leaves everything to them. Where it is the norms that make most rows
+// candidates, a second attempt takes rows and queries about a point amid them.
+// Bound by the epilogue's chain per tile and the trip of the row tiles from L2 (once per 128 queries): the select pass over 1M x
+// 128 rows for 1,000 queries takes 0.82 ms, its 256 GFLOP are 0.31 ms at half of the measured bf16 rate.
+// bruteforce_tile_kernel against this: 1M x 128 rows, 1,000 queries, k = 10: 22.7 to 1.12 ms, k = 100: 39.1 to 2.34 ms; 100,000 x
+// 960, 333 queries 6.5 to 0.58 ms; 1M x 64, 10 queries 1.79 to 0.27 ms; 4,000 x 32, 10 queries 122 to 72 us; 300,000 x 96 in
+// clusters of 1,000 one after another, 1,000 queries, k = 100: 31.7 to 5.9 ms; 50,000 x 64 around 1,000, 100 queries 392 to
+// 182 us. 5,000 equal rows, 100 queries 729 to 819 us: an attempt is lost.
 #include <algorithm>
 #include <vector>
 
@@ -878,8 +881,9 @@ bool segment_tc_eligible(const float *data, uint32_t dim, const uint32_t *h_len,
         pairs += (uint64_t) h_len[s] * h_len[s];
     }
     // values a row meets: below 2^15 (about 1,000 rows of 32 values) the re-rank of a hundred candidates costs more than the pairs.
-    // segment_knn_kernel against this, ms: 60 partitions of 1,000 x 23 0.97 / 1.41; 2 of 2,000 x 20 0.36 / 0.28; 8 of 1,000 x 768
-    // 1.01 / 0.82; 4 of 15,000 x 50 9.8 / 7.0; 10 of 10,000 x 100 16.5 / 6.3; 15 of 4,000 x 960 (lists of 64) 34.0 / 10.3
+    // segment_knn_kernel against this, ms (uniform rows): 60 partitions of 1,000 x 23 0.97 / 1.41; 2 of 2,000 x 20 0.36 / 0.25; 8 of
+    // 1,000 x 768 1.01 / 0.82; 4 of 15,000 x 50 9.8 / 7.2; 10 of 10,000 x 100 16.5 / 6.7, one of them with 3,000 equal rows 16.4 /
+    // 9.0; 200 of 3,000 x 36 22.2 / 12.4; 15 of 4,000 x 960 (lists of 64) 34.1 / 17.0
     return pairs * dim >= taken << 15;
 }
 
