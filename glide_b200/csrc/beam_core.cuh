@@ -76,7 +76,8 @@ __device__ __forceinline__ WarpStrip make_strip(uint32_t *base, uint32_t dim, ui
 // adjacency rows of the candidates they score, one of which the next expansion reads.
 //   rows that fit the lanes   the helpers score a whole adjacency row while the master puts its ids into the
 //                             visited set, a chain as long as a trip to memory; the distances of the ids that
-//                             were not new (about a tenth) are dropped. Four helpers, beam 64, one query:
+//                             were not new are dropped (of the rows read 9 % for one query on 10,000 x 32 rows, 14 % for
+//                             600 on 300,000 x 128 at beam 64, 16 % at beam 128). Four helpers, beam 64, one query:
 //                             207 us alone, 162 with the set in front of the scoring, 120 beside it.
 //   wider rows                the set comes first and the master scores its share too: rows that are dropped
 //                             and a warp that does not read cost more than the set's chain (960 values,
@@ -521,7 +522,7 @@ __device__ __forceinline__ void sort_candidates_two_warps(float *cand_k, uint32_
 // 655 to 627 us, 2,000 at beam 128 1136 to 1078 us.
 // All of this takes an ascending beam. The seed step alone can leave another one: an infinite distance (a row
 // that holds an infinity, a square beyond fp32) or one that is no number sorts behind the empty slots' FLT_MAX,
-// which follow it in the beam all the same. Such a search (kSeedNetworks) takes the networks at every merge, as they
+// which follow it in the beam all the same. Such a search (SeedNetworks) takes the networks at every merge, as they
 // move these entries. No later candidate brings one in: the merges take only what is smaller than a slot's key.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kFewSurvivors = 8;
@@ -633,9 +634,14 @@ __device__ __forceinline__ void trim_beam(float (&bk)[NB], uint32_t (&bv)[NB], u
 // Drops the candidates beyond the beam's last slot ((FLT_MAX, kInvalid), as an empty slot) and does as
 // much of the merge as few survivors allow. kMergeDone: the beam is merged. kMergeSorted: (ck[0], cv[0]) of lane j
 // is the j-th survivor, the merge is left to do. kMergeSort: both are.
-// open_seed (kSeedWide): the seed row held a valid id with distance FLT_MAX; while such an entry may sit among the
+// open_seed: the seed row held a valid id with distance FLT_MAX; while such an entry may sit among the
 // beam's empty slots, which of them a merge replaces is the network's business too.
-constexpr uint32_t kSeedWide = 1, kSeedNetworks = 2;   // what the seed step left behind, see above
+// What the seed step left behind: kSeedWide is wide_first_sort, SeedNetworks a beam that is not ascending (see above). Builds keep
+// them in one word; searches, which have no wide_first_sort, keep the bit in the count of rows. Measured: a flag of its own 208.5 ms
+// in the build of 1M x 128 rows, beside wide_first_sort 203.8, in the count 208 to 212; a word costs searches of wide rows 1 %, the
+// bit in the count nothing.
+constexpr uint32_t kSeedWide = 1;
+template<bool BUILD> struct SeedNetworks { static constexpr uint32_t bit = BUILD ? 2u : 0x80000000u; };
 enum MergeState : int { kMergeDone = 0, kMergeSorted = 1, kMergeSort = 2 };
 
 template<int NB, int NC>
@@ -688,12 +694,15 @@ __device__ __forceinline__ uint32_t beam_loop(float (&bk)[NB], uint32_t (&bv)[NB
                                               uint32_t *rows_read, bool wide_first_sort = false) {
     const uint32_t lane = lane_id();
     constexpr uint32_t MAXB = 32u * NB;
-    uint32_t iter = 0, seed = wide_first_sort ? kSeedWide : 0u;
+    constexpr bool BUILD = NARROW_SORT;
+    uint32_t iter = 0;
     bool terminate = false;
-    uint32_t rows = 0;
+    uint32_t rows = 0, seed = wide_first_sort ? kSeedWide : 0u;
+    uint32_t &state_bits = BUILD ? seed : rows;
+    constexpr uint32_t networks = SeedNetworks<BUILD>::bit;
     while (true) {
         MergeState state = kMergeSort;
-        if (iter != 0 && !(seed & kSeedNetworks)) {
+        if (iter != 0 && !(state_bits & networks)) {
             float ck[NC];
             uint32_t cv[NC];
 #pragma unroll
@@ -768,7 +777,7 @@ __device__ __forceinline__ uint32_t beam_loop(float (&bk)[NB], uint32_t (&bv)[NB
                     bk[i] = take ? s.cand_dist[j] : FLT_MAX;
                     bv[i] = take ? s.cand_id[j] : kInvalid;
                 }
-                if (beyond_empty<NB>(bk)) seed |= kSeedNetworks;
+                if (beyond_empty<NB>(bk)) state_bits |= networks;
             } else if constexpr (NB == 16) {
                 merge_beam_two_warps(bk, bv, p.beam, degree, s.cand_dist, s.cand_id, reinterpret_cast<float *>(s.tail), s.tail + 512);
             } else {
@@ -838,7 +847,7 @@ __device__ __forceinline__ uint32_t beam_loop(float (&bk)[NB], uint32_t (&bv)[NB
         rows += expand_parent<TEAM>(s, parent, own_id, graph, degree, p.hash_bit, data, dim, metric);
         iter++;
     }
-    if (rows_read) *rows_read += rows;
+    if (rows_read) *rows_read += BUILD ? rows : rows & ~networks;
     return iter;
 }
 
@@ -895,7 +904,7 @@ __device__ __forceinline__ uint32_t expand_lanes(const WarpStrip &s, uint32_t pa
 }
 
 // (ck, cv): the seed step's candidates, slot = lane. Otherwise as beam_loop.
-template<int NB, bool TEAM = false, typename D>
+template<int NB, bool TEAM = false, bool BUILD = false, typename D>
 __device__ __forceinline__ uint32_t beam_loop_lanes(float (&bk)[NB], uint32_t (&bv)[NB], const WarpStrip &s,
                                                     const BeamParams &p, uint32_t own_id,
                                                     const uint32_t *__restrict__ graph, uint32_t degree,
@@ -904,12 +913,14 @@ __device__ __forceinline__ uint32_t beam_loop_lanes(float (&bk)[NB], uint32_t (&
                                                     bool wide_first_sort = false) {
     const uint32_t lane = lane_id();
     constexpr uint32_t MAXB = 32u * NB;
-    uint32_t iter = 0, seed = wide_first_sort ? kSeedWide : 0u;
+    uint32_t iter = 0;
     bool terminate = false;
-    uint32_t rows = 0;
+    uint32_t rows = 0, seed = wide_first_sort ? kSeedWide : 0u;
+    uint32_t &state_bits = BUILD ? seed : rows;
+    constexpr uint32_t networks = SeedNetworks<BUILD>::bit;
     while (true) {
         MergeState state = kMergeSort;
-        if (iter != 0 && !(seed & kSeedNetworks)) {
+        if (iter != 0 && !(state_bits & networks)) {
             float k1[1] = {ck};
             uint32_t v1[1] = {cv};
             state = merge_few<NB, 1>(bk, bv, p.beam, k1, v1, (seed & kSeedWide) != 0);
@@ -946,7 +957,7 @@ __device__ __forceinline__ uint32_t beam_loop_lanes(float (&bk)[NB], uint32_t (&
                     bk[i] = take ? c : FLT_MAX;
                     bv[i] = take ? id : kInvalid;
                 }
-                if (beyond_empty<NB>(bk)) seed |= kSeedNetworks;
+                if (beyond_empty<NB>(bk)) state_bits |= networks;
             } else if constexpr (NB == 16) {
                 float *row_k = reinterpret_cast<float *>(s.tail + 1024);
                 uint32_t *row_v = s.tail + 1024 + 32;
@@ -1020,7 +1031,7 @@ __device__ __forceinline__ uint32_t beam_loop_lanes(float (&bk)[NB], uint32_t (&
         rows += expand_lanes<TEAM>(s, parent, own_id, graph, degree, p.hash_bit, data, dim, metric, ck, cv);
         iter++;
     }
-    if (rows_read) *rows_read += rows;
+    if (rows_read) *rows_read += BUILD ? rows : rows & ~networks;
     return iter;
 }
 

@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(256, NB <= 4 ? ctas_per_sm<D>(4, 3) : 2) build
             uint32_t cv;
             rows += seed_lanes(s, a.start_points[seg], point, pknn, a.in_degree, p.hash_bit, pdata, dim, a.metric, ck, cv,
                                &wide);
-            iters = beam_loop_lanes<NB>(bk, bv, s, p, point - seg_start, pknn, a.in_degree, pdata, dim, a.metric, &rows,
+            iters = beam_loop_lanes<NB, false, true>(bk, bv, s, p, point - seg_start, pknn, a.in_degree, pdata, dim, a.metric, &rows,
                                         ck, cv, wide);
         } else {
             rows += seed_from_row(s, a.start_points[seg], point, pknn, a.in_degree, p.hash_bit, pdata, dim, a.metric, &wide);
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(256, NB <= 4 ? ctas_per_sm<D>(4, 3) : 2) build
             float ck;
             uint32_t cv;
             rows += seed_lanes(s, start, exclude, a.graph_in, degree, p.hash_bit, a.data, dim, a.metric, ck, cv, &wide);
-            iters = beam_loop_lanes<NB>(bk, bv, s, p, point, a.graph_in, degree, a.data, dim, a.metric, &rows, ck, cv, wide);
+            iters = beam_loop_lanes<NB, false, true>(bk, bv, s, p, point, a.graph_in, degree, a.data, dim, a.metric, &rows, ck, cv, wide);
         } else {
             rows += seed_from_row(s, start, exclude, a.graph_in, degree, p.hash_bit, a.data, dim, a.metric, &wide);
             iters = beam_loop<NB, NC, true>(bk, bv, s, p, point, a.graph_in, degree, a.data, dim, a.metric, &rows, wide);
